@@ -3,6 +3,7 @@
 #include <math.h>
 
 #include "sg_internal.cuh"
+#include "sg_mpnn_bwd.cuh"
 #include "sg_mpnn_fold.cuh"
 #include "sg_mpnn_fwd.cuh"
 #include "sg_solver.h"
@@ -42,122 +43,6 @@ static void graph_free(GraphH *G) {
   graph_free(G->twin);
   for (void *p : G->allocs) cudaFree(p);
   delete G;
-}
-
-// ---------------------------------------------------------------------------
-// backward (FP32, one warp per vertex; training meshes only)
-// ---------------------------------------------------------------------------
-// B1: dg3 = (Wout^T dz) * [g3 > 0]; dm3 = W3m^T dg3; dh2a = bf(W3h)^T dg3.
-__global__ void k_b1(int32_t n, int lin, const float *__restrict__ prm, const float *__restrict__ dz,
-                     const float *__restrict__ g3, float *__restrict__ dg3,
-                     float *__restrict__ dm3, float *__restrict__ dh2a) {
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t v = wid; v < n; v += nw) {
-    const float d0 = dz[v * 3], d1 = dz[v * 3 + 1], d2 = dz[v * 3 + 2];
-    float dg[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int h = lane * 2 + e;
-      const float d = prm[O_WOUT + h] * d0 + prm[O_WOUT + H + h] * d1 + prm[O_WOUT + 2 * H + h] * d2;
-      dg[e] = (lin || g3[v * H + h] > 0.f) ? d : 0.f;
-      dg3[v * H + h] = dg[e];
-    }
-    // dm3_j = sum_h W3m[h][j] dg3[h]
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      float p = prm[O_W3M + (lane * 2) * K + j] * dg[0] + prm[O_W3M + (lane * 2 + 1) * K + j] * dg[1];
-      for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-      if (lane == 0) dm3[v * K + j] = p;
-    }
-    // dh2a[c] = sum_h bf(W3h[h][c]) dg3[h]; lane owns c = 2*lane + e
-    float acc0 = 0.f, acc1 = 0.f;
-    for (int h = 0; h < H; ++h) {
-      const float dgh = __shfl_sync(0xffffffffu, dg[h & 1], h >> 1);
-      acc0 += bf16r(prm[O_W3H + h * H + lane * 2]) * dgh;
-      acc1 += bf16r(prm[O_W3H + h * H + lane * 2 + 1]) * dgh;
-    }
-    dh2a[v * H + lane * 2] = acc0;
-    dh2a[v * H + lane * 2 + 1] = acc1;
-  }
-}
-
-// Generic middle step: dq = sum_u a dm_u (K); dh = dha + P^T dq; dg = dh *
-// [g > 0]; optional dm_next = Wm^T dg (K), dha_next = bf(Wh)^T dg (H).
-__global__ void k_bmid(int32_t n, int lin, const uint32_t *__restrict__ rowptr,
-                       const uint32_t *__restrict__ colidx, const float *__restrict__ a,
-                       const float *__restrict__ prm, int oP, int oWm, int oWh,
-                       const float *__restrict__ dm, const float *__restrict__ dha,
-                       const float *__restrict__ g, float *__restrict__ dq,
-                       float *__restrict__ dgout, float *__restrict__ dm_next,
-                       float *__restrict__ dha_next) {
-  const int lane = threadIdx.x & 31;
-  const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t v = wid; v < n; v += nw) {
-    // dq (K values): lanes 0..7 gather one component each
-    float dqj = 0.f;
-    if (lane < K)
-      for (uint32_t q = rowptr[v]; q < rowptr[v + 1]; ++q) dqj += a[q] * dm[(size_t)colidx[q] * K + lane];
-    if (lane < K) dq[v * K + lane] = dqj;
-    float dg[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int h = lane * 2 + e;
-      float d = dha[v * H + h];
-#pragma unroll
-      for (int j = 0; j < K; ++j) d += prm[oP + j * H + h] * __shfl_sync(0xffffffffu, dqj, j);
-      dg[e] = (lin || g[v * H + h] > 0.f) ? d : 0.f;
-      dgout[v * H + h] = dg[e];
-    }
-    if (dm_next) {
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        float p = prm[oWm + (lane * 2) * K + j] * dg[0] + prm[oWm + (lane * 2 + 1) * K + j] * dg[1];
-        for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
-        if (lane == 0) dm_next[v * K + j] = p;
-      }
-      float acc0 = 0.f, acc1 = 0.f;
-      for (int h = 0; h < H; ++h) {
-        const float dgh = __shfl_sync(0xffffffffu, dg[h & 1], h >> 1);
-        acc0 += bf16r(prm[oWh + h * H + lane * 2]) * dgh;
-        acc1 += bf16r(prm[oWh + h * H + lane * 2 + 1]) * dgh;
-      }
-      dha_next[v * H + lane * 2] = acc0;
-      dha_next[v * H + lane * 2 + 1] = acc1;
-    }
-  }
-}
-
-// Outer-product reduction dW[o][i] = sum_v X_v[o] * Y_v[i] over a chunk of
-// vertices per CTA; partials part[chunk][O*I], summed in order afterwards.
-// Y is transformed: 0 identity, 1 relu, 2 bf16(relu), 4 bf16.
-constexpr int OUTER_CHUNK = 1024;
-__global__ void k_outer(int32_t n, const float *__restrict__ X, int O, const float *__restrict__ Y,
-                        int I, int ytr, float *__restrict__ part) {
-  const int64_t v0 = (int64_t)blockIdx.x * OUTER_CHUNK;
-  const int64_t v1 = min((int64_t)n, v0 + OUTER_CHUNK);
-  for (int e = threadIdx.x; e < O * I; e += blockDim.x) {
-    const int o = e / I, i = e % I;
-    float acc = 0.f;
-    for (int64_t v = v0; v < v1; ++v) {
-      float y = Y[v * I + i];
-      if (ytr == 1 || ytr == 2) y = fmaxf(y, 0.f);
-      if (ytr == 2 || ytr == 4) y = bf16r(y);
-      acc += X[v * O + o] * y;
-    }
-    part[(size_t)blockIdx.x * O * I + e] = acc;
-  }
-}
-
-__global__ void k_outer_sum(const float *__restrict__ part, int chunks, int len,
-                            float *__restrict__ out) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < len; e += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < chunks; ++c) s += part[(size_t)c * len + e];
-    out[e] = s;
-  }
 }
 
 __global__ void k_adam(int np, float *__restrict__ p, const float *__restrict__ g,
@@ -269,7 +154,6 @@ static int set_sym(GraphH *G, int sym) {
   SG_TRY(galloc(G, (void **)&g.wp, n * 3 * 4));
   SG_TRY(galloc(G, (void **)&g.t, n * 3 * 4));
   SG_TRY(galloc(G, (void **)&g.prmT, NPARAM * 4));
-  SG_TRY(galloc(G, (void **)&g.gtmp, NPARAM * 4));
   GraphH *T = new GraphH();
   G->twin = T;
   T->c = G->c;
@@ -513,8 +397,14 @@ static int ensure_train(GraphH *G) {
   for (float **p : {&g.g1, &g.g2, &g.g3, &g.dg1, &g.dg2, &g.dg3, &g.dh1a, &g.dh2a})
     SG_TRY(galloc(G, (void **)p, n * H * 4));
   for (float **p : {&g.dm2, &g.dm3, &g.dq2, &g.dq3}) SG_TRY(galloc(G, (void **)p, n * K * 4));
-  g.gpart_chunks = (int)((n + OUTER_CHUNK - 1) / OUTER_CHUNK);
-  SG_TRY(galloc(G, (void **)&g.gpart, (size_t)g.gpart_chunks * H * H * 4));
+  // weight-gradient chunks: two waves of CTAs per group, slabs of WG_V
+  // vertices at least, and at most 1,024 vertices in one FP32 sum
+  size_t chunks = (n + WG_V - 1) / WG_V;
+  if (chunks > 2 * (size_t)G->c->num_sms) chunks = 2 * (size_t)G->c->num_sms;
+  if (chunks < (n + 1023) / 1024) chunks = (n + 1023) / 1024;
+  g.gpart_rows = (int)((n + chunks - 1) / chunks);
+  g.gpart_chunks = (int)((n + g.gpart_rows - 1) / g.gpart_rows);
+  SG_TRY(galloc(G, (void **)&g.gpart, (size_t)g.gpart_chunks * NPARAM * 4));
   SG_TRY(galloc(G, (void **)&g.ld, n * 3 * 4));
   SG_TRY(galloc(G, (void **)&g.lq, n * 3 * 4));
   G->train_ready = true;
@@ -588,17 +478,7 @@ static int forward(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int gate, co
   return SG_OK;
 }
 
-static int outer(GraphH *G, const float *X, int O, const float *Y, int I, int ytr, float *dst) {
-  Ctx *c = G->c;
-  Graph &g = G->g;
-  k_outer<<<g.gpart_chunks, 256, 0, c->stream>>>(g.n, X, O, Y, I, ytr, g.gpart);
-  SG_CHECK_LAUNCH();
-  k_outer_sum<<<(O * I + 255) / 256, 256, 0, c->stream>>>(g.gpart, g.gpart_chunks, O * I, dst);
-  SG_CHECK_LAUNCH();
-  return SG_OK;
-}
-
-static int backward_net(GraphH *G, const float *prm, const float *dz, float *grad);
+static int backward_net(GraphH *G, const float *prm, const float *dz, float *grad, int add);
 
 // Weight gradient of <dz, M r>.  Symmetric form: the network's gradient at
 // input L^-1 r with cotangent (I + N) L^-1 dz, plus its gradient at input
@@ -606,7 +486,7 @@ static int backward_net(GraphH *G, const float *prm, const float *dz, float *gra
 // twin's buffers so the first pass's activations survive.
 static int backward(GraphH *G, const float *prm, const float *dz, float *grad) {
   Graph &g = G->g;
-  if (!g.sym) return backward_net(G, prm, dz, grad);
+  if (!g.sym) return backward_net(G, prm, dz, grad, 0);
   GraphH *T = G->twin;
   Ctx *c = G->c;
   SG_TRY(ensure_train(T));
@@ -614,39 +494,35 @@ static int backward(GraphH *G, const float *prm, const float *dz, float *grad) {
   k_f1<<<gv, 256, 0, c->stream>>>(nullptr, 0, g.n, g.linv, dz, T->g.s, nullptr);
   SG_CHECK_LAUNCH();
   SG_TRY(layers(T, c->stream, nullptr, 0, prm, T->g.s, T->g.y, true));
-  SG_TRY(backward_net(G, prm, T->g.y, grad));
-  SG_TRY(backward_net(T, prm, g.y, g.gtmp));
-  k_add_f<<<(NPARAM + 255) / 256, 256, 0, c->stream>>>(NPARAM, grad, g.gtmp);
-  SG_CHECK_LAUNCH();
-  return SG_OK;
+  SG_TRY(backward_net(G, prm, T->g.y, grad, 0));
+  return backward_net(T, prm, g.y, grad, 1);
 }
 
-static int backward_net(GraphH *G, const float *prm, const float *dz, float *grad) {
+static int backward_net(GraphH *G, const float *prm, const float *dz, float *grad, int add) {
   Ctx *c = G->c;
   Graph &g = G->g;
   SG_TRY(ensure_train(G));
-  const int gw = grid_for(c, (int64_t)g.n * 32, 256, 8);
+  const int gw = grid_for(c, ((int64_t)g.n + BW_V - 1) / BW_V * BW_T, BW_T, 5);
   cudaStream_t st = c->stream;
-  k_b1<<<gw, 256, 0, st>>>(g.n, g.lin, prm, dz, g.g3, g.dg3, g.dm3, g.dh2a);
+  k_b1<<<gw, BW_T, 0, st>>>(g.n, g.lin, prm, dz, g.g3, g.dg3, g.dm3, g.dh2a);
   SG_CHECK_LAUNCH();
-  k_bmid<<<gw, 256, 0, st>>>(g.n, g.lin, g.rowptr, g.colidx, g.a, prm, O_P3, O_W2M, O_W2H, g.dm3, g.dh2a,
-                             g.g2, g.dq3, g.dg2, g.dm2, g.dh1a);
+  k_bmid<<<gw, BW_T, 0, st>>>(g.n, g.lin, g.rowptr, g.colidx, g.a, prm, O_P3, O_W2M, O_W2H, g.dm3,
+                              g.dh2a, g.g2, g.dq3, g.dg2, g.dm2, g.dh1a);
   SG_CHECK_LAUNCH();
-  k_bmid<<<gw, 256, 0, st>>>(g.n, g.lin, g.rowptr, g.colidx, g.a, prm, O_P2, 0, 0, g.dm2, g.dh1a, g.g1,
-                             g.dq2, g.dg1, nullptr, nullptr);
+  k_bmid<<<gw, BW_T, 0, st>>>(g.n, g.lin, g.rowptr, g.colidx, g.a, prm, O_P2, 0, 0, g.dm2, g.dh1a,
+                              g.g1, g.dq2, g.dg1, nullptr, nullptr);
   SG_CHECK_LAUNCH();
-  // weight gradients; h = act(g) (relu, or identity in the linear variant)
+  // weight gradients; h = act(g) (relu, or identity in the linear variant);
   // the tensor-core operand is bf16(h), or ~h itself with split activations
-  const int A_ = g.lin ? 0 : 1, AB = g.sym ? 0 : (g.lin ? 4 : 2);
-  SG_TRY(outer(G, dz, 3, g.g3, H, A_, grad + O_WOUT));
-  SG_TRY(outer(G, g.dg3, H, g.g2, H, AB, grad + O_W3H));
-  SG_TRY(outer(G, g.dg3, H, g.m3, K, 0, grad + O_W3M));
-  SG_TRY(outer(G, g.dq3, K, g.g2, H, A_, grad + O_P3));
-  SG_TRY(outer(G, g.dg2, H, g.g1, H, AB, grad + O_W2H));
-  SG_TRY(outer(G, g.dg2, H, g.m2, K, 0, grad + O_W2M));
-  SG_TRY(outer(G, g.dq2, K, g.g1, H, A_, grad + O_P2));
-  SG_TRY(outer(G, g.dg1, H, g.s, 3, 0, grad + O_W1S));
-  SG_TRY(outer(G, g.dg1, H, g.m1, 3, 0, grad + O_W1M));
+  WgradArgs w = {g.n, g.gpart_rows, dz, g.dg1, g.dg2, g.dg3, g.dq2, g.dq3,
+                 g.g1, g.g2, g.g3, g.s, g.m1, g.m2, g.m3, g.gpart};
+  const dim3 grid((unsigned)g.gpart_chunks, 3);
+  if (!g.lin) k_wgrad<true, true><<<grid, 256, 0, st>>>(w);
+  else if (!g.sym) k_wgrad<false, true><<<grid, 256, 0, st>>>(w);
+  else k_wgrad<false, false><<<grid, 256, 0, st>>>(w);
+  SG_CHECK_LAUNCH();
+  k_wgrad_sum<<<(NPARAM + 31) / 32, 256, 0, st>>>(g.gpart, g.gpart_chunks, add, grad);
+  SG_CHECK_LAUNCH();
   return SG_OK;
 }
 

@@ -53,18 +53,17 @@ struct Graph {
   float *dg1 = nullptr, *dg2 = nullptr, *dg3 = nullptr, *dh1a = nullptr, *dh2a = nullptr;
   float *dm2 = nullptr, *dm3 = nullptr, *dq2 = nullptr, *dq3 = nullptr;
   float *gpart = nullptr;  // weight-gradient partials
-  int gpart_chunks = 0;
+  int gpart_chunks = 0, gpart_rows = 0;
   float *ld = nullptr, *lq = nullptr;  // loss temporaries
   double *dres = nullptr;
   int lin = 0;  // identity activations (a linear preconditioner) instead of relu
   // Symmetric factorized form M = L^-T (I+N)^T (I+N) L^-1 (sym = 1, lin = 1):
   // L^-1 per vertex, y = (I+N) L^-1 r, the transposed network's outputs
-  // wp = y + W1s^T h3' and t = W1m^T h3', transposed parameters, and a
-  // gradient buffer for the second weight-gradient pass.
+  // wp = y + W1s^T h3' and t = W1m^T h3', and transposed parameters.
   int sym = 0;
   float *linv = nullptr;   // [n*9]
   float *y = nullptr, *wp = nullptr, *t = nullptr;  // [n*3]
-  float *prmT = nullptr, *gtmp = nullptr;           // [NPARAM]
+  float *prmT = nullptr;                            // [NPARAM]
 };
 
 __device__ __forceinline__ float bf16r(float x) {

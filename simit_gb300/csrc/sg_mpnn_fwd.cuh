@@ -575,11 +575,6 @@ __global__ void k_sym_out(const SolveCtl *ctl, int gate, int32_t n,
   }
 }
 
-__global__ void k_add_f(int n, float *__restrict__ a, const float *__restrict__ b) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    a[i] += b[i];
-}
-
 inline size_t tc_smem_bytes() { return sizeof(TCW) + TC_WARPS * sizeof(TCWarp); }
 
 }  // namespace mpnn

@@ -66,6 +66,41 @@ def test_forward_backward_match_oracle(ctx, form):
     prob.close()
 
 
+@pytest.mark.parametrize("form", ["relu", "linear", "sym"])
+@pytest.mark.parametrize("ncell", [2, 3, 7, 9])
+def test_backward_at_tile_edges(ctx, form, ncell):
+    """27, 64, 512 and 1,000 vertices: below, at and past the backward's
+    tiles of 64 vertices and slabs of 32.  The bound is the one above: the
+    oracle sums in FP64 what the kernels sum in FP32."""
+    from oracle import mpnn_oracle as mo
+    from simit_gb300 import learned
+    prob = _small(ctx, ncell)
+    m = prob.mesh
+    rp, ci = m.pattern.host()
+    vals = prob.A.cpu().numpy()
+    g = learned.Graph(ctx, m, prob.A, form=form)
+    params = learned.init_params(seed=6, out_scale=1.0)
+    rng = np.random.Generator(np.random.Philox(ncell))
+    r, dz = rng.normal(size=(2, m.n * 3)).astype(np.float32)
+    d = ctx.device
+    pt, rt = torch.tensor(params, device=d), torch.tensor(r, device=d)
+    zt, grad = torch.empty_like(rt), torch.full_like(pt, float("nan"))
+    g.forward(pt, rt, zt, train=True)
+    g.backward(pt, torch.tensor(dz, device=d), grad)
+    if form == "sym":
+        gref = mo.backward_sym(mo.forward_sym(params, m.n, rp, ci, vals, r)[1], dz)
+    else:
+        gref = mo.backward(mo.forward(params, m.n, rp, ci, vals, r, linear=form == "linear")[1], dz)
+    gg, o = grad.cpu().numpy(), 0
+    for name, (a, b) in mo.SHAPES:
+        seg = slice(o, o + a * b)
+        o += a * b
+        err = np.linalg.norm(gg[seg] - gref[seg])
+        assert err <= 2e-3 * np.linalg.norm(gref[seg]) + 1e-6, (name, err, np.linalg.norm(gref[seg]))
+    g.close()
+    prob.close()
+
+
 @pytest.mark.parametrize("form", ["relu", "sym"])
 def test_training_reduces_loss(ctx, form):
     from simit_gb300 import learned
