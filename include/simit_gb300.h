@@ -129,9 +129,9 @@ int sg_pattern_maxrow(sg_ctx *ctx, int32_t n, const uint32_t *rowptr,
 /* ---------------------------------------------------------------------
  * Assembly ("map f to E reduce +").  Replaces the reference's map lowering
  * (src/inline.cpp:690-888, src/lower/lower_maps.cpp:54-128) and its GPU
- * atomics (src/backend/gpu/gpu_backend.cpp:788-846).  A group of lanes owns
- * each block row and sums its elements' contributions in ascending element
- * order (the reference's order) without atomics.  exact != 0 selects kernels
+ * atomics (src/backend/gpu/gpu_backend.cpp:788-846).  A tile or a group of
+ * lanes owns each block row and sums its elements' contributions in ascending
+ * element order (the reference's order) without floating-point atomics.  exact != 0 selects kernels
  * compiled without multiply-add contraction in the reference's operation
  * order (FP64 results equal to the reference's up to libm `log`); exact == 0
  * selects contracted kernels (and the closed-form linear-tet stiffness).
@@ -150,13 +150,13 @@ typedef struct sg_mesh {
   const uint32_t *colidx;
   int64_t nnzb;
   int32_t maxrow;             /* sg_pattern_maxrow */
-  /* Optional element-parallel assembly plans (assembly with exact == 0
-   * computes every element once; exact == 1 always runs the row-owner
-   * kernels, the reference's element order bit for bit; NULL / 0 everywhere:
-   * row owners).  Both need slots.
-   *  - slot_src_ptr / slot_src set (sg_slot_sources): element blocks are
-   *    written once, then every slot sums its blocks in ascending element
-   *    order and every vertex its vector contributions (deterministic).
+  /* Optional plans.  The built-in maps read their elements' columns from
+   * slots when it is set (and search the rows otherwise), in the same
+   * summation order.  The caller-evaluated blocks (sg_assemble_blocks) with
+   * exact == 0 use a whole plan; exact == 1 keeps the reference's element
+   * order bit for bit.  Both plans need slots.
+   *  - slot_src_ptr / slot_src set (sg_slot_sources): every slot sums its
+   *    blocks in ascending element order (deterministic).
    *  - else color_order / color_ptr set (sg_element_coloring): blocks are
    *    added into their slots colour by colour (no two elements of a colour
    *    share a vertex, so no atomics; deterministic, colour order). */
@@ -167,9 +167,8 @@ typedef struct sg_mesh {
   int32_t ncolors;
   const uint32_t *slot_src_ptr; /* device [nnzb+1] (sg_slot_sources) */
   const uint32_t *slot_src;     /* device [nE*card*card] */
-  int32_t asm_tile;             /* element tile of the element-blocks plan: threads
-                                   per CTA, 128 / 256 / 512 (0 = 256); the host
-                                   runtime's assembly tuner picks it */
+  int32_t asm_tile;             /* read by no kernel (it was the element-blocks
+                                   plan's tile); kept for the layout */
 } sg_mesh;
 
 /* The inverse slot map for the element-blocks plan: for slot q, the element
@@ -312,8 +311,8 @@ int sg_tet_precompute(sg_ctx *ctx, const sg_mesh *mesh, int dtype,
 /* compute_stiffness of femTet.sim (SG_MODEL_NEOHOOKEAN: dPdF tangent) or of
  * apps/fem/fem_linear.sim:105-174 (SG_MODEL_LINEAR: W*B'*E*B), scaled by h*h,
  * plus the lumped element mass on the diagonal; c int32 [n] (c > 0 =
- * constrained); mu, lam [nE].  The neo-Hookean path uses nE*16*9 values of
- * context scratch. */
+ * constrained); mu, lam [nE].  The exact neo-Hookean path uses nE*16*9
+ * values of context scratch. */
 int sg_assemble_tet_stiffness(sg_ctx *ctx, const sg_mesh *mesh, int dtype,
                               int model, const void *x, const int32_t *c,
                               const void *B, const void *W, const void *mu,

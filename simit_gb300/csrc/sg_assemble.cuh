@@ -24,6 +24,10 @@
 // neo-Hookean tangent, whose element blocks are expensive, a separate
 // element-parallel kernel writes the blocks once to a scratch array and the
 // row owners gather from it (EbGather).
+//
+// The row owners run the exact mode of the tetrahedral maps and the
+// caller-evaluated blocks; the other maps run the row tiles of
+// sg_assemble_tile.cuh.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -232,9 +236,8 @@ __global__ void __launch_bounds__(128) k_rows(AsmArgs<T> a) {
 // ---------------------------------------------------------------------------
 // Element-parallel kernel (one colour of the assembly plan)
 // ---------------------------------------------------------------------------
-// Each element is computed once: the threads of an element (one per block
-// (i, j) for matrix maps, one per local vertex i for vector-only maps) add
-// its contributions into the precomputed slots / rows with plain
+// Caller-evaluated element blocks: the threads of an element (one per block
+// (i, j)) add them into the precomputed slots with plain
 // read-modify-writes.  No two elements of a colour share a vertex, so no
 // other thread touches those values during the launch; colours run in
 // order, so every value is summed in the same order on every run.  An
@@ -246,97 +249,66 @@ __global__ void __launch_bounds__(128) k_rows(AsmArgs<T> a) {
 template <class Elem, int CARD, int BS, typename T>
 __device__ __forceinline__ void colored_row(const AsmArgs<T> &a, int64_t e, int i,
                                             const uint32_t *__restrict__ slots) {
-  const int32_t vi = a.ep[e * CARD + i];
-  if (Elem::HAS_MAT) {
-    for (int j = 0; j < CARD; ++j) {
-      const uint32_t sl = slots[(e * CARD + i) * CARD + j];
-      if ((int64_t)sl >= a.nnzb) {
-        atomicCAS(a.err, 0, 3 /* DEV_SLOT_MISSING */);
-        continue;
-      }
-      for (int l = 0; l < BS; ++l) {
-        T out[2][BS];
-        const int nt = Elem::block(a, e, i, j, l, out);
-        if (nt > 0) {
-          T *dst = a.vals + (size_t)sl * BS * BS + l * BS;
-          for (int q = 0; q < BS; ++q) {
-            T v = dst[q] + out[0][q];
-            if (nt > 1) v += out[1][q];
-            dst[q] = v;
-          }
-        }
-      }
+  for (int j = 0; j < CARD; ++j) {
+    const uint32_t sl = slots[(e * CARD + i) * CARD + j];
+    if ((int64_t)sl >= a.nnzb) {
+      atomicCAS(a.err, 0, 3 /* DEV_SLOT_MISSING */);
+      continue;
     }
-  }
-  if (Elem::HAS_VEC) {
     for (int l = 0; l < BS; ++l) {
-      T o[4];
-      const int nv = Elem::vec(a, e, i, l, o);
-      if (nv > 0) {
-        T v = a.f[(int64_t)vi * BS + l];
-        for (int q = 0; q < nv; ++q) v += o[q];
-        a.f[(int64_t)vi * BS + l] = v;
+      T out[2][BS];
+      const int nt = Elem::block(a, e, i, j, l, out);
+      if (nt > 0) {
+        T *dst = a.vals + (size_t)sl * BS * BS + l * BS;
+        for (int q = 0; q < BS; ++q) {
+          T v = dst[q] + out[0][q];
+          if (nt > 1) v += out[1][q];
+          dst[q] = v;
+        }
       }
     }
   }
 }
 
-// Usual form (distinct vertices), one thread per block (i, j) of a matrix
-// element (its old values loaded first -- independent loads, one memory
-// round trip -- then its rows added and stored), and per vertex i for the
-// vector part (thread j = 0).  Distinct vertices give distinct slots and
-// rows, so nothing aliases.
+// Usual form (distinct vertices), one thread per block (i, j) of an element
+// (its old values loaded first -- independent loads, one memory round trip --
+// then its rows added and stored).  Distinct vertices give distinct slots,
+// so nothing aliases.
 template <class Elem, int CARD, int BS, typename T>
 __device__ __forceinline__ void colored_block(const AsmArgs<T> &a, int64_t e, int i, int j,
                                               const uint32_t *__restrict__ slots) {
-  if (Elem::HAS_MAT) {
-    const uint32_t sl = slots[(e * CARD + i) * CARD + j];
-    if ((int64_t)sl >= a.nnzb) {
-      atomicCAS(a.err, 0, 3 /* DEV_SLOT_MISSING */);
-    } else {
-      T *dst = a.vals + (size_t)sl * BS * BS;
-      T old[BS * BS];
+  const uint32_t sl = slots[(e * CARD + i) * CARD + j];
+  if ((int64_t)sl >= a.nnzb) {
+    atomicCAS(a.err, 0, 3 /* DEV_SLOT_MISSING */);
+    return;
+  }
+  T *dst = a.vals + (size_t)sl * BS * BS;
+  T old[BS * BS];
 #pragma unroll
-      for (int q = 0; q < BS * BS; ++q) old[q] = dst[q];
+  for (int q = 0; q < BS * BS; ++q) old[q] = dst[q];
 #pragma unroll
-      for (int l = 0; l < BS; ++l) {
-        T out[2][BS];
-        const int nt = Elem::block(a, e, i, j, l, out);
+  for (int l = 0; l < BS; ++l) {
+    T out[2][BS];
+    const int nt = Elem::block(a, e, i, j, l, out);
 #pragma unroll
-        for (int q = 0; q < BS; ++q) {
-          if (nt > 0) old[l * BS + q] += out[0][q];
-          if (nt > 1) old[l * BS + q] += out[1][q];
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < BS * BS; ++q) dst[q] = old[q];
+    for (int q = 0; q < BS; ++q) {
+      if (nt > 0) old[l * BS + q] += out[0][q];
+      if (nt > 1) old[l * BS + q] += out[1][q];
     }
   }
-  if (Elem::HAS_VEC && j == 0) {
-    const int32_t vi = a.ep[e * CARD + i];
-    T fv[BS];
 #pragma unroll
-    for (int l = 0; l < BS; ++l) fv[l] = a.f[(int64_t)vi * BS + l];
-#pragma unroll
-    for (int l = 0; l < BS; ++l) {
-      T o[4];
-      const int nv = Elem::vec(a, e, i, l, o);
-      for (int q = 0; q < nv; ++q) fv[l] += o[q];
-    }
-#pragma unroll
-    for (int l = 0; l < BS; ++l) a.f[(int64_t)vi * BS + l] = fv[l];
-  }
+  for (int q = 0; q < BS * BS; ++q) dst[q] = old[q];
 }
 
 template <class Elem, int CARD, int BS, typename T>
 __global__ void __launch_bounds__(256) k_colored(AsmArgs<T> a, const uint32_t *__restrict__ elist,
                                                  int64_t cnt, const uint32_t *__restrict__ slots) {
-  constexpr int TPE = Elem::HAS_MAT ? CARD * CARD : CARD;  // threads per element
+  constexpr int TPE = CARD * CARD;  // threads per element
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < cnt * TPE; t += stride) {
     const int64_t e = elist[t / TPE];
     const int r = (int)(t % TPE);
-    const int i = Elem::HAS_MAT ? r / CARD : r, j = Elem::HAS_MAT ? r % CARD : 0;
+    const int i = r / CARD, j = r % CARD;
     const int32_t *vv = a.ep + e * CARD;
     bool rep = false;
 #pragma unroll
@@ -351,105 +323,21 @@ __global__ void __launch_bounds__(256) k_colored(AsmArgs<T> a, const uint32_t *_
   }
 }
 
-// Elements whose (j, i) block is bitwise the transpose of their (i, j)
-// block declare SYM = true; the element-blocks plan then computes and
-// stores only the CARD (CARD + 1) / 2 blocks with i <= j, in row order
-// (0,0), (0,1), .., (0,CARD-1), (1,1), .., and the slot gather reads the
-// transpose for i > j.
-template <class E, class = void> struct elem_sym : std::false_type {};
-template <class E>
-struct elem_sym<E, std::void_t<decltype(E::SYM)>> : std::integral_constant<bool, E::SYM> {};
-__device__ __forceinline__ void tri_pair(int C, int r, int &i, int &j) {
-  i = 0;
-  while (r >= C - i) {
-    r -= C - i;
-    ++i;
-  }
-  j = i + r;
-}
+// Place of pair (i, j) among the pairs of C vertices in row order.
 __device__ __forceinline__ int tri_index(int C, int i, int j) {  // i <= j
   return i * C - i * (i - 1) / 2 + (j - i);
 }
 
 // ---------------------------------------------------------------------------
-// Element blocks + slot gather (the assembly plan's second form)
+// Slot gather (the assembly plan's second form)
 // ---------------------------------------------------------------------------
-// Phase 1, element-parallel: thread (e, i, j) writes block (i, j) of element
-// e (all its terms summed) to eb[(e*CARD + i)*CARD + j] -- consecutive
-// threads, consecutive blocks, coalesced -- and for vector maps thread
-// (e, i, 0) writes vertex i's contribution to ev[e*CARD + i].  Phase 2:
-// every slot sums its contributing blocks (the inverse slot map, sorted by
-// block index, i.e. ascending element) and every vertex its contributions
-// (its incidence list, ascending element), each written once.  Each element
-// is computed once, nothing is read-modified-written, the order of every
-// sum is fixed.  Needs Elem::fin_* to be the identity.
-// TILE threads per CTA: the element tile is TILE / TPE elements (the
-// schedule the assembly tuner picks).
-template <class Elem, int CARD, int BS, typename T, int TILE>
-__global__ void __launch_bounds__(TILE) k_elem_blocks(AsmArgs<T> a, T *__restrict__ eb,
-                                                      T *__restrict__ ev) {
-  constexpr bool SY = elem_sym<Elem>::value;
-  static_assert(!SY || !Elem::HAS_VEC, "a symmetric element stores blocks only");
-  constexpr int TPE = Elem::HAS_MAT ? (SY ? CARD * (CARD + 1) / 2 : CARD * CARD) : CARD;
-  // a CTA's TILE consecutive blocks are staged in shared memory and leave in
-  // 16-byte stores (the chunk starts TILE * BS*BS * sizeof(T) bytes apart)
-  __shared__ __align__(16) T stage[Elem::HAS_MAT ? TILE * BS * BS : 1];
-  const int64_t total = a.nE * TPE;
-  for (int64_t t0 = (int64_t)blockIdx.x * TILE; t0 < total; t0 += (int64_t)gridDim.x * TILE) {
-    const int64_t t = t0 + threadIdx.x;
-    if (t < total) {
-      const int64_t e = t / TPE;
-      const int r = (int)(t % TPE);
-      int i = Elem::HAS_MAT ? r / CARD : r, j = Elem::HAS_MAT ? r % CARD : 0;
-      if (SY) tri_pair(CARD, r, i, j);
-      if (Elem::HAS_MAT) {
-#pragma unroll
-        for (int l = 0; l < BS; ++l) {
-          T out[2][BS];
-          const int nt = Elem::block(a, e, i, j, l, out);
-#pragma unroll
-          for (int q = 0; q < BS; ++q) {
-            T v = nt > 0 ? out[0][q] : T(0);
-            if (nt > 1) v += out[1][q];
-            stage[threadIdx.x * BS * BS + l * BS + q] = v;
-          }
-        }
-      }
-      if (Elem::HAS_VEC && j == 0) {
-#pragma unroll
-        for (int l = 0; l < BS; ++l) {
-          T o[4];
-          const int nv = Elem::vec(a, e, i, l, o);
-          T v = T(0);
-          for (int q = 0; q < nv; ++q) v += o[q];
-          ev[(e * CARD + i) * BS + l] = v;
-        }
-      }
-    }
-    if (Elem::HAS_MAT) {
-      __syncthreads();
-      const int64_t nval = (min(total, t0 + TILE) - t0) * BS * BS;
-      T *dst = eb + t0 * BS * BS;
-      constexpr int PER = 16 / sizeof(T);
-      if (nval == TILE * BS * BS && (BS * BS * TILE) % PER == 0) {
-        const float4 *src4 = reinterpret_cast<const float4 *>(stage);
-        float4 *dst4 = reinterpret_cast<float4 *>(dst);
-        for (int k = threadIdx.x; k < TILE * BS * BS / PER; k += TILE) dst4[k] = src4[k];
-      } else {
-        for (int64_t k = threadIdx.x; k < nval; k += TILE) dst[k] = stage[k];
-      }
-      __syncthreads();
-    }
-  }
-}
-
+// The assembly of caller-evaluated element blocks with the slot lists: every
+// slot sums its contributing blocks (the inverse slot map, sorted by block
+// index, i.e. ascending element), each written once, in a fixed order.
 // vals[q] = sum of eb blocks src[sptr[q] .. sptr[q+1]); thread per (slot,
 // row l); the block indices of up to 8 contributions are loaded before
 // their values, and all values before the sum (ascending order kept).
-// SC > 0: eb holds only the i <= j blocks of elements of SC endpoints
-// (elem_sym); a contribution b = e SC^2 + i SC + j with i > j reads block
-// (j, i) transposed.
-template <int BS, typename T, int SC = 0>
+template <int BS, typename T>
 __global__ void __launch_bounds__(256) k_slot_gather(int64_t nnzb, const uint32_t *__restrict__ sptr,
                                                      const uint32_t *__restrict__ src,
                                                      const T *__restrict__ eb, T *__restrict__ vals) {
@@ -467,19 +355,10 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t nnzb, const uint32_
       for (int u = 0; u < 8; ++u) b[u] = k0 + u < k1 ? src[k0 + u] : 0u;
       T x[8][BS];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        size_t blk = b[u];
-        bool tr = false;
-        if (SC > 0) {
-          const uint32_t e = b[u] / (SC * SC), rr = b[u] - e * (SC * SC);
-          const int i = (int)rr / SC, j = (int)rr % SC;
-          tr = i > j;
-          blk = (size_t)e * (SC * (SC + 1) / 2) + tri_index(SC, tr ? j : i, tr ? i : j);
-        }
+      for (int u = 0; u < 8; ++u)
 #pragma unroll
         for (int m = 0; m < BS; ++m)
-          x[u][m] = k0 + u < k1 ? eb[blk * BS * BS + (tr ? m * BS + l : l * BS + m)] : T(0);
-      }
+          x[u][m] = k0 + u < k1 ? eb[(size_t)b[u] * BS * BS + l * BS + m] : T(0);
 #pragma unroll
       for (int u = 0; u < 8; ++u)
         if (k0 + u < k1)
@@ -491,31 +370,12 @@ __global__ void __launch_bounds__(256) k_slot_gather(int64_t nnzb, const uint32_
   }
 }
 
-// f[v] = sum of ev over v's incidences (ascending element); thread per (v, l).
-template <int BS, typename T>
-__global__ void __launch_bounds__(256) k_vert_gather(int32_t n, const uint32_t *__restrict__ ve_ptr,
-                                                     const uint32_t *__restrict__ ve_idx,
-                                                     const T *__restrict__ ev, T *__restrict__ f) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < (int64_t)n * BS;
-       t += stride) {
-    const int64_t v = t / BS;
-    const int l = (int)(t % BS);
-    T acc = T(0);
-    const uint32_t k1 = ve_ptr[v + 1];
-    for (uint32_t k = ve_ptr[v]; k < k1; ++k) acc += ev[(size_t)ve_idx[k] * BS + l];
-    f[t] = acc;
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Springs (card 2, 3x3 blocks): compute_mass_damping + compute_elasticity of
 // apps/springs/isprings.sim:21-68 (form 0) and test/input/program/
 // isprings.sim (form 1); MDK = MD + K, f = fmg + fe.
 // ---------------------------------------------------------------------------
 template <typename T> struct SpringElem {
-  static constexpr bool HAS_MAT = true, HAS_VEC = true;
-  static constexpr int LANES = 6;
   // the spring's 3x3 k (row l) and fe0 (component l)
   __device__ static void kfe(const AsmArgs<T> &a, int64_t s, int l, T krow[3], T &fe0l) {
     const int32_t e0 = a.ep[2 * s], e1 = a.ep[2 * s + 1];
@@ -555,27 +415,6 @@ template <typename T> struct SpringElem {
       }
     }
   }
-  __device__ static int block(const AsmArgs<T> &a, int64_t s, int i, int j, int l,
-                             T out[2][3]) {
-    const bool f0 = a.fixed[a.ep[2 * s]] != 0, f1 = a.fixed[a.ep[2 * s + 1]] != 0;
-    bool write;
-    if (!f0 && !f1) write = true;
-    else write = (i == j) && ((i == 0) ? !f0 : !f1);
-    if (!write) return 0;
-    T kr[3], fe;
-    kfe(a, s, l, kr, fe);
-    const bool neg = (i != j);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) out[0][q] = neg ? -kr[q] : kr[q];
-    return 1;
-  }
-  __device__ static int vec(const AsmArgs<T> &a, int64_t s, int i, int l, T out[4]) {
-    if (a.fixed[a.ep[2 * s + i]]) return 0;
-    T kr[3], fe;
-    kfe(a, s, l, kr, fe);
-    out[0] = (i == 0) ? fe : -fe;
-    return 1;
-  }
   // MD(p,p): fixed -> only entry (0,0) = 1 (a scalar written to a block);
   // else (mass + h*viscous) * I.  MDK = MD + K (MD is the first operand).
   __device__ static T fin_block(const AsmArgs<T> &a, int32_t p, bool dg, int l, int m, T acc) {
@@ -598,55 +437,9 @@ template <typename T> struct SpringElem {
 // I; A = diag*I + scale*K (the lowered matrix expression: diagonal first).
 // ---------------------------------------------------------------------------
 template <typename T> struct ScalarSpringElem {
-  static constexpr bool HAS_MAT = true, HAS_VEC = false;
-  static constexpr int LANES = 2;
-  __device__ static int block(const AsmArgs<T> &a, int64_t s, int i, int j, int, T out[2][1]) {
-    out[0][0] = (i == j) ? a.a[s] : -a.a[s];
-    return 1;
-  }
-  __device__ static int vec(const AsmArgs<T> &, int64_t, int, int, T *) { return 0; }
   __device__ static T fin_block(const AsmArgs<T> &a, int32_t, bool dg, int, int, T acc) {
     return dg ? a.diag + (a.scale * acc) : T(0) + (a.scale * acc);
   }
-  __device__ static T fin_vec(const AsmArgs<T> &, int32_t, int, T acc) { return acc; }
-};
-
-// ---------------------------------------------------------------------------
-// P1 heat (scalar): A_ij = W/20 (1 + δij) + (dt*kappa*W) (g_i . g_j),
-// b_i = Σ_j W/20 (1 + δij) T0_j.  g_i = row i of B, g_3 = -(g_0+g_1+g_2).
-// ---------------------------------------------------------------------------
-template <typename T> struct HeatElem {
-  static constexpr bool HAS_MAT = true, HAS_VEC = true;
-  static constexpr int LANES = 4;
-  __device__ static void grad(const T *Bt, int i, T g[3]) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-      g[d] = (i < 3) ? Bt[i * 3 + d] : -((Bt[0 * 3 + d] + Bt[1 * 3 + d]) + Bt[2 * 3 + d]);
-  }
-  __device__ static int block(const AsmArgs<T> &a, int64_t t, int i, int j, int, T out[2][1]) {
-    const T *Bt = a.B + 9 * t;
-    T gi[3], gj[3];
-    grad(Bt, i, gi);
-    grad(Bt, j, gj);
-    const T mw = a.W[t] / T(20.0);
-    const T kw = (a.dt * a.kappa[t]) * a.W[t];
-    const T mij = (i == j) ? T(2.0) * mw : mw;
-    const T gg = (gi[0] * gj[0] + gi[1] * gj[1]) + gi[2] * gj[2];
-    out[0][0] = mij + kw * gg;
-    return 1;
-  }
-  __device__ static int vec(const AsmArgs<T> &a, int64_t t, int i, int, T out[4]) {
-    const T mw = a.W[t] / T(20.0);
-    T bi = 0;
-    for (int j = 0; j < 4; ++j) {
-      const T mij = (i == j) ? T(2.0) * mw : mw;
-      bi += mij * a.T0[a.ep[4 * t + j]];
-    }
-    out[0] = bi;
-    return 1;
-  }
-  __device__ static T fin_block(const AsmArgs<T> &, int32_t, bool, int, int, T acc) { return acc; }
-  __device__ static T fin_vec(const AsmArgs<T> &, int32_t, int, T acc) { return acc; }
 };
 
 // Vertex mass of precomputeTetMat: m(v) += (0.25*rho)*W in element order.
@@ -822,27 +615,20 @@ template <typename T> struct EbGatherElem {
 };
 
 // fem_linear.sim:105-174: Ke = ((W * Bm') * E) * Bm with Voigt E and the
-// strain-displacement Bm built from dN, in that operation order (EXACT), or
-// the algebraically equal closed form (fast):
-//   K_ij[a][b] = W (lam g_ia g_jb + mu g_ib g_ja + mu (g_i . g_j) δab).
+// strain-displacement Bm built from dN, in that operation order.
 // K(v(i), v(j)) += h*h*K_ij when both vertices are free; then m*I on (i, i).
-template <typename T, bool EXACT> struct LinTetElem {
+template <typename T> struct LinTetElem {
   static constexpr bool HAS_MAT = true, HAS_VEC = false;
-  // the fast form's (j, i) block is bitwise the transpose of (i, j)
-  static constexpr bool SYM = !EXACT;
   static constexpr int LANES = 12;
-  __device__ static void dN(const T *Bt, int vi, T g[3]) {
+  // column r (0..11) of Bm: 6 entries
+  __device__ static void bm_col(const T *Bt, int r, T col[6]) {
+    const int vi = r / 3, di = r % 3;
+    T g[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       if (vi < 3) g[d] = Bt[vi * 3 + d];
       else g[d] = ((T(0) - Bt[0 * 3 + d]) - Bt[1 * 3 + d]) - Bt[2 * 3 + d];
     }
-  }
-  // column r (0..11) of Bm: 6 entries
-  __device__ static void bm_col(const T *Bt, int r, T col[6]) {
-    const int vi = r / 3, di = r % 3;
-    T g[3];
-    dN(Bt, vi, g);
 #pragma unroll
     for (int k = 0; k < 6; ++k) col[k] = T(0);
     col[di] = g[di];
@@ -855,58 +641,33 @@ template <typename T, bool EXACT> struct LinTetElem {
     const bool both = a.c[vv[i]] <= 0 && a.c[vv[j]] <= 0;
     const T *Bt = a.B + 9 * t;
     const T W = a.W[t], u = a.mu[t], lm = a.lam[t];
-    T k3[3] = {T(0), T(0), T(0)};
-    if (both) {
-      if (EXACT) {
-        // E(c, a): l off-diagonal in the 3x3 normal part, l+2u on it, u shear
-        T cr[6];
-        bm_col(Bt, 3 * i + l, cr);
-        T Trow[6];
-#pragma unroll
-        for (int ac = 0; ac < 6; ++ac) {
-          T s = 0;
-#pragma unroll
-          for (int k = 0; k < 6; ++k) {
-            T Eka;
-            if (k < 3 && ac < 3) Eka = (k == ac) ? lm + T(2.0) * u : lm;
-            else Eka = (k == ac) ? u : T(0);
-            s += (W * cr[k]) * Eka;
-          }
-          Trow[ac] = s;
-        }
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          T cc[6];
-          bm_col(Bt, 3 * j + m, cc);
-          T s = 0;
-#pragma unroll
-          for (int k = 0; k < 6; ++k) s += Trow[k] * cc[k];
-          k3[m] = (a.h * a.h) * s;
-        }
-      } else {
-        // Every product pairs one factor of vertex i with one of vertex j and
-        // no operation is contracted, so the (j, i) block is bitwise the
-        // transpose of the (i, j) block and the assembled matrix is exactly
-        // symmetric (the symmetric-storage SpMV reads only its upper half).
-        T gi[3], gj[3];
-        dN(Bt, i, gi);
-        dN(Bt, j, gj);
-        const T gij =
-            add_rn(add_rn(mul_rn(gi[0], gj[0]), mul_rn(gi[1], gj[1])), mul_rn(gi[2], gj[2]));
-        const T hw = mul_rn(mul_rn(a.h, a.h), W);
-        const T ug = mul_rn(u, gij);
-#pragma unroll
-        for (int m = 0; m < 3; ++m) {
-          T t = add_rn(mul_rn(lm, mul_rn(gi[l], gj[m])), mul_rn(u, mul_rn(gi[m], gj[l])));
-          if (l == m) t = add_rn(t, ug);
-          k3[m] = mul_rn(hw, t);
-        }
-      }
-    }
     int nt = 0;
     if (both) {
+      // E(c, a): l off-diagonal in the 3x3 normal part, l+2u on it, u shear
+      T cr[6];
+      bm_col(Bt, 3 * i + l, cr);
+      T Trow[6];
 #pragma unroll
-      for (int m = 0; m < 3; ++m) out[0][m] = k3[m];
+      for (int ac = 0; ac < 6; ++ac) {
+        T s = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+          T Eka;
+          if (k < 3 && ac < 3) Eka = (k == ac) ? lm + T(2.0) * u : lm;
+          else Eka = (k == ac) ? u : T(0);
+          s += (W * cr[k]) * Eka;
+        }
+        Trow[ac] = s;
+      }
+#pragma unroll
+      for (int m = 0; m < 3; ++m) {
+        T cc[6];
+        bm_col(Bt, 3 * j + m, cc);
+        T s = 0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) s += Trow[k] * cc[k];
+        out[0][m] = (a.h * a.h) * s;
+      }
       nt = 1;
     }
     if (i == j) {

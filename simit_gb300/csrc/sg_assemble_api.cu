@@ -113,7 +113,7 @@ int sg_assemble_tet_stiffness(sg_ctx *h, const sg_mesh *m, int dt, int model, co
   SG_REQUIRE(model == SG_MODEL_LINEAR || x, "sg_assemble_tet_stiffness: x is null");
   void *eb = nullptr;
   Scratch s(c);
-  if (model == SG_MODEL_NEOHOOKEAN) {
+  if (model == SG_MODEL_NEOHOOKEAN && exact) {
     const size_t bytes = (size_t)m->nE * 144 * dtype_size(dt);
     SG_TRY(s.reserve(bytes + 256));
     eb = s.alloc<char>(bytes);

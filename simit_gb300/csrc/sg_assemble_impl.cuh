@@ -3,6 +3,7 @@
 // (default contraction, namespace sg::fast); SG_ASM_NS names the namespace
 // and SG_ASM_EXACT selects the operation-order-exact element forms.
 #include "sg_assemble.cuh"
+#include "sg_assemble_tile.cuh"
 #include "sg_internal.cuh"
 #include "sg_asm_api.h"
 
@@ -30,62 +31,82 @@ static int launch_rows(Ctx *c, AsmArgs<T> &a) {
   return SG_OK;
 }
 
-// The element-parallel form over the mesh's colouring plan (fast
-// instantiation only; the exact one keeps the reference's element order
-// through the row owners).  Outputs are zeroed first, then one launch per
-// colour.  Returns 1 through *used when it ran.
-template <class Elem, int CARD, int BS, typename T>
-static int launch_colored(Ctx *c, AsmArgs<T> &a, const sg_mesh *m, bool *used) {
+// Row tiles (sg_assemble_tile.cuh).  Rows a tile: 32, halved while the tiles
+// are fewer than two an SM or their buffers exceed half of an SM's shared
+// memory.  The buffers hold 15 % more than the mesh's average, and a record
+// for three in four incidences (0.51 of them are distinct elements on a
+// Morton-ordered five-tet lattice, 0.65 in lattice order); a tile that needs
+// more is taken in parts.
+template <class E, typename T>
+static int launch_tile(Ctx *c, AsmArgs<T> &a, const sg_mesh *m) {
+  if (a.n == 0) return SG_OK;
+  const bool plan = m->slots && ((m->slot_src_ptr && m->slot_src) ||
+                                 (m->color_order && m->color_ptr && m->ncolors > 0));
+  TileCfg g;
+  g.maxrow = plan ? INT32_MAX : a.maxrow;
+  if (E::HAS_MAT && !plan && (size_t)a.maxrow * (E::BS * E::BS * sizeof(T) + 4) > 96 * 1024)
+    return set_error(SG_ERR_UNSUPPORTED, "assembly: a row of %d blocks exceeds shared memory",
+                     a.maxrow);
+  // with the slot lists a block's mass joins its stiffness before the slot's
+  // sum, as the caller-evaluated blocks of that plan come summed
+  g.pre = m->slots && m->slot_src_ptr && m->slot_src;
+  g.slots = m->slots;
+  g.ep16 = (uintptr_t)a.ep % 16 == 0 && (uintptr_t)m->slots % 16 == 0;
+  for (g.step = 1; g.step * 2 <= (plan ? 254 : a.maxrow) && g.step < 128;) g.step *= 2;
+  const double inc = (double)a.nE * E::CARD / a.n, len = (double)a.nnzb / a.n;
+  size_t sh = 0;
+  for (g.rows = TILE_MAXROWS;; g.rows >>= 1) {
+    g.icap = (int)(g.rows * inc * 1.15) + 32;
+    if (g.icap > 32768) g.icap = 32768;
+    g.ucap = (int)(g.icap * (g.rows >= 32 ? 0.75 : 0.9));
+    g.scap = (int)(g.rows * len * 1.15) + 32;
+    if (g.scap > 32768) g.scap = 32768;
+    g.mcap = g.scap * (inc > 32 ? 3 : 1) + 64;
+    for (g.hcap = 64; g.hcap < g.ucap + g.ucap / 4; g.hcap *= 2) {}
+    sh = tile_smem<E, T>(g);
+    const bool small = a.n < (int64_t)g.rows * 2 * c->num_sms;
+    if (g.rows <= 4 || (!small && sh <= 112 * 1024)) break;
+  }
+  if (sh > 220 * 1024) {  // a few rows already exceed an SM: the row-by-row path
+    g.icap = g.ucap = g.scap = g.mcap = 64;
+    g.hcap = 128;
+    sh = tile_smem<E, T>(g);
+  }
+  if (sh > 44 * 1024)  // (with the kernel's static tables, past the default limit)
+    SG_CHECK_CUDA(cudaFuncSetAttribute(k_tile<E, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)sh));
+  a.err = c->d_err;
+  k_tile<E, T><<<(a.n + g.rows - 1) / g.rows, TILE_T, sh, c->stream>>>(a, g);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
+}
+
+// Caller-evaluated element blocks over the mesh's plan (fast instantiation
+// only; the exact one keeps the reference's element order through the row
+// owners): a gather by slot, or the blocks of one colour after another into
+// cleared values.  Sets *used when it ran.
+template <int BS, int CARD, typename T>
+static int launch_plan(Ctx *c, AsmArgs<T> &a, const sg_mesh *m, bool *used) {
   *used = false;
-  if (SG_ASM_EXACT || !m->slots || m->card != CARD) return SG_OK;
+  if (SG_ASM_EXACT || !m->slots) return SG_OK;
   a.err = c->d_err;
   if (m->slot_src_ptr && m->slot_src) {
-    // element blocks (context scratch) + slot / vertex gathers
-    constexpr bool SY = elem_sym<Elem>::value;
-    constexpr int BPE = SY ? CARD * (CARD + 1) / 2 : CARD * CARD;  // stored blocks per element
-    const size_t neb = Elem::HAS_MAT ? (size_t)m->nE * BPE * BS * BS : 0;
-    const size_t nev = Elem::HAS_VEC ? (size_t)m->nE * CARD * BS : 0;
-    Scratch s(c);
-    SG_TRY(s.reserve(Scratch::bytes_for(neb + 1, sizeof(T)) + Scratch::bytes_for(nev + 1, sizeof(T))));
-    T *eb = s.alloc<T>(neb + 1), *ev = s.alloc<T>(nev + 1);
-    if (m->nE > 0) {
-      const int64_t th = m->nE * (Elem::HAS_MAT ? BPE : CARD);
-      const int tile = m->asm_tile;
-      if (tile == 128)
-        k_elem_blocks<Elem, CARD, BS, T, 128><<<grid_for(c, th, 128, 16), 128, 0, c->stream>>>(
-            a, eb, ev);
-      else if (tile == 512)
-        k_elem_blocks<Elem, CARD, BS, T, 512><<<grid_for(c, th, 512, 4), 512, 0, c->stream>>>(
-            a, eb, ev);
-      else
-        k_elem_blocks<Elem, CARD, BS, T, 256><<<grid_for(c, th, 256, 8), 256, 0, c->stream>>>(
-            a, eb, ev);
-      SG_CHECK_LAUNCH();
-    }
-    if (Elem::HAS_MAT && m->nnzb > 0) {
-      k_slot_gather<BS, T, SY ? CARD : 0><<<grid_for(c, m->nnzb * BS, 256, 8), 256, 0, c->stream>>>(
-          m->nnzb, m->slot_src_ptr, m->slot_src, eb, a.vals);
-      SG_CHECK_LAUNCH();
-    }
-    if (Elem::HAS_VEC && m->n > 0) {
-      k_vert_gather<BS, T><<<grid_for(c, (int64_t)m->n * BS, 256, 8), 256, 0, c->stream>>>(
-          m->n, m->ve_ptr, m->ve_idx, ev, a.f);
+    if (m->nnzb > 0) {
+      k_slot_gather<BS, T><<<grid_for(c, m->nnzb * BS, 256, 8), 256, 0, c->stream>>>(
+          m->nnzb, m->slot_src_ptr, m->slot_src, a.eb, a.vals);
       SG_CHECK_LAUNCH();
     }
     *used = true;
     return SG_OK;
   }
   if (!m->color_order || !m->color_ptr || m->ncolors <= 0) return SG_OK;
-  if (Elem::HAS_MAT)
-    SG_CHECK_CUDA(cudaMemsetAsync(a.vals, 0, (size_t)m->nnzb * BS * BS * sizeof(T), c->stream));
-  if (Elem::HAS_VEC)
-    SG_CHECK_CUDA(cudaMemsetAsync(a.f, 0, (size_t)m->n * BS * sizeof(T), c->stream));
+  SG_CHECK_CUDA(cudaMemsetAsync(a.vals, 0, (size_t)m->nnzb * BS * BS * sizeof(T), c->stream));
   for (int k = 0; k < m->ncolors; ++k) {
     const int64_t b0 = m->color_ptr[k], cnt = (int64_t)m->color_ptr[k + 1] - b0;
     if (cnt <= 0) continue;
-    const int64_t threads = cnt * (Elem::HAS_MAT ? CARD * CARD : CARD);
-    k_colored<Elem, CARD, BS, T><<<grid_for(c, threads, 256, 8), 256, 0, c->stream>>>(
-        a, m->color_order + b0, cnt, m->slots);
+    k_colored<BlocksElem<T, BS, CARD>, CARD, BS, T>
+        <<<grid_for(c, cnt * CARD * CARD, 256, 8), 256, 0, c->stream>>>(a, m->color_order + b0,
+                                                                        cnt, m->slots);
     SG_CHECK_LAUNCH();
   }
   *used = true;
@@ -117,7 +138,7 @@ int springs(Ctx *c, const sg_mesh *m, int form, const void *x, const void *v, co
   for (int q = 0; q < 3; ++q) a.grav[q] = (T)grav[q];
   a.form = form;
   a.vals = (T *)vals; a.f = (T *)f;
-  return launch_rows<SpringElem<T>, 8, 3, T>(c, a);
+  return launch_tile<SpringTile<T>, T>(c, a, m);
 }
 
 template <typename T>
@@ -126,7 +147,7 @@ int scalar_springs(Ctx *c, const sg_mesh *m, const void *av, double diag, double
   AsmArgs<T> a;
   fill_mesh(a, m);
   a.a = (const T *)av; a.diag = (T)diag; a.scale = (T)scale; a.vals = (T *)vals;
-  return launch_rows<ScalarSpringElem<T>, 2, 1, T>(c, a);
+  return launch_tile<ScalarSpringTile<T>, T>(c, a, m);
 }
 
 template <typename T>
@@ -136,10 +157,7 @@ int heat(Ctx *c, const sg_mesh *m, const void *B, const void *W, const void *kap
   fill_mesh(a, m);
   a.B = (const T *)B; a.W = (const T *)W; a.kappa = (const T *)kappa; a.dt = (T)dt;
   a.T0 = (const T *)T0; a.vals = (T *)vals; a.f = (T *)b;
-  bool used = false;
-  SG_TRY((launch_colored<HeatElem<T>, 4, 1, T>(c, a, m, &used)));
-  if (used) return SG_OK;
-  return launch_rows<HeatElem<T>, 4, 1, T>(c, a);
+  return launch_tile<HeatTile<T, SG_ASM_EXACT>, T>(c, a, m);
 }
 
 template <typename T>
@@ -165,7 +183,7 @@ int blocks(Ctx *c, const sg_mesh *m, int bs, const void *eb, void *vals) {
 #define SG_BLK(BSV, CV)                                                            \
   if (bs == BSV && m->card == CV) {                                                \
     bool used = false;                                                             \
-    SG_TRY((launch_colored<BlocksElem<T, BSV, CV>, CV, BSV, T>(c, a, m, &used)));  \
+    SG_TRY((launch_plan<BSV, CV, T>(c, a, m, &used)));                             \
     if (used) return SG_OK;                                                        \
     return launch_rows<BlocksElem<T, BSV, CV>, 16, BSV, T>(c, a);                  \
   }
@@ -186,21 +204,18 @@ int tet_stiffness(Ctx *c, const sg_mesh *m, int model, const void *x, const int3
   a.x = (const T *)x; a.c = cons; a.B = (const T *)B; a.W = (const T *)W;
   a.mu = (const T *)mu; a.lam = (const T *)lam; a.h = (T)h; a.rho = (T)rho;
   a.vals = (T *)vals;
+  if (!SG_ASM_EXACT)
+    return model == SG_MODEL_NEOHOOKEAN ? launch_tile<NeoTile<T>, T>(c, a, m)
+                                        : launch_tile<LinTetTile<T>, T>(c, a, m);
   if (model == SG_MODEL_NEOHOOKEAN) {
     a.eb = (const T *)eb_scratch;
     if (m->nE > 0) {
       k_neo_blocks<T><<<grid_for(c, m->nE, 128, 16), 128, 0, c->stream>>>(a);
       SG_CHECK_LAUNCH();
     }
-    bool used = false;
-    SG_TRY((launch_colored<EbGatherElem<T>, 4, 3, T>(c, a, m, &used)));
-    if (used) return SG_OK;
     return launch_rows<EbGatherElem<T>, 16, 3, T>(c, a);
   }
-  bool used = false;
-  SG_TRY((launch_colored<LinTetElem<T, SG_ASM_EXACT>, 4, 3, T>(c, a, m, &used)));
-  if (used) return SG_OK;
-  return launch_rows<LinTetElem<T, SG_ASM_EXACT>, 16, 3, T>(c, a);
+  return launch_rows<LinTetElem<T>, 16, 3, T>(c, a);
 }
 
 template <typename T>
@@ -213,14 +228,10 @@ int tet_force(Ctx *c, const sg_mesh *m, int model, const void *x, const void *v,
   a.mu = (const T *)mu; a.lam = (const T *)lam; a.h = (T)h; a.rho = (T)rho;
   for (int q = 0; q < 3; ++q) a.grav[q] = (T)grav[q];
   a.f = (T *)f;
-  bool used = false;
-  if (model == SG_MODEL_NEOHOOKEAN) {
-    SG_TRY((launch_colored<TetForceElem<T, true>, 4, 3, T>(c, a, m, &used)));
-    if (used) return SG_OK;
-    return launch_rows<TetForceElem<T, true>, 4, 3, T>(c, a);
-  }
-  SG_TRY((launch_colored<TetForceElem<T, false>, 4, 3, T>(c, a, m, &used)));
-  if (used) return SG_OK;
+  if (!SG_ASM_EXACT)
+    return model == SG_MODEL_NEOHOOKEAN ? launch_tile<TetForceTile<T, true>, T>(c, a, m)
+                                        : launch_tile<TetForceTile<T, false>, T>(c, a, m);
+  if (model == SG_MODEL_NEOHOOKEAN) return launch_rows<TetForceElem<T, true>, 4, 3, T>(c, a);
   return launch_rows<TetForceElem<T, false>, 4, 3, T>(c, a);
 }
 

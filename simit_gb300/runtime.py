@@ -406,11 +406,12 @@ _ASM_TUNE_CACHE = {}
 class Mesh:
     """A bound edge set + its device pattern, as the sg_mesh structure.
 
-    plan: the element-parallel assembly plan that assembly with exact=False
-    uses -- "gather" (element blocks written once, then every slot and
-    vertex gathers its contributions in ascending element order), "colored"
-    (blocks added into their slots colour by colour) -- or None (row-owner
-    kernels).  colored=True is plan="colored"."""
+    plan: what assembly with exact=False has beside the pattern -- "gather"
+    (the slots and each slot's element blocks in ascending element order),
+    "colored" (the slots and an element colouring) -- or None.  The built-in
+    maps read the slots of either (without one they search the rows);
+    assemble_blocks gathers by slot or adds colour by colour.
+    colored=True is plan="colored"."""
 
     def __init__(self, ctx, n, endpoints, card, with_slots=False, colored=False, plan=None):
         self.ctx = ctx
@@ -464,7 +465,7 @@ class Mesh:
         self.s.slot_src = self.slot_src.data_ptr()
 
     def set_asm_tile(self, tile):
-        """Element tile (threads per CTA) of the element-blocks plan."""
+        """sg_mesh.asm_tile (no kernel reads it)."""
         assert tile in (0, 128, 256, 512)
         self.s.asm_tile = int(tile)
 
@@ -538,6 +539,15 @@ class Mesh:
         with self.ctx.stream():
             return torch.zeros(max(1, count), dtype=dtype, device=self.ctx.device)
 
+    def _out(self, count, dtype):
+        """An array the assembly kernels write in full (every slot of every
+        row, every vertex): not cleared, which at 128^3 in FP32 is 0.13 ms of
+        a stiffness map."""
+        if count == 0:
+            return self.empty(count, dtype)
+        with self.ctx.stream():
+            return torch.empty(count, dtype=dtype, device=self.ctx.device)
+
 
 def _d(t, dtype, dev):
     if t is None:
@@ -553,8 +563,8 @@ def assemble_springs(mesh, x, v, m, fixed, k, l0, h, viscous, grav, form=0,
         d = mesh.ctx.device
         x, v, m, k, l0 = (_d(a, dtype, d) for a in (x, v, m, k, l0))
         fixed = _d(fixed, torch.uint8, d)
-        vals = mesh.empty(mesh.nnzb * 9, dtype)
-        f = mesh.empty(mesh.n * 3, dtype)
+        vals = mesh._out(mesh.nnzb * 9, dtype)
+        f = mesh._out(mesh.n * 3, dtype)
         call("sg_assemble_springs", mesh.ctx.h, mesh.ref(), dtype_code(vals), form, ptr(x), ptr(v),
              ptr(m), ptr(fixed), ptr(k), ptr(l0), h, viscous, _host_f64(grav), ptr(vals), ptr(f),
              int(exact))
@@ -564,7 +574,7 @@ def assemble_springs(mesh, x, v, m, fixed, k, l0, h, viscous, grav, form=0,
 def assemble_scalar_springs(mesh, a, diag, scale, dtype=torch.float64, exact=True):
     with mesh.ctx.stream():
         a = _d(a, dtype, mesh.ctx.device)
-        vals = mesh.empty(mesh.nnzb, dtype)
+        vals = mesh._out(mesh.nnzb, dtype)
         call("sg_assemble_scalar_springs", mesh.ctx.h, mesh.ref(), dtype_code(vals), ptr(a), diag,
              scale, ptr(vals), int(exact))
         return vals
@@ -606,7 +616,7 @@ def assemble_blocks(mesh, eb, bs, dtype=torch.float64, exact=True):
     [nE, card, card, bs, bs] into the mesh's pattern (values [nnzb*bs*bs])."""
     with mesh.ctx.stream():
         eb = _d(eb, dtype, mesh.ctx.device).contiguous()
-        vals = mesh.empty(mesh.nnzb * bs * bs, dtype)
+        vals = mesh._out(mesh.nnzb * bs * bs, dtype)
         call("sg_assemble_blocks", mesh.ctx.h, mesh.ref(), dtype_code(vals), int(bs), ptr(eb),
              ptr(vals), int(exact))
         return vals
@@ -615,9 +625,9 @@ def assemble_blocks(mesh, eb, bs, dtype=torch.float64, exact=True):
 def tet_precompute(mesh, x, rho, dtype=torch.float64):
     with mesh.ctx.stream():
         x = _d(x, dtype, mesh.ctx.device)
-        B = mesh.empty(mesh.nE * 9, dtype)
-        W = mesh.empty(mesh.nE, dtype)
-        m = mesh.empty(mesh.n, dtype)
+        B = mesh._out(mesh.nE * 9, dtype)
+        W = mesh._out(mesh.nE, dtype)
+        m = mesh._out(mesh.n, dtype)
         call("sg_tet_precompute", mesh.ctx.h, mesh.ref(), dtype_code(B), ptr(x), rho, ptr(B), ptr(W),
              ptr(m))
         return B, W, m
@@ -629,7 +639,7 @@ def assemble_tet_stiffness(mesh, model, x, c, B, W, mu, lam, h, rho, dtype=torch
         d = mesh.ctx.device
         x, B, W, mu, lam = (_d(a, dtype, d) for a in (x, B, W, mu, lam))
         c = _d(c, torch.int32, d)
-        vals = mesh.empty(mesh.nnzb * 9, dtype)
+        vals = mesh._out(mesh.nnzb * 9, dtype)
         call("sg_assemble_tet_stiffness", mesh.ctx.h, mesh.ref(), dtype_code(vals), model, ptr(x),
              ptr(c), ptr(B), ptr(W), ptr(mu), ptr(lam), h, rho, ptr(vals), int(exact))
         return vals
@@ -641,7 +651,7 @@ def assemble_tet_force(mesh, model, x, v, c, B, W, mu, lam, h, rho, grav, dtype=
         d = mesh.ctx.device
         x, v, B, W, mu, lam = (_d(a, dtype, d) for a in (x, v, B, W, mu, lam))
         c = _d(c, torch.int32, d)
-        f = mesh.empty(mesh.n * 3, dtype)
+        f = mesh._out(mesh.n * 3, dtype)
         call("sg_assemble_tet_force", mesh.ctx.h, mesh.ref(), dtype_code(f), model, ptr(x), ptr(v),
              ptr(c), ptr(B), ptr(W), ptr(mu), ptr(lam), h, rho, _host_f64(grav), ptr(f), int(exact))
         return f
@@ -651,8 +661,8 @@ def assemble_heat(mesh, B, W, kappa, dt, T0, dtype=torch.float64, exact=True):
     with mesh.ctx.stream():
         d = mesh.ctx.device
         B, W, kappa, T0 = (_d(a, dtype, d) for a in (B, W, kappa, T0))
-        vals = mesh.empty(mesh.nnzb, dtype)
-        b = mesh.empty(mesh.n, dtype)
+        vals = mesh._out(mesh.nnzb, dtype)
+        b = mesh._out(mesh.n, dtype)
         call("sg_assemble_heat", mesh.ctx.h, mesh.ref(), dtype_code(vals), ptr(B), ptr(W), ptr(kappa),
              dt, ptr(T0), ptr(vals), ptr(b), int(exact))
         return vals, b

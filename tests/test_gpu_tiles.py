@@ -1,0 +1,150 @@
+"""GPU checks of the row-tile assembly at the sizes where it changes path:
+rows longer than a tile can address, rows of more than one mask word, meshes
+whose numbering shares few elements between neighbouring rows (a tile taken
+in parts), elements that list a vertex twice, vertices without elements, and
+meshes of fewer rows than a tile.  Exact mode against the oracle bit for
+bit; the contracted kernels within 1e-12 of the largest value in FP64 and
+1e-5 in FP32 (about 300 terms a sum at most, each rounded a few times)."""
+import numpy as np
+import pytest
+import torch
+
+from simit_gb300 import _lib, meshgen
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(gpu_ctx):
+    return gpu_ctx
+
+
+def _np(t):
+    return t.detach().cpu().numpy()
+
+
+def _springs(kind):
+    """(n, endpoints): hub = vertex 0 in 400 springs (a row past 8-bit
+    positions) and vertex 1 in 90 (three mask words); random = every second
+    vertex unused; tiny = one spring."""
+    g = meshgen.rng(21)
+    if kind == "tiny":
+        return 2, np.array([[1, 0]])
+    if kind == "random":
+        return 700, 2 * g.integers(0, 350, size=(2500, 2))
+    hub = np.stack([np.zeros(400, int), 2 + np.arange(400)], 1)
+    two = np.stack([2 + g.permutation(400)[:90], np.ones(90, int)], 1)
+    ep = np.concatenate([hub, two, g.integers(2, 402, size=(300, 2))])
+    return 402, ep[g.permutation(len(ep))]
+
+
+@pytest.mark.parametrize("kind", ["tiny", "random", "hub"])
+@pytest.mark.parametrize("form", [0, 1])
+def test_springs(ctx, oracle, kind, form):
+    from simit_gb300.runtime import Mesh, assemble_springs
+    n, ep = _springs(kind)
+    ep = ep[ep[:, 0] != ep[:, 1]]
+    # the oracle wants every vertex in some element (a diagonal block each)
+    used, ep = np.unique(ep, return_inverse=True)
+    n, ep = len(used), ep.reshape(-1, 2)
+    g = meshgen.rng(5)
+    x, v = g.normal(size=n * 3), g.normal(size=n * 3)
+    m, k = g.uniform(1, 2, n), g.uniform(10, 20, len(ep))
+    l0 = g.uniform(0.5, 1, len(ep))
+    fixed = (g.uniform(size=n) < 0.2).astype(np.uint8)
+    grav = np.array([0.1, 0.2, -9.81])
+    mesh = Mesh(ctx, n, ep.astype(np.int32).reshape(-1), 2)
+    rp, ci = mesh.pattern.host()
+    oA, of = oracle.springs_assemble(form, x, v, m, fixed, mesh.pattern.endpoints.cpu().numpy(),
+                                     k, l0, 0.01, 0.1, grav, rp, ci)
+    A, f = assemble_springs(mesh, x, v, m, fixed, k, l0, 0.01, 0.1, grav, form=form)
+    ctx.sync()
+    assert np.array_equal(_np(A), oA) and np.array_equal(_np(f), of)
+    A, f = assemble_springs(mesh, x, v, m, fixed, k, l0, 0.01, 0.1, grav, form=form,
+                            dtype=torch.float32, exact=False)
+    ctx.sync()
+    assert np.abs(_np(A) - oA).max() <= 1e-5 * np.abs(oA).max()
+    assert np.abs(_np(f) - of).max() <= 1e-5 * np.abs(of).max()
+
+
+@pytest.mark.parametrize("kind", ["tiny", "random", "hub"])
+def test_repeated_endpoints(ctx, kind):
+    """Scalar springs, some of them from a vertex to itself, against the
+    same blocks through the row owners, bit for bit."""
+    from simit_gb300.runtime import Mesh, assemble_blocks, assemble_scalar_springs
+    n, ep = _springs(kind)
+    ep = ep.copy()
+    ep[::5, 1] = ep[::5, 0]
+    a = meshgen.rng(6).normal(size=len(ep))
+    eb = np.stack([a, -a, -a, a], 1)
+    mesh = Mesh(ctx, n, ep.astype(np.int32).reshape(-1), 2)
+    ref = assemble_blocks(mesh, eb, 1, exact=True)
+    got = assemble_scalar_springs(mesh, a, 0.0, 1.0)
+    ctx.sync()
+    assert torch.equal(got, ref)
+
+
+def _tets(kind):
+    """(positions [n, 3], tets): lattice, its vertices renumbered at random
+    (with elements in random order too), or a fan of tetrahedra around one
+    edge (two vertices in 130 elements, rows of 132 blocks)."""
+    g = meshgen.rng(8)
+    if kind == "fan":
+        t = np.linspace(0, 2 * np.pi, 131)[:-1]
+        ring = np.stack([np.cos(t), np.sin(t), 0.1 * np.sin(7 * t)], 1)
+        X = np.concatenate([[[0, 0, -1.0], [0, 0, 1.0]], ring])
+        k = np.arange(130)
+        T = np.stack([np.zeros(130, int), np.ones(130, int), 2 + k, 2 + (k + 1) % 130], 1)
+    else:
+        mg = meshgen.tet_grid(9, 8, 7)
+        X, T = mg["X0"].reshape(-1, 3), mg["tets"].reshape(-1, 4).astype(int)
+        if kind == "random":
+            new = g.permutation(len(X))
+            Y = np.empty_like(X)
+            Y[new] = X
+            X, T = Y, new[T][g.permutation(len(T))]
+    d = X[T[:, :3]] - X[T[:, 3:]]
+    flip = np.einsum("ti,ti->t", d[:, 0], np.cross(d[:, 1], d[:, 2])) > 0
+    T[flip, 0], T[flip, 1] = T[flip, 1].copy(), T[flip, 0].copy()
+    return X, T
+
+
+@pytest.mark.parametrize("kind", ["lattice", "random", "fan"])
+@pytest.mark.parametrize("plan", [None, "gather"])
+def test_tets(ctx, oracle, kind, plan):
+    from simit_gb300.runtime import (Mesh, assemble_heat, assemble_tet_force,
+                                     assemble_tet_stiffness, tet_precompute)
+    X, T = _tets(kind)
+    n, nT = len(X), len(T)
+    tets = T.astype(np.int32).reshape(-1)
+    g = meshgen.rng(9)
+    x = X.reshape(-1) + g.uniform(-1e-3, 1e-3, n * 3)
+    v = g.normal(size=n * 3)
+    mu, lam = g.uniform(1e3, 1e5, nT), g.uniform(1e3, 1e5, nT)
+    c = (g.uniform(size=n) < 0.2).astype(np.int32)
+    kappa, T0 = 10 ** g.uniform(-2, 2, nT), g.uniform(size=n)
+    grav = np.array([0.1, 0.2, -9.81])
+    mesh = Mesh(ctx, n, tets, 4, plan=plan)
+    rp, ci = mesh.pattern.host()
+    oB, oW, _ = oracle.tet_precompute(X.reshape(-1), tets, 1e3)
+    B, W, _ = tet_precompute(mesh, X.reshape(-1), 1e3)
+    oA, ob = oracle.heat_assemble(n, tets, oB, oW, kappa, 1e-2, T0, rp, ci)
+    A, b = assemble_heat(mesh, B, W, kappa, 1e-2, T0)
+    ctx.sync()
+    assert np.array_equal(_np(A), oA) and np.array_equal(_np(b), ob)
+
+    def close(got, ref, tol):
+        ctx.sync()
+        assert np.abs(_np(got) - ref).max() <= tol * np.abs(ref).max()
+
+    for dt, tol in ((torch.float64, 1e-12), (torch.float32, 1e-5)):
+        A, b = assemble_heat(mesh, B, W, kappa, 1e-2, T0, dtype=dt, exact=False)
+        close(A, oA, tol)
+        close(b, ob, tol)
+    for model in (0, 1):
+        oK = oracle.tet_stiffness(model, x, c, tets, oB, oW, mu, lam, 0.01, 1e3, rp, ci)
+        of = oracle.tet_force(model, x, v, c, tets, oB, oW, mu, lam, 0.01, 1e3, grav)
+        K = assemble_tet_stiffness(mesh, model, x, c, B, W, mu, lam, 0.01, 1e3, exact=False)
+        f = assemble_tet_force(mesh, model, x, v, c, B, W, mu, lam, 0.01, 1e3, grav, exact=False)
+        close(K, oK, 1e-12)
+        close(f, of, 1e-12)
