@@ -548,14 +548,16 @@ int sg_residual(sg_ctx *ctx, const sg_matrix *A, const double *x, const double *
  * Batched PCG: nsys independent 3x3-blocked systems concatenated into one
  * block-diagonal FP32 matrix (system s = block rows [sys_ptr[s],
  * sys_ptr[s+1]), columns inside that range only), solved in ONE persistent
- * launch: each CTA takes whole systems from a queue in the given order
- * (`order`, largest first for load balance) and runs mixed-precision
- * block-Jacobi PCG on them with CTA-local barriers only.  Each system stops
+ * launch of mixed-precision block-Jacobi PCG: either each CTA takes whole
+ * systems from a queue in the given order (`order`, largest first for load
+ * balance) with CTA-local barriers only, or the whole (cooperative) grid
+ * iterates on all systems at once.  Each system stops
  * at ||b_s - A_s x_s|| <= tol ||b_s|| (confirmed in FP64) or maxiters.
  * b, x FP32 [n*3] device (x: guess in, solution out); iters, status
- * (SG_STATUS_*), relres per system (device).  config selects threads per
- * CTA and lanes per row (0 .. sg_batched_configs()-1; the autotuner in the
- * host runtime picks one).  Asynchronous; capturable after a first call has
+ * (SG_STATUS_*), relres per system (device).  config selects the schedule,
+ * threads per CTA and lanes per row (0 .. sg_batched_configs()-1: 0..5 one CTA
+ * per system, 6 and 7 the whole grid on all; the autotuner in the host runtime
+ * picks one).  Asynchronous; capturable after a first call has
  * sized the context scratch.  Replaces running one Simit program per mesh
  * (no batched counterpart in the reference).
  * ------------------------------------------------------------------- */

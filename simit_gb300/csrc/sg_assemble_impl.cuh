@@ -72,9 +72,12 @@ static int launch_tile(Ctx *c, AsmArgs<T> &a, const sg_mesh *m) {
     g.hcap = 128;
     sh = tile_smem<E, T>(g);
   }
-  if (sh > 44 * 1024)  // (with the kernel's static tables, past the default limit)
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, []() -> int {
     SG_CHECK_CUDA(cudaFuncSetAttribute(k_tile<E, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sh));
+                                       220 * 1024));
+    return SG_OK;
+  }));
   a.err = c->d_err;
   k_tile<E, T><<<(a.n + g.rows - 1) / g.rows, TILE_T, sh, c->stream>>>(a, g);
   SG_CHECK_LAUNCH();

@@ -46,8 +46,9 @@ int check_device_error(Ctx *c, const char *what) {
                                   "bulk-copy barrier wait timed out",
                                   "an element needs more than 128 colours",
                                   "bulk copies still in flight after a timeout (results "
-                                  "undefined; destroy and recreate the context)"};
-    const char *nm = (e > 0 && e < 9) ? names[e] : "unknown";
+                                  "undefined; destroy and recreate the context)",
+                                  "a grid barrier timed out (results undefined)"};
+    const char *nm = (e > 0 && e < 10) ? names[e] : "unknown";
     return set_error(SG_ERR_DEVICE, "%s: device check failed (%d: %s)", what, e,
                      nm);
   }

@@ -94,6 +94,7 @@ enum DevErr : int {
   DEV_TOO_MANY_COLORS = 7,  // element colouring needs more than SG_MAX_COLORS
   DEV_TMA_UNDRAINED = 8,    // after a timeout, a copy was still in flight at exit:
                             // results undefined, reset the context
+  DEV_GRID_TIMEOUT = 9,     // a grid barrier's wait ran out of polls
 };
 
 int set_error(int code, const char *fmt, ...);

@@ -76,3 +76,70 @@ def test_graph_replay_is_deterministic(ctx, batch):
     ctx.sync()
     assert torch.equal(v1, batch.vout)
     assert 0 <= batch.config < _lib.load().sg_batched_configs()
+
+
+GRID_CONFIGS = (6, 7)  # the whole grid on all systems
+
+
+@pytest.mark.parametrize("sides", [[2], [8], [3, 9, 33, 8], [2] * 400 + [5, 70], [64, 100]])
+def test_grid_wide_matches_per_system(ctx, sides):
+    """The grid-wide schedule against the per-system one: one tiny system,
+    systems of exactly a chunk, more systems than a CTA keeps in shared
+    memory, systems over many CTAs -- same status, and the same solution as
+    far as two solves to a 1e-6 residual agree (1e-4, as above)."""
+    parts, off = [], 0
+    from simit_gb300 import meshgen
+    g = meshgen.rng(4)
+    for s in sides:
+        sh = meshgen.cloth_sheet(s)
+        x = sh["x"].reshape(-1, 3).copy()
+        x[:, 2] += g.uniform(-0.2, 0.2, len(x)) / (s - 1)
+        parts.append((x.reshape(-1), sh["ep"] + off, np.where(sh["is_bend"] > 0, 50.0, 5e3),
+                      sh["l0"], sh["fixed"]))
+        off += sh["n"]
+    x, ep, k, l0, fixed = [np.concatenate(t) for t in zip(*parts)]
+    host = {"n": off, "x": x, "ep": ep.astype(np.int32), "k": k, "l0": l0, "fixed": fixed,
+            "sys_ptr": np.concatenate([[0], np.cumsum(np.square(sides))]).astype(np.int32),
+            "sides": np.asarray(sides)}
+    cb = problems.ClothBatch(ctx, host, config=3)
+    cb.step()
+    ctx.sync()
+    ref, st = cb.vout.cpu().numpy(), cb.status.cpu().numpy()
+    for cfg in GRID_CONFIGS:
+        cb.step(config=cfg)
+        ctx.sync()
+        assert np.array_equal(cb.status.cpu().numpy(), st)
+        assert np.all(cb.relres.cpu().numpy()[st == 1] <= 1e-6)
+        v = cb.vout.cpu().numpy()
+        assert np.linalg.norm(v - ref) <= 1e-4 * np.linalg.norm(ref)
+        first = cb.vout.clone()
+        cb.step(config=cfg)
+        ctx.sync()
+        assert torch.equal(first, cb.vout)
+    # the iteration limit: stopped after as many iterations, with its status
+    for maxiters in (0, 5):
+        cb.step(config=3, maxiters=maxiters)
+        ctx.sync()
+        st, it = cb.status.cpu().numpy(), cb.iters.cpu().numpy()
+        for cfg in GRID_CONFIGS:
+            cb.step(config=cfg, maxiters=maxiters)
+            ctx.sync()
+            assert np.array_equal(cb.status.cpu().numpy(), st)
+            assert np.array_equal(cb.iters.cpu().numpy(), it)
+
+
+def test_grid_wide_systems_without_rows(ctx):
+    """Empty systems among the others finish at once, converged."""
+    host = problems.cloth_batch(nsheets=3, lo=6, hi=20, seed=9)
+    sp = host["sys_ptr"]
+    host = dict(host, sys_ptr=np.array([0, 0, sp[1], sp[1], sp[1], sp[2], sp[3], sp[3]], np.int32))
+    cb = problems.ClothBatch(ctx, host, config=3)
+    cb.step()
+    ctx.sync()
+    st, it = cb.status.cpu().numpy(), cb.iters.cpu().numpy()
+    assert np.all(st == 1)
+    for cfg in GRID_CONFIGS:
+        cb.step(config=cfg)
+        ctx.sync()
+        assert np.array_equal(cb.status.cpu().numpy(), st)
+        assert np.all(cb.iters.cpu().numpy()[it == 0] == 0)
