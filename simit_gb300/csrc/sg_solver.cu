@@ -791,11 +791,12 @@ int solver_init(Ctx *c, const sg_matrix *A, const sg_solve_opts *o_in, Solver *S
   // K1: the TMA-staged kernel for 3x3 or scalar blocks with 16-byte aligned
   // arrays (unless a lane count is forced), else G lanes per row.
   const bool aligned = ((uintptr_t)A->vals % 16 == 0) && ((uintptr_t)A->colidx % 16 == 0);
-  if ((A->bs == 3 || A->bs == 1) && aligned &&
-      (o->lanes < 0 || (o->lanes == 0 && S->kind != KIND_F64))) {
+  const int dvar = S->kind == KIND_F64 ? default_f64_variant(A->n, A->bs)
+                                       : default_tma_variant(A->bs);
+  if ((A->bs == 3 || A->bs == 1) && aligned && (o->lanes < 0 || (o->lanes == 0 && dvar >= 0))) {
     SG_TRY(cached_stats(c, A->n, A->rowptr, &S->pstats, true));
     S->maxrow = S->pstats.maxrow;
-    S->tma_var = o->lanes < 0 ? -o->lanes - 1 : default_tma_variant(A->bs);
+    S->tma_var = o->lanes < 0 ? -o->lanes - 1 : dvar;
     const int vdt = (S->kind == KIND_F64) ? SG_F64 : SG_F32;
     const int xdt = S->kind == KIND_MIXED ? SG_F32 : SG_F64;
     int grid = 0;

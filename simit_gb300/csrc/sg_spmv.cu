@@ -28,6 +28,48 @@ constexpr int kNumTmaVariants = sizeof(kTmaVariants) / sizeof(kTmaVariants[0]);
 constexpr int kDefaultTmaVariant = 9;   // 3x3: per-warp, 4 lanes per row, 2 stages
 constexpr int kDefaultTmaVariant1 = 12; // scalar: per-warp, 4 lanes, 4 passes (32 rows)
 int default_tma_variant(int bs) { return bs == 1 ? kDefaultTmaVariant1 : kDefaultTmaVariant; }
+// FP64 3x3 matrices: k_bsr3_f64, past the numbered variants (it is the default,
+// g = 0).  Its tiles of 64 rows leave SMs without work on small matrices, where
+// the streaming kernel's shorter chain wins: 729 rows 9.2 us against 8.7, 4,913
+// rows 8.8 against 9.1, 9,261 rows 8.9 against 10.5.
+constexpr int kF64Variant = kNumTmaVariants;
+int default_f64_variant(int32_t n, int bs) { return bs == 3 && n >= 4096 ? kF64Variant : -1; }
+
+template <bool DOT>
+static int f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size_t *smem,
+                      int *capb) {
+  const int bound = F64_ROWS * (ps.maxrow > 0 ? ps.maxrow : 1);
+  const int t = ps.tile32 * (F64_ROWS / 32);
+  *capb = t > 0 && t < bound ? t : bound;
+  *smem = f64_smem_bytes(*capb);
+  if (*smem > 200 * 1024) return SG_ERR_UNSUPPORTED;
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, []() -> int {
+    SG_CHECK_CUDA(cudaFuncSetAttribute(k_bsr3_f64<DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       200 * 1024));
+    return SG_OK;
+  }));
+  int per_sm = 0;
+  SG_CHECK_CUDA(
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bsr3_f64<DOT>, F64_T, *smem));
+  if (per_sm < 1) return SG_ERR_UNSUPPORTED;
+  const int ntiles = (n + F64_ROWS - 1) / F64_ROWS;
+  *grid = per_sm * c->num_sms < ntiles ? per_sm * c->num_sms : ntiles;
+  return SG_OK;
+}
+
+template <bool DOT>
+static int f64_launch(Ctx *c, cudaStream_t st, const SolveCtl *ctl, int32_t n, const uint32_t *rp,
+                      const uint32_t *ci, const void *v, const void *x, void *y, double *part,
+                      const PatternStats &ps, int grid) {
+  int g = 0, capb = 0;
+  size_t smem = 0;
+  SG_TRY(f64_config<DOT>(c, n, ps, &g, &smem, &capb));
+  k_bsr3_f64<DOT><<<grid, F64_T, smem, st>>>(ctl, n, rp, ci, (const double *)v, (const double *)x,
+                                             (double *)y, part, capb, c->d_err);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
+}
 
 // Blocks in the largest tile of `rows` consecutive rows (the buffer size).
 static int tile_cap(int rows, const PatternStats &ps) {
@@ -169,6 +211,15 @@ static int tma_any(Ctx *c, cudaStream_t st, bool launch, int bs, int vdt, int xd
                    const void *v, const void *x, void *y, double *part, const PatternStats &ps,
                    int *grid, size_t *smem) {
   const SolveCtl *k = (const SolveCtl *)ctl;
+  if (var == kF64Variant) {
+    if (bs != 3 || vdt != SG_F64 || xdt != SG_F64) return SG_ERR_UNSUPPORTED;
+    if (launch)
+      return dot ? f64_launch<true>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid)
+                 : f64_launch<false>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid);
+    int capb = 0;
+    return dot ? f64_config<true>(c, n, ps, grid, smem, &capb)
+               : f64_config<false>(c, n, ps, grid, smem, &capb);
+  }
   if (vdt == SG_F32 && xdt == SG_F32)
     return tma_dispatch<float, float>(c, st, launch, bs, var, dot, k, n, rp, ci, v, x, y, part, ps,
                                       grid, smem);
@@ -197,6 +248,7 @@ int bsr3_tma_launch(Ctx *c, cudaStream_t st, const void *ctl, int bs, int vdt, i
 
 // Longest row and largest 16- / 32-row tiles (blocks) of a pattern.
 __global__ void k_pattern_stats(const uint32_t *rowptr, int32_t n, uint32_t *out) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) out[5] = rowptr[n];
   uint32_t mr = 0, t16 = 0, t32 = 0, t4 = 0, t8 = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -237,6 +289,7 @@ int cached_stats(Ctx *c, int32_t n, const uint32_t *rowptr, PatternStats *ps, bo
     ps->tile32 = c->mr_t32[slot];
     ps->tile4 = c->mr_t4[slot];
     ps->tile8 = c->mr_t8[slot];
+    ps->nnzb = c->mr_nnzb[slot];
     return SG_OK;
   }
   Scratch s(c);
@@ -258,6 +311,7 @@ int cached_stats(Ctx *c, int32_t n, const uint32_t *rowptr, PatternStats *ps, bo
   c->mr_t32[slot] = ps->tile32 = (int32_t)h[2];
   c->mr_t4[slot] = ps->tile4 = (int32_t)h[3];
   c->mr_t8[slot] = ps->tile8 = (int32_t)h[4];
+  c->mr_nnzb[slot] = ps->nnzb = h[5];
   return SG_OK;
 }
 
@@ -429,16 +483,17 @@ extern "C" int sg_bspmv(sg_ctx *h, int32_t n, int32_t bs, const uint32_t *rowptr
   if (g < 0) SG_REQUIRE((bs == 3 || bs == 1) && aligned && -g - 1 < kNumTmaVariants,
                         "sg_bspmv: g=%d selects TMA variant %d: bs=3 or 1, 16-byte aligned "
                         "arrays, -%d <= g <= -1", g, -g - 1, kNumTmaVariants);
-  if ((g == 0 && (bs == 3 || bs == 1) && aligned && !(vdt == SG_F64 && xdt == SG_F64)) ||
-      g < 0) {
+  const bool f64 = vdt == SG_F64 && xdt == SG_F64;
+  const int fvar = f64 ? default_f64_variant(n, bs) : default_tma_variant(bs);
+  if ((g == 0 && (bs == 3 || bs == 1) && aligned && fvar >= 0) || g < 0) {
     // TMA-staged kernel (lanes per row from the row length unless given).
-    // FP64 matrices default to the plain kernel, which keeps more warps in
-    // flight for the FP64 pipe.
+    // Small and scalar FP64 matrices default to the plain kernel, which keeps
+    // more warps in flight for the FP64 pipe.
     int grid = 0;
     size_t sh = 0;
     PatternStats ps;
     SG_TRY(cached_stats(c, n, rowptr, &ps));
-    const int var = g < 0 ? -g - 1 : default_tma_variant(bs);
+    const int var = g < 0 ? -g - 1 : fvar;
     if (bsr3_tma_config(c, bs, vdt, xdt, var, 0, n, ps, &grid, &sh) == SG_OK)
       return bsr3_tma_launch(c, c->stream, nullptr, bs, vdt, xdt, var, 0, n, rowptr, colidx, vals,
                              x, y, nullptr, ps, grid, sh);
@@ -446,12 +501,13 @@ extern "C" int sg_bspmv(sg_ctx *h, int32_t n, int32_t bs, const uint32_t *rowptr
     // the streaming G-lane kernel needs no staging
     g = 0;
   }
-  // nnzb is only needed for the default lane choice; read rowptr[n] then.
+  // nnzb is only needed for the default lane choice (reading rowptr[n] on each
+  // call waited for the stream: 14 us)
   int64_t nnzb = 0;
   if (g == 0) {
-    SG_CHECK_CUDA(cudaMemcpyAsync(c->h_stage, rowptr + n, 4, cudaMemcpyDeviceToHost, c->stream));
-    SG_CHECK_CUDA(cudaStreamSynchronize(c->stream));
-    nnzb = *(uint32_t *)c->h_stage;
+    PatternStats ps;
+    SG_TRY(cached_stats(c, n, rowptr, &ps));
+    nnzb = ps.nnzb;
   }
   return bspmv_launch(c, n, bs, rowptr, colidx, vdt, vals, xdt, x, y, g, nnzb);
 }

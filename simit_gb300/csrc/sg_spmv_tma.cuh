@@ -14,6 +14,8 @@
 #include "sg_solver_kernels.cuh"
 #include "sg_tma.cuh"
 
+#include <type_traits>
+
 namespace sg {
 
 template <typename MT, int BB = 9>
@@ -407,6 +409,149 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32)
   __shared__ double shred[33];
   wtma_body<1, G, NST, P, MT, VT, DOT>(ctl, n, rowptr, colidx, vals, x, y, part, capb, err, sm,
                                        shred);
+}
+
+// FP64 3x3 blocked SpMV, rows sorted by length inside a tile.
+//
+// An SM of this GPU has one FP64 pipe that takes a warp instruction every 16
+// cycles, however many of the warp's lanes are active, so the product is bound
+// by FP64 warp instructions (0.40 ms at 128^3: 9 multiply-adds a block in full
+// warps) before it is by memory (0.33 ms).  Here a lane owns one component of
+// one row: 3 multiply-adds a block, no reduction across lanes.  A CTA stages
+// the values and columns of F64_ROWS rows with one bulk copy each, ranks the
+// rows by length meanwhile, and gives each warp 32 (row, component) pairs of
+// neighbouring rank, so that the lanes of a warp end together (the five-tet
+// lattice alternates rows of 7 and 19 blocks).  With 4 lanes a row, two thirds
+// of the multiply-adds' lanes and all of the shuffled additions were idle work.
+// At 128^3: 0.555 ms, streaming with 4 lanes a row 1.04; 64^3: 85 us, 142.
+// 64 rows: six full warps; three CTAs an SM keep the copies of two in flight
+// (32 rows, six CTAs: 0.58 ms; 96 rows, two: 0.70).  Groups of 2, 6 or 8
+// gathers instead of 4: 0.548 to 0.556; predicated groups: 0.60 (4), 0.77 (6).
+constexpr int F64_ROWS = 64, F64_T = 3 * F64_ROWS;
+constexpr int F64_U = 4;  // blocks whose gathers a lane has in flight
+inline size_t f64_smem_bytes(int capb) {
+  return 16 + tma_vbytes<double>(capb) + tma_cbytes(capb);
+}
+
+template <bool DOT>
+__device__ __forceinline__ void f64_task(uint32_t q0, uint32_t q1, int64_t row, int comp,
+                                         const double *vb, const uint32_t *cb, size_t voff,
+                                         size_t coff, const double *__restrict__ x,
+                                         double *__restrict__ y, DotAcc<double> &acc) {
+  double a[2] = {0.0, 0.0};  // even and odd blocks: half the dependent chain
+  // U blocks, their gathers in flight together.  Whole groups only: a
+  // predicated-off multiply-add still takes its place on the pipe.
+  auto group = [&](auto width) {
+    constexpr int U = decltype(width)::value;
+    double xg[U][3];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const double *xc = x + (size_t)cb[q0 + k - coff] * 3;
+      xg[k][0] = ldg(xc);
+      xg[k][1] = ldg(xc + 1);
+      xg[k][2] = ldg(xc + 2);
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const double *v = vb + ((size_t)(q0 + k) * 9 + comp * 3 - voff);
+      a[k & 1] = fma(v[2], xg[k][2], fma(v[1], xg[k][1], fma(v[0], xg[k][0], a[k & 1])));
+    }
+    q0 += U;
+  };
+  while (q0 + F64_U <= q1) group(std::integral_constant<int, F64_U>());
+  if (q0 + 2 <= q1) group(std::integral_constant<int, 2>());
+  if (q0 < q1) group(std::integral_constant<int, 1>());
+  const double yv = a[0] + a[1];
+  y[row * 3 + comp] = yv;
+  if (DOT) acc.add(x[row * 3 + comp], yv);
+}
+
+template <bool DOT>
+__global__ void __launch_bounds__(F64_T, 3)
+    k_bsr3_f64(const SolveCtl *__restrict__ ctl, int32_t n, const uint32_t *__restrict__ rowptr,
+               const uint32_t *__restrict__ colidx, const double *__restrict__ vals,
+               const double *__restrict__ x, double *__restrict__ y, double *__restrict__ part,
+               int capb, int *err) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ double shred[33];
+  __shared__ uint32_t rp[F64_ROWS + 1];
+  __shared__ uint8_t order[F64_ROWS];
+  if (ctl && ctl->status != ST_RUNNING) return;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm);
+  double *vb = reinterpret_cast<double *>(sm + 16);
+  uint32_t *cb = reinterpret_cast<uint32_t *>(sm + 16 + tma_vbytes<double>(capb));
+  const int tid = threadIdx.x;
+  if (tid == 0) {
+    mbar_init(bar, 1);
+    mbar_fence_init();
+  }
+  const int ntiles = (n + F64_ROWS - 1) / F64_ROWS;
+  DotAcc<double> acc;
+  uint32_t phase = 0, next = 0;  // next: the next tile's row pointers, a thread each
+  if (tid <= F64_ROWS && (int)blockIdx.x < ntiles)
+    next = rowptr[min((int64_t)n, (int64_t)blockIdx.x * F64_ROWS + tid)];
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int64_t r0 = (int64_t)tile * F64_ROWS;
+    const int nr = (int)min((int64_t)F64_ROWS, n - r0);
+    __syncthreads();  // the previous tile's buffers and tables are free
+    if (tid <= F64_ROWS) rp[tid] = next;
+    __syncthreads();
+    const uint32_t b0 = rp[0], b1 = rp[nr];
+    const bool staged = b1 - b0 <= (uint32_t)capb;
+    const size_t vs = staged ? ((size_t)b0 * 72) & ~size_t(15) : 0;
+    const size_t cs = staged ? ((size_t)b0 * 4) & ~size_t(15) : 0;
+    const size_t ve = ((size_t)b1 * 72) & ~size_t(15), ce = ((size_t)b1 * 4) & ~size_t(15);
+    if (staged && tid == 0) {
+      fence_proxy_async_smem();
+      const uint32_t vn = ve > vs ? (uint32_t)(ve - vs) : 0u, cn = ce > cs ? (uint32_t)(ce - cs) : 0u;
+      mbar_arrive_expect_tx(bar, vn + cn);
+      if (vn) bulk_g2s(vb, reinterpret_cast<const unsigned char *>(vals) + vs, vn, bar);
+      if (cn) bulk_g2s(cb, reinterpret_cast<const unsigned char *>(colidx) + cs, cn, bar);
+    }
+    // meanwhile: the rows by length, longest first, and the next row pointers
+    if (tid < nr) {
+      const uint32_t len = rp[tid + 1] - rp[tid];
+      int rank = 0;
+      for (int u = 0; u < nr; ++u) {
+        const uint32_t lu = rp[u + 1] - rp[u];
+        rank += lu > len || (lu == len && u < tid);
+      }
+      order[rank] = (uint8_t)tid;
+    }
+    if (tid <= F64_ROWS && tile + (int)gridDim.x < ntiles)
+      next = rowptr[min((int64_t)n, r0 + (int64_t)gridDim.x * F64_ROWS + tid)];
+    if (staged) {
+      // the tails of less than 16 bytes
+      if (tid >= 32 && tid < 32 + (int)((((size_t)b1 * 72) - ve) / 8))
+        vb[(ve - vs) / 8 + tid - 32] = vals[ve / 8 + tid - 32];
+      if (tid >= 64 && tid < 64 + (int)((((size_t)b1 * 4) - max(ce, cs)) / 4))
+        cb[(max(ce, cs) - cs) / 4 + tid - 64] = colidx[max(ce, cs) / 4 + tid - 64];
+      bool ok = mbar_wait(bar, phase);
+      if (!ok) {
+        if (tid == 0) {
+          atomicCAS(err, 0, 6 /* DEV_TMA_TIMEOUT */);
+          if (!mbar_wait(bar, phase)) atomicExch(err, 8 /* DEV_TMA_UNDRAINED */);
+        }
+      }
+      if (__syncthreads_or(!ok)) break;
+      phase ^= 1u;
+    } else {
+      __syncthreads();
+    }
+    const int rank = tid / 3, comp = tid - rank * 3;
+    if (rank < nr) {
+      const int rl = order[rank];
+      if (staged)
+        f64_task<DOT>(rp[rl], rp[rl + 1], r0 + rl, comp, vb, cb, vs / 8, cs / 4, x, y, acc);
+      else
+        f64_task<DOT>(rp[rl], rp[rl + 1], r0 + rl, comp, vals, colidx, 0, 0, x, y, acc);
+    }
+  }
+  if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
+    const double t = block_sum(acc.value(), shred);
+    SolveCtl *c = const_cast<SolveCtl *>(ctl);
+    finalize_partials(&t, 1, part, &c->tick1, &c->pq_tot, shred);
+  }
 }
 
 }  // namespace sg

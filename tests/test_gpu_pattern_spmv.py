@@ -198,6 +198,36 @@ def test_spmv_tma_stale_statistics(ctx, oracle):
             assert np.all(np.abs(y.cpu().numpy() - ref) <= 2e-6 * scale + 1e-30), variant
 
 
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 4159, 4161, 9000])
+def test_spmv_f64_sorted_rows(ctx, oracle, n):
+    """The FP64 3x3 product at the sizes around its tiles of 64 rows (and
+    below its smallest matrix), with empty rows, a hub row of 300 blocks and
+    rows of every length modulo its groups of gathers; then a longer pattern
+    under statistics cached for the first one."""
+    from simit_gb300.runtime import bspmv
+    d = ctx.device
+    t = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).to(d)  # noqa
+    g = meshgen.rng(n)
+    ep = 2 * g.integers(0, n // 2, size=5 * n)  # odd vertices: empty rows
+    ep = np.concatenate([ep[:len(ep) // 2 * 2],
+                         np.stack([np.full(300, 10), g.integers(0, n, 300)], 1).reshape(-1)])
+    ep2 = np.concatenate([ep, np.stack([np.full(900, n - 1), g.integers(0, n, 900)], 1).reshape(-1)])
+    rp2, ci2 = oracle.pattern(n, ep2.astype(np.int32), 2)
+    rp_d = torch.zeros(n + 1, dtype=torch.int32, device=d)
+    ci_d = torch.zeros(len(ci2), dtype=torch.int32, device=d)
+    for e in (ep, ep2):
+        rp, ci = oracle.pattern(n, e.astype(np.int32), 2)
+        rp_d.copy_(t(rp))
+        ci_d[:len(ci)].copy_(t(ci))
+        vals, x = g.uniform(-1, 1, size=len(ci) * 9), g.uniform(-1, 1, size=n * 3)
+        ref = oracle.spmv(n, 3, rp, ci, vals, x)
+        scale = oracle.spmv(n, 3, rp, ci, np.abs(vals), np.abs(x))
+        y = bspmv(ctx, n, 3, rp_d, ci_d, t(vals), t(x),
+                  y=torch.full((n * 3,), float("nan"), dtype=torch.float64, device=d))
+        ctx.sync()
+        assert np.all(np.abs(y.cpu().numpy() - ref) <= 1e-14 * scale + 1e-300)
+
+
 def test_spmv_tma_variant_out_of_range(ctx, oracle):
     from simit_gb300._lib import SimitError
     from simit_gb300.runtime import bspmv
