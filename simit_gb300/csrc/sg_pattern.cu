@@ -10,8 +10,11 @@
 // Design: no std::set and no global sort.  Incidences are bucketed by vertex
 // with integer atomics (counts only), and each vertex's bucket is then sorted
 // by (e*card + i) inside one warp, so every result is deterministic.  Row
-// columns come from a per-warp shared-memory bitonic sort + unique of the
-// bucket's endpoints; slots from a binary search of the sorted row.
+// columns: a warp per vertex puts the endpoints of its elements into a small
+// shared-memory set and sorts what is left (a five-tet lattice row has 7 or 19
+// columns among 32 or 128 endpoints), which is all the filling pass needs and
+// more than the counting one does; slots from a binary search of the sorted
+// row.
 #include "sg_internal.cuh"
 
 namespace sg {
@@ -119,8 +122,94 @@ __global__ void inc_sort(const uint32_t *ve_ptr, uint32_t *ve_idx, int32_t n,
   }
 }
 
-// One warp per vertex: gather the endpoints of every incident element, sort,
-// unique.  Pass 0 writes the unique count to rowcnt[v]; pass 1 writes the
+// One warp per vertex: the distinct endpoints of its incident elements.  Pass 0
+// writes their number to rowcnt[v], pass 1 the sorted columns at
+// colidx[rowptr[v]...].  A row of more than SET_MAX distinct columns sets
+// *over, and the caller runs rows_build.
+//
+// Bound by the gathers of the endpoints and shared-memory operations: at 64^3
+// cells the passes take 114 and 141 us; sorting all 32..128 endpoints of
+// every row in shared memory, twice, took 491 us a pass.
+constexpr int MAX_SORT_CAP = 16384;  // keys per warp (64 KB) of rows_build and inc_sort
+constexpr int SET_CAP = 256, SET_MAX = 192;  // table entries, columns kept
+__global__ void __launch_bounds__(256) rows_set(const int32_t *ep, int32_t card,
+                                                const uint32_t *ve_ptr, const uint32_t *ve_idx,
+                                                int32_t n, int pass, uint32_t *rowcnt,
+                                                const uint32_t *rowptr, uint32_t *colidx,
+                                                uint32_t *over, int vec4) {
+  __shared__ uint32_t tabs[8][SET_CAP], lists[8][SET_CAP];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t *tab = tabs[warp], *list = lists[warp];
+  for (int64_t v = (int64_t)blockIdx.x * 8 + warp; v < n; v += (int64_t)gridDim.x * 8) {
+    const uint32_t b = ve_ptr[v], e = ve_ptr[v + 1];
+    const int64_t len = (int64_t)(e - b) * card;
+    int cap = 32;  // a table at most half full, if the row is short
+    while (cap < SET_CAP && cap < 2 * len) cap <<= 1;
+    for (int i = lane; i < cap; i += 32) tab[i] = 0xffffffffu;
+    __syncwarp();
+    // v itself is in every element of its row: it goes in once, ahead
+    int cnt = len > 0 ? 1 : 0;
+    if (lane == 0) list[0] = (uint32_t)v;
+    bool full = len > MAX_SORT_CAP;  // (rows_build's limit, and its error)
+    // a lane takes an incidence; its endpoints one after the other
+    for (uint32_t k0 = b; k0 < e && !full; k0 += 32) {
+      const uint32_t k = k0 + lane;
+      const int64_t first = k < e ? (int64_t)(ve_idx[k] / (uint32_t)card) * card : -1;
+      int4 four = make_int4(0, 0, 0, 0);
+      if (vec4 && first >= 0) four = reinterpret_cast<const int4 *>(ep)[first / 4];
+      for (int j = 0; j < card && !full; ++j) {
+        uint32_t val = (uint32_t)v;
+        if (first >= 0)
+          val = (uint32_t)(!vec4 ? ep[first + j]
+                                 : j == 0 ? four.x : j == 1 ? four.y : j == 2 ? four.z : four.w);
+        bool fresh = false;
+        if (val != (uint32_t)v) {
+          uint32_t h = val * 0x9E3779B1u >> 16;
+          for (;; ++h) {  // at most cnt + 32 <= SET_MAX + 32 entries are taken
+            h &= (uint32_t)cap - 1u;
+            const uint32_t old = atomicCAS(&tab[h], 0xffffffffu, val);
+            fresh = old == 0xffffffffu;
+            if (fresh || old == val) break;
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, fresh);
+        if (fresh) list[cnt + __popc(m & ((1u << lane) - 1u))] = val;
+        cnt += __popc(m);
+        full = cnt > SET_MAX;
+      }
+    }
+    __syncwarp();
+    if (full) {
+      if (lane == 0) atomicExch(over, 1u);
+      if (pass == 0 && lane == 0) rowcnt[v] = 0;
+      continue;
+    }
+    if (pass == 0) {
+      if (lane == 0) rowcnt[v] = (uint32_t)cnt;
+      continue;
+    }
+    uint32_t *out = colidx + rowptr[v];
+    if (cnt <= 32) {  // register bitonic
+      uint32_t key = lane < cnt ? list[lane] : 0xffffffffu;
+      for (int k = 2; k <= 32; k <<= 1)
+        for (int j = k >> 1; j > 0; j >>= 1) {
+          const uint32_t other = __shfl_xor_sync(0xffffffffu, key, j);
+          key = (((lane & j) == 0) == ((lane & k) == 0)) ? min(key, other) : max(key, other);
+        }
+      if (lane < cnt) out[lane] = key;
+    } else {
+      const int p2 = pow2_at_least(cnt);
+      for (int i = cnt + lane; i < p2; i += 32) list[i] = 0xffffffffu;
+      __syncwarp();
+      warp_bitonic_sort(list, p2);
+      for (int i = lane; i < cnt; i += 32) out[i] = list[i];
+    }
+    __syncwarp();
+  }
+}
+
+// The same for rows of any length up to the sort capacity: gather the endpoints
+// of every incident element, sort, unique.  Pass 0 writes the unique count to rowcnt[v]; pass 1 writes the
 // columns at colidx[rowptr[v]...].
 __global__ void rows_build(const int32_t *ep, int32_t card, const uint32_t *ve_ptr,
                            const uint32_t *ve_idx, int32_t n, int cap, int pass,
@@ -172,10 +261,11 @@ __global__ void rows_build(const int32_t *ep, int32_t card, const uint32_t *ve_p
   }
 }
 
-// Thread per (e, i): binary search each ep[e, j] in row ep[e, i].
+// Thread per (e, i): the position of each ep[e, j] in row ep[e, i], four
+// columns searched a step at a time so that their loads overlap.
 __global__ void slots_build(const int32_t *ep, int64_t nE, int32_t card, int32_t n,
                            const uint32_t *rowptr, const uint32_t *colidx,
-                           uint32_t *slots, int *err) {
+                           uint32_t *slots, int *err, int vec4) {
   const int64_t m = nE * card;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -186,19 +276,44 @@ __global__ void slots_build(const int32_t *ep, int64_t nE, int32_t card, int32_t
       for (int j = 0; j < card; ++j) slots[t * card + j] = 0xffffffffu;
       continue;
     }
-    const uint32_t lo0 = rowptr[row], hi0 = rowptr[row + 1];
-    for (int j = 0; j < card; ++j) {
-      const uint32_t col = (uint32_t)ep[e * card + j];
-      uint32_t lo = lo0, hi = hi0;
-      while (lo < hi) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (colidx[mid] < col) lo = mid + 1; else hi = mid;
+    const uint32_t lo0 = rowptr[row], len = rowptr[row + 1] - lo0;
+    uint32_t top = 1;  // the largest power of two <= len
+    while (top <= len / 2) top *= 2;
+    for (int j0 = 0; j0 < card; j0 += 4) {
+      uint32_t col[4], lo[4];
+      if (vec4) {
+        const int4 f = reinterpret_cast<const int4 *>(ep)[e];
+        col[0] = f.x; col[1] = f.y; col[2] = f.z; col[3] = f.w;
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) col[j] = j0 + j < card ? (uint32_t)ep[e * card + j0 + j] : 0u;
       }
-      if (lo >= hi0 || colidx[lo] != col) {
-        dev_fail(err, DEV_SLOT_MISSING);
-        lo = 0xffffffffu;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) lo[j] = 0u;
+      for (uint32_t st = top; st; st >>= 1) {  // lo: columns below col
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t q = lo[j] + st;
+          if (q <= len && colidx[lo0 + q - 1] < col[j]) lo[j] = q;
+        }
       }
-      slots[t * card + j] = lo;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j0 + j >= card) break;
+        if (lo[j] >= len || colidx[lo0 + lo[j]] != col[j]) {
+          dev_fail(err, DEV_SLOT_MISSING);
+          lo[j] = 0xffffffffu;
+        } else {
+          lo[j] += lo0;
+        }
+      }
+      if (vec4) {
+        reinterpret_cast<uint4 *>(slots)[t] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j0 + j < card) slots[t * card + j0 + j] = lo[j];
+      }
     }
   }
 }
@@ -210,13 +325,18 @@ static int sort_cap(uint32_t maxlen) {
   return p;
 }
 
-static int max_row_len(Ctx *c, Scratch &s, const uint32_t *ptr, int32_t n,
-                       uint32_t *h_max) {
-  uint32_t *d = s.alloc<uint32_t>(1);
+// The longest row to the context's staging word (valid after the next wait).
+static int max_row_len_async(Ctx *c, uint32_t *d, const uint32_t *ptr, int32_t n) {
   SG_CHECK_CUDA(cudaMemsetAsync(d, 0, 4, c->stream));
   max_u32_diff<<<grid_for(c, n, 256, 4), 256, 0, c->stream>>>(ptr, n, d);
   SG_CHECK_LAUNCH();
   SG_CHECK_CUDA(cudaMemcpyAsync(c->h_stage, d, 4, cudaMemcpyDeviceToHost, c->stream));
+  return SG_OK;
+}
+
+static int max_row_len(Ctx *c, Scratch &s, const uint32_t *ptr, int32_t n,
+                       uint32_t *h_max) {
+  SG_TRY(max_row_len_async(c, s.alloc<uint32_t>(1), ptr, n));
   SG_CHECK_CUDA(cudaStreamSynchronize(c->stream));
   *h_max = *(uint32_t *)c->h_stage;
   return SG_OK;
@@ -229,8 +349,6 @@ static int warps_for_cap(int cap) {
   if (w > 8) w = 8;
   return w;
 }
-
-constexpr int MAX_SORT_CAP = 16384;  // keys per warp (64 KB)
 
 static int check_pattern_args(int32_t n, const int32_t *ep, int64_t nE, int32_t card) {
   SG_REQUIRE(n >= 0 && nE >= 0 && card >= 1 && card <= 64,
@@ -255,7 +373,7 @@ int sg_incidence_build(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
   SG_TRY(check_pattern_args(n, ep, nE, card));
   const int64_t m = nE * card;
   Scratch s(c);
-  SG_TRY(s.reserve(Scratch::bytes_for(n + 1, 4) * 2 + scan_scratch_bytes(n) + 512));
+  SG_TRY(s.reserve(Scratch::bytes_for(n + 1, 4) * 2 + scan_scratch_bytes(n) + 1024));
   uint32_t *cnt = s.alloc<uint32_t>(n + 1);
   uint32_t *cursor = s.alloc<uint32_t>(n + 1);
   SG_CHECK_CUDA(cudaMemsetAsync(cnt, 0, (n + 1) * sizeof(uint32_t), c->stream));
@@ -264,14 +382,16 @@ int sg_incidence_build(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
     SG_CHECK_LAUNCH();
   }
   SG_TRY(exclusive_scan_u32(c, s, cnt, ve_ptr, n));
+  // the error word and the largest degree come back with one wait
+  uint32_t *d_max = s.alloc<uint32_t>(1);
+  SG_TRY(max_row_len_async(c, d_max, ve_ptr, n));
   SG_TRY(check_device_error(c, "sg_incidence_build"));
   if (m == 0) return SG_OK;
+  const uint32_t maxdeg = *(uint32_t *)c->h_stage;
   SG_CHECK_CUDA(cudaMemcpyAsync(cursor, ve_ptr, n * sizeof(uint32_t),
                                 cudaMemcpyDeviceToDevice, c->stream));
   inc_fill<<<grid_for(c, m, 256, 8), 256, 0, c->stream>>>(ep, m, n, cursor, ve_idx);
   SG_CHECK_LAUNCH();
-  uint32_t maxdeg = 0;
-  SG_TRY(max_row_len(c, s, ve_ptr, n, &maxdeg));
   if (maxdeg > (uint32_t)MAX_SORT_CAP)
     return set_error(SG_ERR_UNSUPPORTED,
                      "sg_incidence_build: vertex degree %u exceeds %d", maxdeg, MAX_SORT_CAP);
@@ -283,7 +403,19 @@ int sg_incidence_build(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
   inc_sort<<<grid_for(c, (int64_t)n * 32, w * 32, 8), w * 32, (size_t)w * cap * 4, c->stream>>>(
       ve_ptr, ve_idx, n, cap, c->d_err);
   SG_CHECK_LAUNCH();
-  return check_device_error(c, "sg_incidence_build");
+  return SG_OK;  // (cap holds the longest list: nothing left to check)
+}
+
+// rows_set; *over (cleared here) is set when a row has too many columns.
+static int rows_set_launch(Ctx *c, const int32_t *ep, int32_t card, const uint32_t *ve_ptr,
+                           const uint32_t *ve_idx, int32_t n, int pass, uint32_t *rowcnt,
+                           const uint32_t *rowptr, uint32_t *colidx, uint32_t *over) {
+  SG_CHECK_CUDA(cudaMemsetAsync(over, 0, 4, c->stream));
+  rows_set<<<grid_for(c, (int64_t)n * 32, 256, 8), 256, 0, c->stream>>>(
+      ep, card, ve_ptr, ve_idx, n, pass, rowcnt, rowptr, colidx, over,
+      card == 4 && (uintptr_t)ep % 16 == 0);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
 }
 
 static int rows_launch(Ctx *c, Scratch &s, const int32_t *ep, int32_t card,
@@ -319,11 +451,19 @@ int sg_pattern_count(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
   Scratch s(c);
   SG_TRY(s.reserve(Scratch::bytes_for(n + 1, 4) + scan_scratch_bytes(n) + 1024));
   uint32_t *rowcnt = s.alloc<uint32_t>(n + 1);
-  SG_TRY(rows_launch(c, s, ep, card, ve_ptr, ve_idx, n, 0, rowcnt, nullptr, nullptr));
-  SG_TRY(exclusive_scan_u32(c, s, rowcnt, rowptr, n));
-  SG_CHECK_CUDA(cudaMemcpyAsync(c->h_stage, rowptr + n, 4, cudaMemcpyDeviceToHost, c->stream));
-  SG_TRY(check_device_error(c, "sg_pattern_count"));
-  *h_nnzb = *(uint32_t *)c->h_stage;
+  uint32_t *over = s.alloc<uint32_t>(1);
+  uint32_t *hs = (uint32_t *)c->h_stage;
+  SG_TRY(rows_set_launch(c, ep, card, ve_ptr, ve_idx, n, 0, rowcnt, nullptr, nullptr, over));
+  for (int k = 0; k < 2; ++k) {
+    Scratch t = s;  // (a second scan reuses the first one's scratch)
+    SG_TRY(exclusive_scan_u32(c, t, rowcnt, rowptr, n));
+    SG_CHECK_CUDA(cudaMemcpyAsync(hs, rowptr + n, 4, cudaMemcpyDeviceToHost, c->stream));
+    SG_CHECK_CUDA(cudaMemcpyAsync(hs + 1, over, 4, cudaMemcpyDeviceToHost, c->stream));
+    SG_TRY(check_device_error(c, "sg_pattern_count"));
+    if (!hs[1] || k) break;
+    SG_TRY(rows_launch(c, s, ep, card, ve_ptr, ve_idx, n, 0, rowcnt, nullptr, nullptr));
+  }
+  *h_nnzb = hs[0];
   return SG_OK;
 }
 
@@ -336,6 +476,11 @@ int sg_pattern_fill(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
   SG_TRY(check_pattern_args(n, ep, nE, card));
   Scratch s(c);
   SG_TRY(s.reserve(1024));
+  uint32_t *over = s.alloc<uint32_t>(1);
+  SG_TRY(rows_set_launch(c, ep, card, ve_ptr, ve_idx, n, 1, nullptr, rowptr, colidx, over));
+  SG_CHECK_CUDA(cudaMemcpyAsync(c->h_stage, over, 4, cudaMemcpyDeviceToHost, c->stream));
+  SG_TRY(check_device_error(c, "sg_pattern_fill"));
+  if (!*(uint32_t *)c->h_stage) return SG_OK;
   SG_TRY(rows_launch(c, s, ep, card, ve_ptr, ve_idx, n, 1, nullptr, rowptr, colidx));
   return check_device_error(c, "sg_pattern_fill");
 }
@@ -349,8 +494,9 @@ int sg_slots_build(sg_ctx *h, int32_t n, const int32_t *ep, int64_t nE,
   SG_TRY(check_pattern_args(n, ep, nE, card));
   const int64_t m = nE * card;
   if (m == 0) return SG_OK;
-  slots_build<<<grid_for(c, m, 256, 8), 256, 0, c->stream>>>(ep, nE, card, n, rowptr,
-                                                              colidx, slots, c->d_err);
+  slots_build<<<grid_for(c, m, 256, 8), 256, 0, c->stream>>>(
+      ep, nE, card, n, rowptr, colidx, slots, c->d_err,
+      card == 4 && (uintptr_t)ep % 16 == 0 && (uintptr_t)slots % 16 == 0);
   SG_CHECK_LAUNCH();
   return check_device_error(c, "sg_slots_build");
 }

@@ -198,6 +198,35 @@ def test_spmv_tma_stale_statistics(ctx, oracle):
             assert np.all(np.abs(y.cpu().numpy() - ref) <= 2e-6 * scale + 1e-30), variant
 
 
+@pytest.mark.parametrize("card", [2, 3, 4, 5])
+@pytest.mark.parametrize("hub", [0, 45, 110, 400])
+def test_pattern_and_sources_row_limits(ctx, oracle, card, hub):
+    """Pattern, slots and slot lists against the oracle for rows below and
+    past the sets of 192 columns and the lists of 128 slots (a vertex in
+    `hub` elements), more than 32 incidences a vertex, elements that list a
+    vertex twice, and vertices without elements."""
+    from simit_gb300.runtime import Mesh
+    n = 700
+    g = meshgen.rng(100 * card + hub)
+    ep = g.integers(0, n // 2, size=(900, card)) * 2
+    ep[::9, card - 1] = ep[::9, 0]
+    if hub:
+        h = g.integers(0, n, size=(hub, card))
+        h[:, hub % card] = 7
+        ep = np.concatenate([ep, h])[g.permutation(900 + hub)]
+    flat = ep.astype(np.int32).reshape(-1)
+    mesh = Mesh(ctx, n, flat, card, plan="gather")
+    rp, ci = mesh.pattern.host()
+    orp, oci = oracle.pattern(n, flat, card)
+    assert np.array_equal(rp, orp) and np.array_equal(ci, oci)
+    slots = mesh.pattern.slots[:len(flat) * card].cpu().numpy().view(np.uint32)
+    assert np.array_equal(slots, oracle.slots(flat, card, orp, oci))
+    order = np.argsort(slots, kind="stable")  # each slot's blocks, ascending
+    sp = np.concatenate([[0], np.cumsum(np.bincount(slots, minlength=len(ci)))])
+    assert np.array_equal(mesh.slot_src_ptr.cpu().numpy().view(np.uint32), sp)
+    assert np.array_equal(mesh.slot_src[:len(order)].cpu().numpy().view(np.uint32), order)
+
+
 @pytest.mark.parametrize("n", [4095, 4096, 4097, 4159, 4161, 9000])
 def test_spmv_f64_sorted_rows(ctx, oracle, n):
     """The FP64 3x3 product at the sizes around its tiles of 64 rows (and
