@@ -121,6 +121,8 @@ __global__ void k_f32_to_f64(int64_t len, const float *__restrict__ a, double *_
 // ---------------------------------------------------------------------------
 enum Kind { KIND_F64 = 0, KIND_F64_M32 = 1, KIND_MIXED = 2 };
 
+static int dot_grid(const Ctx *c, int64_t len) { return grid_for(c, len, RED_T, 4); }
+
 static int alloc_dev(Solver *S, void **p, size_t bytes) {
   if (bytes == 0) bytes = 256;
   SG_CHECK_CUDA(cudaMalloc(p, bytes));
@@ -704,7 +706,7 @@ namespace sg {
 
 void dot_launch(Ctx *c, int64_t len, const double *a, const double *b, double *part,
                 double *dres) {
-  const int P = grid_for(c, len, RED_T, 4);
+  const int P = dot_grid(c, len);
   k_dot2<<<P, RED_T, 0, c->stream>>>(len, a, b, part);
   k_sum_parts<<<1, RED_T, 0, c->stream>>>(part, P, dres);
 }
@@ -815,7 +817,9 @@ int solver_init(Ctx *c, const sg_matrix *A, const sg_solve_opts *o_in, Solver *S
     S->tma = 1;  // K1 leaves the finished p.q in ctl, as the TMA kernels do
     S->P1 = S->sym->grid[1];
   }
-  const int np = S->P1 > S->P2 ? S->P1 : S->P2;
+  // part3 also takes b.b's partials, whose grid can be the largest of the three
+  int np = S->P1 > S->P2 ? S->P1 : S->P2;
+  if (dot_grid(c, S->len) > np) np = dot_grid(c, S->len);
   SG_TRY(alloc_dev(S, (void **)&S->ctl, sizeof(SolveCtl)));
   SG_CHECK_CUDA(cudaMallocHost((void **)&S->hctl, sizeof(SolveCtl)));
   SG_TRY(alloc_dev(S, &S->r, S->len * vt));
