@@ -68,26 +68,28 @@ __global__ void k_scale(int64_t len, const float *a, float s, float *out) {
     out[i] = s * a[i];
 }
 
-// rz = r.z and zq = z.q partials for the CG's K3 (grid = P2 blocks).
-__global__ void __launch_bounds__(RED_T) k_rz_zq(const SolveCtl *ctl, int64_t len,
+// r.z and z.q of the layered preconditioner's z, summed by the last CTA with
+// the r.r partials that K2 left at part (same grid), and the iteration's
+// decision for K3.
+__global__ void __launch_bounds__(RED_T) k_rz_zq(SolveCtl *ctl, int par, int64_t len,
                                                  const float *__restrict__ r,
                                                  const float *__restrict__ z,
                                                  const float *__restrict__ q,
                                                  double *__restrict__ part) {
-  __shared__ double sh[33];
-  if (ctl && ctl->status != ST_RUNNING) return;
+  __shared__ double sh[3 * RED_T];
+  if (ctl->status != ST_RUNNING) return;
   DotAcc<float> rz, zq;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
        i += (int64_t)gridDim.x * blockDim.x) {
     rz.add(r[i], z[i]);
     zq.add(z[i], q[i]);
   }
-  const double t0 = block_sum(rz.value(), sh);
-  const double t1 = block_sum(zq.value(), sh);
-  if (threadIdx.x == 0) {
-    part[gridDim.x + blockIdx.x] = t0;
-    part[2 * gridDim.x + blockIdx.x] = t1;
-  }
+  const double v[2] = {rz.value(), zq.value()};
+  double t[3], tot[3];
+  block_sums<2>(v, t + 1, sh);
+  t[0] = part[blockIdx.x];
+  if (finalize_partials<3>(t, part, &ctl->tick2, tot, sh) && threadIdx.x == 0)
+    cg_decide(ctl, par, tot[0], tot[1], tot[2], ctl->last_alpha);
 }
 
 // ---------------------------------------------------------------------------
@@ -322,14 +324,14 @@ static int horner_launch(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int ga
 }
 
 // The folded application z = M r (symmetric form): x = L^-1 r (unless the
-// iteration's K2 wrote it: xin_ready), the six Horner steps (the first one
-// gathers x and applies G_6), z = L^-T w_0.  part (nullable): dot partials of
-// the final pass (grid np blocks); want_rr / want_zq select its slices.  The
-// FP16 evaluation (half_a) stores x and the Horner sums in block floating
+// iteration's K2 wrote it), the six Horner steps (the first one gathers x and
+// applies G_6), z = L^-T w_0.  Inside an iteration (decide_ctl) the last step
+// ends the application itself and decides the iteration, with three partials
+// per CTA of the steps' grid (np of them) at part; otherwise part (nullable)
+// gets the np partials of r.z.  The FP16 evaluation (half_a) stores x and the Horner sums in block floating
 // point, the FP32 one as float4.
 static int fold_apply(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int gate, bool half_a,
-                      const float *r, float *z, const float *q, double *part, int np, int want_rr,
-                      int want_zq, bool xin_ready, bool fused = false,
+                      const float *r, float *z, const float *q, double *part, int np,
                       SolveCtl *decide_ctl = nullptr, int par = 0) {
   Ctx *c = G->c;
   Graph &g = G->g;
@@ -338,7 +340,7 @@ static int fold_apply(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int gate,
   // k_lrn_finish moves r, q and z as float4
   SG_REQUIRE(((uintptr_t)r | (uintptr_t)z | (uintptr_t)q) % 16 == 0,
              "mpnn: r, z and q must be 16-byte aligned");
-  if (!xin_ready) {
+  if (!decide_ctl) {
     if (half_a)
       k_lrn_xin<true><<<grid_for(c, g.n, 256, 8), 256, 0, st>>>(g.n, B.l6b, r, B.xin);
     else
@@ -346,39 +348,32 @@ static int fold_apply(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int gate,
     SG_CHECK_LAUNCH();
   }
   // step 5 gathers x; step d < 5 reads w[(5 - d) & 1]; step d writes
-  // w[(6 - d) & 1] (w_0 in w[0]).  fused: step 0 ends the application itself
-  // (z and the dot partials, np of them: the steps' grid)
+  // w[(6 - d) & 1] (w_0 in w[0])
   for (int d = 5; d >= 0; --d) {
     FinArgs fa;
-    if (fused && d == 0) {
+    const bool last = decide_ctl && d == 0;
+    if (last) {
       int hg = 0;
       SG_TRY(horner_grid(G, half_a, &hg));
-      SG_REQUIRE(!part || np == hg, "mpnn: %d dot partials asked of a %d-CTA last step", np, hg);
+      SG_REQUIRE(np == hg, "mpnn: %d dot partials asked of a %d-CTA last step", np, hg);
       fa.r = r;
       fa.q = q;
       fa.z = z;
       fa.part = part;
-      fa.want_rr = want_rr;
-      fa.want_zq = want_zq;
-      if (decide_ctl && part && want_rr && want_zq) {
-        fa.ctl = decide_ctl;
-        fa.decide = 1;
-        fa.par = par;
-      }
+      fa.ctl = decide_ctl;
+      fa.par = par;
     }
     SG_TRY(horner_launch(G, st, ctl, gate, half_a, B, d, d == 5 ? B.xin : B.w[(5 - d) & 1],
-                         B.w[(6 - d) & 1], (fused && d == 0) ? &fa : nullptr));
+                         B.w[(6 - d) & 1], last ? &fa : nullptr));
   }
-  if (fused) return SG_OK;
-  // z = L^-T w_0 and the dots, in vertex order; one dot partial per block:
+  if (decide_ctl) return SG_OK;
+  // z = L^-T w_0 and the dot, in vertex order; one dot partial per block:
   // np of them when asked
   const int g0 = part ? np : finish_grid(c, B.sl.nslice);
   if (half_a)
-    k_lrn_finish<true><<<g0, LG_T, 0, st>>>(ctl, gate, g.n, B.l6b, B.xin, B.w[0], r, q, z, part,
-                                            want_rr, want_zq);
+    k_lrn_finish<true><<<g0, LG_T, 0, st>>>(ctl, gate, g.n, B.l6b, B.xin, B.w[0], r, z, part);
   else
-    k_lrn_finish<false><<<g0, LG_T, 0, st>>>(ctl, gate, g.n, B.l6, B.xin, B.w[0], r, q, z, part,
-                                             want_rr, want_zq);
+    k_lrn_finish<false><<<g0, LG_T, 0, st>>>(ctl, gate, g.n, B.l6, B.xin, B.w[0], r, z, part);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -543,16 +538,12 @@ static bool folded(const LearnedExt *L) { return L->exec != SG_MPNN_EXEC_LAYERED
 // x = L^-1 r; x += alpha p moves to K3.
 static int learned_k2(Solver *S, cudaStream_t st, int par) {
   LearnedExt *L = (LearnedExt *)S->ext;
-  // the TMA-staged and symmetric-storage K1 leave the p.q total in ctl
-  const int pq_fin = (S->tma || S->sym) ? 1 : 0;
   const mpnn::FoldBufs &B = L->G->fb;
   if (L->exec == SG_MPNN_EXEC_FOLDED)
-    mpnn::k_lrn_update<true><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->A.n, S->part1, S->P1,
-                                                      pq_fin, (const float *)S->q,
-                                                      (float *)S->r, B.l6b, B.xin);
+    mpnn::k_lrn_update<true><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->A.n, (const float *)S->q,
+                                                       (float *)S->r, B.l6b, B.xin);
   else
-    mpnn::k_lrn_update<false><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->A.n, S->part1, S->P1,
-                                                       pq_fin, (const float *)S->q,
+    mpnn::k_lrn_update<false><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->A.n, (const float *)S->q,
                                                        (float *)S->r, B.l6, B.xin);
   SG_CHECK_LAUNCH();
   return SG_OK;
@@ -565,10 +556,10 @@ static int learned_prec(Solver *S, cudaStream_t st, int par) {
     // decided (status, beta) in ctl for K3
     return mpnn::fold_apply(L->G, st, S->ctl, 1, L->exec == SG_MPNN_EXEC_FOLDED,
                             (const float *)S->r, (float *)S->z, (const float *)S->q, S->part2,
-                            S->np2_ext, 1, 1, true, true, S->ctl, par);
+                            S->np2_ext, S->ctl, par);
   SG_TRY(mpnn::forward(L->G, st, S->ctl, 1, L->prm, (const float *)S->r, (float *)S->z, false));
-  mpnn::k_rz_zq<<<S->P2, RED_T, 0, st>>>(S->ctl, S->len, (const float *)S->r, (const float *)S->z,
-                                         (const float *)S->q, S->part2);
+  mpnn::k_rz_zq<<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, (const float *)S->r,
+                                         (const float *)S->z, (const float *)S->q, S->part2);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -593,8 +584,7 @@ static int learned_apply(Solver *S, cudaStream_t st) {
     // the parameters may have changed since the last solve: fold them again
     SG_TRY(mpnn::fold_params(L->G, st, L->prm));
     return mpnn::fold_apply(L->G, st, S->ctl, 0, L->exec == SG_MPNN_EXEC_FOLDED,
-                            (const float *)S->r, (float *)S->z, nullptr, S->part3, S->P2, 0, 0,
-                            false);
+                            (const float *)S->r, (float *)S->z, nullptr, S->part3, S->P2);
   }
   SG_TRY(mpnn::forward(L->G, st, S->ctl, 0, L->prm, (const float *)S->r, (float *)S->z, false));
   k_rz_only<<<S->P2, RED_T, 0, st>>>(S->len, (const float *)S->r, (const float *)S->z, S->part3);
@@ -633,7 +623,6 @@ static int learned_setup(Solver *S) {
     SG_TRY(mpnn::ensure_folded(L->G));
     S->ext_k2 = learned_k2;
     S->k3_xupd = 1;
-    S->ext_decides = 1;
     // the last Horner step, with the end of the application folded in,
     // runs on the steps' grid and leaves that many partials per dot for K3
     int g0 = 0;
@@ -749,7 +738,7 @@ int sg_mpnn_forward(sg_mpnn_graph *hg, const float *params, const float *r, floa
   if (!train && G->exec != SG_MPNN_EXEC_LAYERED && G->g.sym) {
     SG_TRY(mpnn::fold_params(G, G->c->stream, params));
     return mpnn::fold_apply(G, G->c->stream, nullptr, 0, G->exec == SG_MPNN_EXEC_FOLDED, r, z,
-                            nullptr, nullptr, 0, 0, 0, false);
+                            nullptr, nullptr, 0);
   }
   if (train) SG_TRY(mpnn::ensure_train(G));
   return mpnn::forward(G, G->c->stream, nullptr, 0, params, r, z, train != 0);

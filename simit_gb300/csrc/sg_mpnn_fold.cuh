@@ -399,21 +399,18 @@ struct FoldBufs {
 // the solve status (gate); after a fallback to block Jacobi the steps do
 // nothing (k_lrn_finish then uses x).  AT: edge-weight type; FP16 weights
 // go with block-floating-point vectors.
-// The end of an application folded into the last Horner step (FIN): each
-// row's w_0 becomes z = L^-T w_0 at once, and the dots r.r, r.z, z.q of the
-// new z accumulate as it goes, one partial per CTA (grid-size apart, as
-// k_lrn_finish leaves them).  part null: z alone.
+// The end of an iteration's application folded into the last Horner step
+// (FIN): each row's w_0 becomes z = L^-T w_0 at once, the dots r.r, r.z, z.q
+// of the new z accumulate as it goes, and the CTA that finishes last sums the
+// partials (part: three per CTA) and makes the iteration's decision
+// (cg_decide: status, beta) for K3, which then only streams.
 struct FinArgs {
   const float *r = nullptr;
   const float *q = nullptr;
   float *z = nullptr;
   double *part = nullptr;
-  int want_rr = 0, want_zq = 0;
-  // decide (with all three dots): the CTA that finishes last also sums the
-  // partials and makes the iteration's decision (cg_decide: status, beta)
-  // for K3, which then only streams
   SolveCtl *ctl = nullptr;
-  int decide = 0, par = 0;
+  int par = 0;
 };
 
 constexpr int HT_WARPS = 4;   // warps per CTA
@@ -440,7 +437,6 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
   constexpr size_t STG = ht_stage_bytes<AT>();
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ float G[9], G6[9];
-  __shared__ double shd[33];
   if (ctl && gate && ctl->status != ST_RUNNING) return;
   // after a fallback to block Jacobi the steps do nothing, and the last one
   // (FIN) turns x itself into z = L^-T x
@@ -458,43 +454,27 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
     zp[0] = z0;
     zp[1] = z1;
     zp[2] = z2;
-    if (!fa.part) return;
-    const float *rp = fa.r + (size_t)v * 3;
+    const float *rp = fa.r + (size_t)v * 3, *qp = fa.q + (size_t)v * 3;
     const float r0 = rp[0], r1 = rp[1], r2 = rp[2];
-    if (fa.want_rr) {
-      rr.add(r0, r0);
-      rr.add(r1, r1);
-      rr.add(r2, r2);
-    }
+    rr.add(r0, r0);
+    rr.add(r1, r1);
+    rr.add(r2, r2);
     rz.add(r0, z0);
     rz.add(r1, z1);
     rz.add(r2, z2);
-    if (fa.want_zq) {
-      const float *qp = fa.q + (size_t)v * 3;
-      zq.add(z0, qp[0]);
-      zq.add(z1, qp[1]);
-      zq.add(z2, qp[2]);
-    }
+    zq.add(z0, qp[0]);
+    zq.add(z1, qp[1]);
+    zq.add(z2, qp[2]);
   };
   auto fin_partials = [&]() {
-    if (!FIN || !fa.part) return;
-    const double t1 = block_sum(rz.value(), shd);
-    const double t0 = fa.want_rr ? block_sum(rr.value(), shd) : 0.0;
-    const double t2 = fa.want_zq ? block_sum(zq.value(), shd) : 0.0;
-    if (fa.decide) {
-      // r.r | r.z | z.q, each gridDim.x partials, summed in index order by
-      // the last CTA, which decides the iteration
-      const double t[3] = {t0, t1, t2};
-      double tot[3];
-      if (finalize_partials(t, 3, fa.part, &fa.ctl->tick2, tot, shd) && threadIdx.x == 0)
-        cg_decide(fa.ctl, fa.par, tot[0], tot[1], tot[2], fa.ctl->last_alpha);
-      return;
-    }
-    if (threadIdx.x == 0) {
-      if (fa.want_rr) fa.part[blockIdx.x] = t0;
-      fa.part[(fa.want_rr ? gridDim.x : 0) + blockIdx.x] = t1;
-      if (fa.want_zq) fa.part[2 * gridDim.x + blockIdx.x] = t2;
-    }
+    if (!FIN) return;
+    // the stages are free: their memory holds the sums' operands
+    static_assert(ht_smem_bytes<AT>() >= SUM_OFF + 3 * HT_WARPS * 32 * 8, "sums");
+    const double v[3] = {rr.value(), rz.value(), zq.value()};
+    double t[3], tot[3];
+    block_sums<3>(v, t, sum_buf(sm));
+    if (finalize_partials<3>(t, fa.part, &fa.ctl->tick2, tot, sum_buf(sm)) && threadIdx.x == 0)
+      cg_decide(fa.ctl, fa.par, tot[0], tot[1], tot[2], fa.ctl->last_alpha);
   };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (FIN && fb) {
@@ -624,30 +604,25 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
 
 // The end of an application after the last Horner step wrote w_0:
 // z = L^-T w_0 (z = L^-T x = D^-1 r after a fallback to block Jacobi) and
-// the dot partials of the new z when part != null: r.r at part[0 .. np),
-// r.z at part[np .. 2np), z.q at part[2np .. 3np) (np = gridDim.x) when
-// want_rr / want_zq, else r.z alone at part[0 .. np).  A thread takes 4
-// vertices at a time in vertex order (three float4 each of r, q and z, six
-// of L^-1: r, q and z must be 16-byte aligned); the last n % 4 vertices go
-// to thread 0 of block 0.
+// with part, the partials of r.z (one per block).  A thread takes 4 vertices
+// at a time in vertex order (three float4 each of r and z, six of L^-1: r and
+// z must be 16-byte aligned); the last n % 4 vertices go to thread 0 of
+// block 0.
 template <bool CV>
 __global__ void __launch_bounds__(LG_T) k_lrn_finish(const SolveCtl *ctl, int gate, int32_t n,
                                                      const void *__restrict__ l6,
                                                      const void *__restrict__ xin,
                                                      const void *__restrict__ w0,
                                                      const float *__restrict__ r,
-                                                     const float *__restrict__ q,
                                                      float *__restrict__ z,
-                                                     double *__restrict__ part, int want_rr,
-                                                     int want_zq) {
+                                                     double *__restrict__ part) {
   __shared__ double sh[33];
   if (ctl && gate && ctl->status != ST_RUNNING) return;
   const bool fb = ctl && ctl->fallback;
   const void *w = fb ? xin : w0;
-  DotAcc<float> rr, rz, zq;
+  DotAcc<float> rz;
   const int64_t nu = n / 4;
   const float4 *r4 = reinterpret_cast<const float4 *>(r);
-  const float4 *q4 = reinterpret_cast<const float4 *>(q);
   float4 *z4 = reinterpret_cast<float4 *>(z);
   auto one = [&](const float *L, float a, float b, float c, float *zv) {
     // (L^-1)^T w, L^-1 = [[l0,0,0],[l1,l2,0],[l3,l4,l5]]
@@ -655,9 +630,9 @@ __global__ void __launch_bounds__(LG_T) k_lrn_finish(const SolveCtl *ctl, int ga
     zv[1] = L[2] * b + L[4] * c;
     zv[2] = L[5] * c;
   };
-  // four vertices: L^-1 in lv[24], z into zv[12], then the dot terms
+  // four vertices: L^-1 in lv[24], z into zv[12], then r.z's terms
   auto four = [&](int64_t v0, int cnt, const float *lv, bool vec) {
-    float zv[12], rv[12], qv[12];
+    float zv[12], rv[12];
     for (int j = 0; j < cnt; ++j) {
       float a, b, c;
       ld3<CV>(w, (size_t)(v0 + j), a, b, c);
@@ -676,22 +651,11 @@ __global__ void __launch_bounds__(LG_T) k_lrn_finish(const SolveCtl *ctl, int ga
       for (int k = 0; k < 3; ++k) {
         const float4 a4 = r4[v0 / 4 * 3 + k];
         rv[4 * k] = a4.x; rv[4 * k + 1] = a4.y; rv[4 * k + 2] = a4.z; rv[4 * k + 3] = a4.w;
-        if (want_zq) {
-          const float4 b4 = q4[v0 / 4 * 3 + k];
-          qv[4 * k] = b4.x; qv[4 * k + 1] = b4.y; qv[4 * k + 2] = b4.z; qv[4 * k + 3] = b4.w;
-        }
       }
     } else {
-      for (int k = 0; k < cnt * 3; ++k) {
-        rv[k] = r[v0 * 3 + k];
-        if (want_zq) qv[k] = q[v0 * 3 + k];
-      }
+      for (int k = 0; k < cnt * 3; ++k) rv[k] = r[v0 * 3 + k];
     }
-    for (int k = 0; k < cnt * 3; ++k) {
-      if (want_rr) rr.add(rv[k], rv[k]);
-      rz.add(rv[k], zv[k]);
-      if (want_zq) zq.add(zv[k], qv[k]);
-    }
+    for (int k = 0; k < cnt * 3; ++k) rz.add(rv[k], zv[k]);
   };
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nu;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -707,14 +671,8 @@ __global__ void __launch_bounds__(LG_T) k_lrn_finish(const SolveCtl *ctl, int ga
     four(nu * 4, cnt, lv, false);
   }
   if (!part) return;
-  const double t1 = block_sum(rz.value(), sh);
-  const double t0 = want_rr ? block_sum(rr.value(), sh) : 0.0;
-  const double t2 = want_zq ? block_sum(zq.value(), sh) : 0.0;
-  if (threadIdx.x == 0) {
-    if (want_rr) part[blockIdx.x] = t0;
-    part[(want_rr ? gridDim.x : 0) + blockIdx.x] = t1;
-    if (want_zq) part[2 * gridDim.x + blockIdx.x] = t2;
-  }
+  const double t = block_sum(rz.value(), sh);
+  if (threadIdx.x == 0) part[blockIdx.x] = t;
 }
 
 // x = L^-1 r for a fresh r (set-up, restarts and the standalone forward).
@@ -737,46 +695,50 @@ __global__ void k_lrn_xin(int32_t n, const void *__restrict__ l6, const float *_
 // n % 4 vertices go to thread 0 of the last CTA.
 template <bool CV>
 __global__ void __launch_bounds__(RED_T) k_lrn_update(SolveCtl *ctl, int par, int32_t n,
-                                                      const double *__restrict__ part_in,
-                                                      int np1, int pq_fin,
                                                       const float *__restrict__ q,
                                                       float *__restrict__ r,
                                                       const void *__restrict__ l6,
                                                       void *__restrict__ xin) {
-  __shared__ double sh[33];
+  __shared__ double sa;
   if (ctl->status != ST_RUNNING) return;
-  const double pq = pq_fin ? ctl->pq_tot : sum_parts(part_in, np1, sh);
-  if (!(pq > 0.0) || !isfinite(pq)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->status = isfinite(pq) ? ST_BREAKDOWN : ST_NAN;
-    return;
-  }
-  const double alpha = ctl->rz[par] / pq;
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->last_alpha = alpha;
-  const float a = (float)alpha;
   const int64_t nu = n / 4;
   const float4 *q4 = reinterpret_cast<const float4 *>(q);
   float4 *r4 = reinterpret_cast<float4 *>(r);
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu;
-       u += (int64_t)gridDim.x * blockDim.x) {
-    float rv[12], lv[24];
+  float4 qv[3], rq[3];
+  float lv[24];
+  auto load = [&](int64_t u) {
+    if (u >= nu) return;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      const float4 b = q4[u * 3 + k], c = r4[u * 3 + k];
-      rv[4 * k] = c.x - a * b.x;
-      rv[4 * k + 1] = c.y - a * b.y;
-      rv[4 * k + 2] = c.z - a * b.z;
-      rv[4 * k + 3] = c.w - a * b.w;
+      qv[k] = q4[u * 3 + k];
+      rq[k] = r4[u * 3 + k];
     }
     ld_linv4<CV>(l6, u, lv);
+  };
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  load(u);
+  double alpha;
+  float a;
+  if (!cg_alpha(ctl, par, &sa, &alpha, &a)) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->last_alpha = alpha;
+  for (; u < nu; u += step) {
+    float rv[12];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
+    for (int k = 0; k < 3; ++k) {
+      rv[4 * k] = rq[k].x - a * qv[k].x;
+      rv[4 * k + 1] = rq[k].y - a * qv[k].y;
+      rv[4 * k + 2] = rq[k].z - a * qv[k].z;
+      rv[4 * k + 3] = rq[k].w - a * qv[k].w;
       r4[u * 3 + k] = make_float4(rv[4 * k], rv[4 * k + 1], rv[4 * k + 2], rv[4 * k + 3]);
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float *L = lv + 6 * j, *R = rv + 3 * j;
       st3<CV>(xin, (size_t)(u * 4 + j), L[0] * R[0], L[1] * R[0] + L[2] * R[1],
               L[3] * R[0] + L[4] * R[1] + L[5] * R[2]);
     }
+    load(u + step);
   }
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
     for (int64_t v = nu * 4; v < n; ++v) {

@@ -16,7 +16,9 @@ namespace sg {
 
 __global__ void k_sum_parts(const double *part, int np, double *out) {
   __shared__ double sh[33];
-  double t = sum_parts(part, np, sh);
+  double a = 0;
+  for (int i = threadIdx.x; i < np; i += blockDim.x) a += part[i];
+  const double t = block_sum(a, sh);
   if (threadIdx.x == 0) *out = t;
 }
 
@@ -119,6 +121,7 @@ __global__ void k_f32_to_f64(int64_t len, const float *__restrict__ a, double *_
 }
 
 // ---------------------------------------------------------------------------
+constexpr int FIRST_ITERS = 8;  // even: a batch begins in parity slot 0
 enum Kind { KIND_F64 = 0, KIND_F64_M32 = 1, KIND_MIXED = 2 };
 
 static int dot_grid(const Ctx *c, int64_t len) { return grid_for(c, len, RED_T, 4); }
@@ -164,105 +167,119 @@ static int launch_k1(Solver *S, cudaStream_t st) {
   return SG_OK;
 }
 
-template <int PREC>
-static void launch_k2_v4(Solver *S, cudaStream_t st, int par) {
-  k_cg_update_v4<PREC, PREC != PK_EXTERNAL><<<S->P2, RED_T, 0, st>>>(
-      S->ctl, par, S->len, S->part1, S->P1, S->tma, (const float *)S->p, (const float *)S->q,
-      (float *)S->r, (float *)S->xupd, (float *)S->z, (const float *)S->dinv, S->part2);
-}
-
-template <typename VT, typename XT>
-static int launch_k2(Solver *S, cudaStream_t st, int par) {
-  if (S->ext_k2) return S->ext_k2(S, st, par);
-  const VT *p = (const VT *)S->p, *q = (const VT *)S->q, *dinv = (const VT *)S->dinv;
-  VT *r = (VT *)S->r, *z = (VT *)S->z;
-  XT *x = (XT *)S->xupd;
-  if (sizeof(VT) == 4 && sizeof(XT) == 4) {
-    switch (S->prec) {
-      case PK_NONE: launch_k2_v4<PK_NONE>(S, st, par); break;
-      case PK_JACOBI: launch_k2_v4<PK_JACOBI>(S, st, par); break;
-      case PK_BLOCK3: {
-        static PerDeviceOnce attr;
-        const size_t sm = K2W_WARPS * sizeof(K2WarpSmem);
-        SG_TRY(once_per_device(attr, S->c->device, [&]() -> int {
-          SG_CHECK_CUDA(cudaFuncSetAttribute(k_cg_update_w<true, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-          return SG_OK;
-        }));
-        const int64_t nchunks = (S->len / 12 + 31) / 32;
-        int64_t grid = (nchunks + K2W_WARPS - 1) / K2W_WARPS;
-        // 2 CTAs of 8 warps per SM (3 fit, and measured 3 % slower per step)
-        if (grid > 2 * (int64_t)S->c->num_sms) grid = 2 * (int64_t)S->c->num_sms;
-        if (grid < 1) grid = 1;
-        S->k3_xupd = 1;  // x += alpha p moves to K3
-        SG_CHECK_CUDA(launch_k(S->c, k_cg_update_w<true, false>, (int)grid, K2W_WARPS * 32, sm, st,
-                               S->ctl, par, S->len, (const double *)S->part1, S->P1, S->tma,
-                               (const float *)S->p, (const float *)S->q, (float *)S->r,
-                               (float *)S->xupd, (float *)S->z, (const float *)S->dinv,
-                               S->part2));
-        break;
-      }
-      default: launch_k2_v4<PK_EXTERNAL>(S, st, par); break;
-    }
-    SG_CHECK_LAUNCH();
+static int launch_k2_f32(Solver *S, cudaStream_t st, int par) {
+  const float *p = (const float *)S->p, *q = (const float *)S->q, *dinv = (const float *)S->dinv;
+  float *r = (float *)S->r, *x = (float *)S->xupd, *z = (float *)S->z;
+  if (S->prec == PK_BLOCK3) {
+    static PerDeviceOnce attr;
+    SG_TRY(once_per_device(attr, S->c->device, []() -> int {
+      SG_CHECK_CUDA(cudaFuncSetAttribute(k_cg_update_w, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)(K2W_WARPS * sizeof(K2WarpSmem))));
+      return SG_OK;
+    }));
+    // one chunk per warp while that fills the SMs, a block per SM: the warps
+    // spread over all SMs before a block gets a second one.  At most 2 blocks
+    // of 8 warps per SM (3 measured 3 % slower per step at 128^3).
+    const int64_t nchunks = (S->len / 12 + 31) / 32, sms = S->c->num_sms;
+    int64_t warps = (nchunks + sms - 1) / sms;
+    warps = warps < 1 ? 1 : warps > K2W_WARPS ? K2W_WARPS : warps;
+    int64_t grid = (nchunks + warps - 1) / warps;
+    grid = grid < 1 ? 1 : grid > 2 * sms ? 2 * sms : grid;
+    SG_CHECK_CUDA(launch_k(S->c, k_cg_update_w, (int)grid, (int)warps * 32,
+                           (size_t)warps * sizeof(K2WarpSmem), st, S->ctl, par, S->len, q, r, z,
+                           dinv, S->part2));
     return SG_OK;
   }
   switch (S->prec) {
     case PK_NONE:
-      k_cg_update<VT, XT, PK_NONE><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, S->part1, S->P1,
-                                                            p, q, r, x, z, dinv, S->part2);
+      k_cg_update_v4<PK_NONE><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z, dinv,
+                                                       S->part2);
       break;
     case PK_JACOBI:
-      k_cg_update<VT, XT, PK_JACOBI><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, S->part1,
-                                                              S->P1, p, q, r, x, z, dinv, S->part2);
-      break;
-    case PK_BLOCK3:
-      k_cg_update<VT, XT, PK_BLOCK3><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, S->part1,
-                                                              S->P1, p, q, r, x, z, dinv, S->part2);
+      k_cg_update_v4<PK_JACOBI><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z, dinv,
+                                                         S->part2);
       break;
     default:
-      k_cg_update<VT, XT, PK_EXTERNAL><<<S->P2, RED_T, 0, st>>>(
-          S->ctl, par, S->len, S->part1, S->P1, p, q, r, x, z, dinv, S->part2);
+      k_cg_update_v4<PK_EXTERNAL><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z,
+                                                           dinv, S->part2);
       break;
   }
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
 
-template <typename VT>
-static int launch_k3(Solver *S, cudaStream_t st, int par) {
-  const VT *z = (const VT *)(S->prec == PK_NONE ? S->r : S->z);
-  const int np2 = S->np2_ext > 0 ? S->np2_ext : S->P2;
-  // K2 decided, unless an external preconditioner ran after it and did not
-  if (sizeof(VT) == 4)
-    SG_CHECK_CUDA(launch_k(S->c, k_cg_direction_v4, S->P2, RED_T, 0, st, S->ctl, par, S->len,
-                           (const double *)S->part2, np2,
-                           (int)(S->prec != PK_EXTERNAL || S->ext_decides),
-                           (const float *)z, (float *)S->p, (float *)S->xupd, S->k3_xupd));
-  else
-    k_cg_direction<VT><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->len, S->part2, S->P2, z,
-                                                (VT *)S->p);
+// FP64 vectors: two entries (or a vertex) per thread, four blocks per SM.
+static int k2_grid_f64(const Solver *S) {
+  return grid_for(S->c, S->prec == PK_BLOCK3 ? S->len / 3 : (S->len + 1) / 2, RED_T, 4);
+}
+
+static int launch_k2_f64(Solver *S, cudaStream_t st, int par) {
+  const double *p = (const double *)S->p, *q = (const double *)S->q;
+  const double *dinv = (const double *)S->dinv;
+  double *r = (double *)S->r, *x = (double *)S->xupd, *z = (double *)S->z;
+  const int grid = k2_grid_f64(S);
+  switch (S->prec) {
+    case PK_NONE:
+      k_cg_update_f64<PK_NONE><<<grid, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z, dinv,
+                                                       S->part2);
+      break;
+    case PK_JACOBI:
+      k_cg_update_f64<PK_JACOBI><<<grid, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z, dinv,
+                                                         S->part2);
+      break;
+    default:
+      k_cg_update_f64<PK_BLOCK3><<<grid, RED_T, 0, st>>>(S->ctl, par, S->len, p, q, r, x, z, dinv,
+                                                         S->part2);
+      break;
+  }
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
 
-template <typename MT, typename VT, typename XT>
+static int launch_k3(Solver *S, cudaStream_t st) {
+  const void *z = S->prec == PK_NONE ? S->r : S->z;
+  if (S->kind == KIND_MIXED)
+    SG_CHECK_CUDA(launch_k(S->c, k_cg_direction_v4, grid_for(S->c, S->len / 4, RED_T, 8), RED_T, 0,
+                           st, (const SolveCtl *)S->ctl, S->len, (const float *)z, (float *)S->p,
+                           (float *)S->xupd, S->k3_xupd));
+  else
+    k_cg_direction_f64<<<grid_for(S->c, (S->len + 1) / 2, RED_T, 8), RED_T, 0, st>>>(
+        S->ctl, S->len, (const double *)z, (double *)S->p);
+  SG_CHECK_LAUNCH();
+  return SG_OK;
+}
+
+// One iteration on st; par: its parity slot (the first of a batch has 0).
+template <typename MT, typename VT>
+static int launch_iteration(Solver *S, cudaStream_t st, int par) {
+  int rc = launch_k1<MT, VT>(S, st);
+  if (rc == SG_OK)
+    rc = S->ext_k2 ? S->ext_k2(S, st, par)
+         : S->kind == KIND_MIXED ? launch_k2_f32(S, st, par) : launch_k2_f64(S, st, par);
+  if (rc == SG_OK && S->ext_prec) rc = S->ext_prec(S, st, par);
+  if (rc == SG_OK) rc = launch_k3(S, st);
+  return rc;
+}
+
+// count iterations enqueued one by one, from parity slot 0.
+template <typename MT, typename VT>
+static int launch_iterations(Solver *S, int count) {
+  // optional programmatic dependent launch for the kernels launched through
+  // launch_k (K1 per-warp TMA SpMV, K2 warp-staged update, K3 FP32 direction)
+  S->c->pdl = S->o.pdl != 0;
+  int rc = SG_OK;
+  for (int k = 0; k < count && rc == SG_OK; ++k)
+    rc = launch_iteration<MT, VT>(S, S->c->stream, k & 1);
+  S->c->pdl = false;
+  return rc;
+}
+
+template <typename MT, typename VT>
 static int capture_batch(Solver *S) {
   cudaStream_t st = S->c->stream;
   cudaGraph_t g = nullptr;
   SG_CHECK_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-  int rc = SG_OK;
-  // optional programmatic dependent launch for the kernels launched through
-  // launch_k (K1 per-warp TMA SpMV, K2 warp-staged update, K3 FP32 direction)
-  S->c->pdl = S->o.pdl != 0;
-  for (int k = 0; k < S->batch && rc == SG_OK; ++k) {
-    const int par = k & 1;
-    rc = launch_k1<MT, VT>(S, st);
-    if (rc == SG_OK) rc = launch_k2<VT, XT>(S, st, par);
-    if (rc == SG_OK && S->ext_prec) rc = S->ext_prec(S, st, par);
-    if (rc == SG_OK) rc = launch_k3<VT>(S, st, par);
-  }
-  S->c->pdl = false;
+  const int rc = launch_iterations<MT, VT>(S, S->batch);
   cudaError_t e = cudaStreamEndCapture(st, &g);
   if (rc != SG_OK) {
     if (g) cudaGraphDestroy(g);
@@ -277,8 +294,17 @@ static int capture_batch(Solver *S) {
   return SG_OK;
 }
 
-// r_hi = b - A x_hi in FP64 (FP64 accumulation); returns ||r_hi||^2 (sync).
-static int true_residual(Solver *S, const double *b, double *rr) {
+// dres[0 .. count) to the host: the wait for everything enqueued so far.
+static int read_sums(Solver *S, int count, double *out) {
+  cudaStream_t st = S->c->stream;
+  SG_CHECK_CUDA(cudaMemcpyAsync(S->c->h_stage, S->dres, 8 * count, cudaMemcpyDeviceToHost, st));
+  SG_CHECK_CUDA(cudaStreamSynchronize(st));
+  memcpy(out, S->c->h_stage, 8 * count);
+  return SG_OK;
+}
+
+// r_hi = b - A x_hi in FP64 (FP64 accumulation), ||r_hi||^2 into *out.
+static int true_residual(Solver *S, const double *b, double *out) {
   const sg_matrix &A = S->A;
   S->launches += 2;
   cudaStream_t st = S->c->stream;
@@ -303,17 +329,14 @@ static int true_residual(Solver *S, const double *b, double *rr) {
                                                         S->part3);
   }
   SG_CHECK_LAUNCH();
-  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, PT, S->dres);
+  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, PT, out);
   SG_CHECK_LAUNCH();
-  SG_CHECK_CUDA(cudaMemcpyAsync(S->c->h_stage, S->dres, 8, cudaMemcpyDeviceToHost, st));
-  SG_CHECK_CUDA(cudaStreamSynchronize(st));
-  *rr = *(double *)S->c->h_stage;
   return SG_OK;
 }
 
 // The same residual from the float split of x_hi without FP64 multiply-adds
 // (k_true_residual3c); S->xsplit must hold the split of the current x_hi.
-static int true_residual_fast(Solver *S, const double *b, double *rr) {
+static int true_residual_fast(Solver *S, const double *b, double *out) {
   const sg_matrix &A = S->A;
   S->launches += 2;
   cudaStream_t st = S->c->stream;
@@ -322,17 +345,14 @@ static int true_residual_fast(Solver *S, const double *b, double *rr) {
                                              S->xsplit, S->xsplit + S->len, b, S->rhi,
                                              S->part3);
   SG_CHECK_LAUNCH();
-  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, PT, S->dres);
+  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, PT, out);
   SG_CHECK_LAUNCH();
-  SG_CHECK_CUDA(cudaMemcpyAsync(S->c->h_stage, S->dres, 8, cudaMemcpyDeviceToHost, st));
-  SG_CHECK_CUDA(cudaStreamSynchronize(st));
-  *rr = *(double *)S->c->h_stage;
   return SG_OK;
 }
 
-// r = (VT) r_hi; z = M r (or the external preconditioner); returns r.z (sync).
+// r = (VT) r_hi; z = M r (or the external preconditioner); r.z into *out.
 template <typename VT>
-static int restart_from_rhi(Solver *S, double *rz) {
+static int restart_from_rhi(Solver *S, double *out) {
   cudaStream_t st = S->c->stream;
   S->launches += 3;
   k_cast_r<VT><<<S->P2, RED_T, 0, st>>>(S->len, S->rhi, (VT *)S->r);
@@ -356,11 +376,8 @@ static int restart_from_rhi(Solver *S, double *rz) {
     }
     SG_CHECK_LAUNCH();
   }
-  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, S->P2, S->dres);
+  k_sum_parts<<<1, RED_T, 0, st>>>(S->part3, S->P2, out);
   SG_CHECK_LAUNCH();
-  SG_CHECK_CUDA(cudaMemcpyAsync(S->c->h_stage, S->dres, 8, cudaMemcpyDeviceToHost, st));
-  SG_CHECK_CUDA(cudaStreamSynchronize(st));
-  *rz = *(double *)S->c->h_stage;
   return SG_OK;
 }
 
@@ -378,11 +395,30 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
   SG_CHECK_CUDA(cudaMemsetAsync(S->ctl, 0, sizeof(SolveCtl), st));
   if (mixed) SG_CHECK_CUDA(cudaMemsetAsync(S->xlo, 0, S->len * sizeof(XT), st));
   // b'b
+  const bool fast = S->xsplit != nullptr;
+  // b.b, the start's r.r and r.z, read with one wait where the residual to
+  // start from does not depend on the tolerance (below: it may be FP32)
+  double start[3] = {0, 0, 0};
+  const bool one_wait = S->x_zero || !fast;
   dot_launch(c, S->len, b, b, S->part3, S->dres);
   S->launches += 2;
-  SG_CHECK_CUDA(cudaMemcpyAsync(c->h_stage, S->dres, 8, cudaMemcpyDeviceToHost, st));
-  SG_CHECK_CUDA(cudaStreamSynchronize(st));
-  const double bb = *(double *)c->h_stage;
+  const void *z = S->prec == PK_NONE ? S->r : S->z;
+  auto first_direction = [&]() -> int {
+    SG_CHECK_CUDA(cudaMemcpyAsync(S->p, z, S->len * sizeof(VT), cudaMemcpyDeviceToDevice, st));
+    return SG_OK;
+  };
+  if (one_wait) {
+    if (S->x_zero)  // the residual is b itself, exactly (no SpMV)
+      SG_CHECK_CUDA(cudaMemcpyAsync(S->rhi, b, S->len * 8, cudaMemcpyDeviceToDevice, st));
+    else
+      SG_TRY(true_residual(S, b, S->dres + 1));
+    SG_TRY(restart_from_rhi<VT>(S, S->dres + 2));
+    SG_TRY(first_direction());
+    SG_TRY(read_sums(S, 3, start));
+  } else {
+    SG_TRY(read_sums(S, 1, start));
+  }
+  const double bb = start[0];
   res->bnorm2 = bb;
   double tol2;
   switch (S->o.stop) {
@@ -393,15 +429,19 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
   // Checks run the compensated FP32 residual when the matrix is FP32; one
   // that meets the tolerance (with 10 % slack in the norm) is recomputed with
   // FP64 accumulation, and only that decides convergence.
-  const bool fast = S->xsplit != nullptr;
   bool exact = false;  // the last residual was the FP64 one
+  // The residual that decides convergence most often finds it, so x goes out
+  // with it (unless x overlaps b, which a further check would read).
+  bool sent = false;
+  const bool apart = x + S->len <= b || b + S->len <= x;
   auto check = [&](double *out) -> int {
     if (fast) {
       k_fold_split<XT><<<S->P2, RED_T, 0, st>>>(S->len, S->xw, (XT *)S->xlo, S->xsplit,
                                                  S->xsplit + S->len);
       SG_CHECK_LAUNCH();
       S->launches += 1;
-      SG_TRY(true_residual_fast(S, b, out));
+      SG_TRY(true_residual_fast(S, b, S->dres));
+      SG_TRY(read_sums(S, 1, out));
       if (std::isfinite(*out) && *out > 1.21 * tol2) {
         exact = false;
         return SG_OK;
@@ -412,26 +452,29 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
       S->launches += 1;
     }
     exact = true;
-    return true_residual(S, b, out);
+    SG_TRY(true_residual(S, b, S->dres));
+    if (apart) {
+      SG_CHECK_CUDA(cudaMemcpyAsync(x, S->xw, S->len * 8, cudaMemcpyDeviceToDevice, st));
+      sent = true;
+    }
+    return read_sums(S, 1, out);
   };
-  double rr = 0;
-  if (S->x_zero) {
-    // x = 0: the residual is b itself, exactly (no SpMV, no split of x)
-    SG_CHECK_CUDA(cudaMemcpyAsync(S->rhi, b, S->len * 8, cudaMemcpyDeviceToDevice, st));
-    rr = bb;
-    exact = true;
-  } else {
-    SG_TRY(check(&rr));
-  }
+  double rr = S->x_zero ? bb : start[1];
+  exact = true;
+  if (!one_wait) SG_TRY(check(&rr));
   res->normr2 = rr;
   res->true_normr2 = rr;
   int iters = 0;
   int status = 0;
   if (!(rr > tol2)) status = SG_STATUS_CONVERGED;
   if (!std::isfinite(rr)) status = SG_STATUS_NAN;
-  double rz = 0;
+  double rz = start[2];
   int fallback = 0;
-  if (!status) SG_TRY(restart_from_rhi<VT>(S, &rz));
+  if (!status && !one_wait) {
+    SG_TRY(restart_from_rhi<VT>(S, S->dres));
+    SG_TRY(first_direction());
+    SG_TRY(read_sums(S, 1, &rz));
+  }
   if (!status && S->flexible && !(rz > 0.0)) {
     // the variable preconditioner gives no descent direction from the start:
     // switch to its fallback (block Jacobi) before the first iteration
@@ -440,11 +483,9 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
     const int one = 1;
     SG_CHECK_CUDA(cudaMemcpyAsync((char *)S->ctl + offsetof(SolveCtl, fallback), &one,
                                   sizeof(int), cudaMemcpyHostToDevice, st));
-    SG_TRY(restart_from_rhi<VT>(S, &rz));
-  }
-  if (!status) {
-    const VT *z = (const VT *)(S->prec == PK_NONE ? S->r : S->z);
-    SG_CHECK_CUDA(cudaMemcpyAsync(S->p, z, S->len * sizeof(VT), cudaMemcpyDeviceToDevice, st));
+    SG_TRY(restart_from_rhi<VT>(S, S->dres));
+    SG_TRY(first_direction());
+    SG_TRY(read_sums(S, 1, &rz));
   }
   const double delta = S->o.reliable_delta > 0 ? S->o.reliable_delta : 0.1;
   double rr_ref = rr;
@@ -466,9 +507,19 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
       break;
     }
     SG_CHECK_CUDA(cudaMemcpyAsync(S->ctl, h, sizeof(SolveCtl), cudaMemcpyHostToDevice, st));
-    for (;;) {
-      SG_CHECK_CUDA(cudaGraphLaunch(S->gexec, st));
-      S->launches += S->graph_kernels;
+    // A solve's first iterations are launched one by one: one that ends
+    // within them does not run the rest of a graph's batch, whose kernels
+    // cost 1.8 us each although they return at once (a spring step of 5
+    // iterations spent 150 of its 350 us on them), and a longer one pays a
+    // wait (about 10 us) once.  Not after a residual replacement.
+    for (int lead = iters == 0 ? FIRST_ITERS : 0;; lead = 0) {
+      if (lead > 0 && lead < S->batch) {
+        SG_TRY((launch_iterations<MT, VT>(S, lead)));
+        S->launches += S->graph_kernels / S->batch * lead;
+      } else {
+        SG_CHECK_CUDA(cudaGraphLaunch(S->gexec, st));
+        S->launches += S->graph_kernels;
+      }
       SG_CHECK_CUDA(cudaMemcpyAsync(h, S->ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, st));
       SG_CHECK_CUDA(cudaStreamSynchronize(st));
       if (h->status != ST_RUNNING) break;
@@ -484,7 +535,7 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
         break;
       }
     }
-    exact = false;  // x moved since the last residual
+    exact = sent = false;  // x moved since the last residual
     if (S->k3_xupd && (h->status == ST_NEED_CHECK || h->status == ST_MAXITER)) {
       // K2 updated r with alpha and stopped the batch; K3 returned early
       k_x_pending<<<S->P2, RED_T, 0, st>>>(S->len, (float)h->last_alpha, (const float *)S->p,
@@ -528,14 +579,22 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
     }
     const double rz_old = h->rz[cur ^ 1];
     double rz_new = 0;
-    SG_TRY(restart_from_rhi<VT>(S, &rz_new));
-    const VT *z = (const VT *)(S->prec == PK_NONE ? S->r : S->z);
-    k_p_update<VT><<<S->P2, RED_T, 0, st>>>(S->len, z, switched ? 0.0 : rz_new / rz_old,
+    SG_TRY(restart_from_rhi<VT>(S, S->dres));
+    SG_TRY(read_sums(S, 1, &rz_new));
+    k_p_update<VT><<<S->P2, RED_T, 0, st>>>(S->len, (const VT *)z, switched ? 0.0 : rz_new / rz_old,
                                             (VT *)S->p);
     S->launches += 1;
     SG_CHECK_LAUNCH();
     rz = rz_new;
     rr_ref = rr;
+  }
+  if (status == SG_STATUS_CONVERGED && exact && sent) {
+    // converged on an FP64 residual of the x that went out with it
+    res->true_normr2 = rr;
+    res->status = status;
+    res->iters = iters;
+    res->kernels = S->launches;
+    return SG_OK;
   }
   if (mixed && status) {
     k_add_lo<XT><<<S->P2, RED_T, 0, st>>>(S->len, S->xw, (XT *)S->xlo);
@@ -549,7 +608,8 @@ static int solve_impl(Solver *S, const double *b, double *x, sg_solve_result *re
     res->true_normr2 = rr;
   } else if (S->o.verify || mixed) {
     double rt = 0;
-    SG_TRY(true_residual(S, b, &rt));
+    SG_TRY(true_residual(S, b, S->dres));
+    SG_TRY(read_sums(S, 1, &rt));
     res->true_normr2 = rt;
   } else {
     res->true_normr2 = rr;
@@ -817,9 +877,12 @@ int solver_init(Ctx *c, const sg_matrix *A, const sg_solve_opts *o_in, Solver *S
     S->tma = 1;  // K1 leaves the finished p.q in ctl, as the TMA kernels do
     S->P1 = S->sym->grid[1];
   }
-  // part3 also takes b.b's partials, whose grid can be the largest of the three
+  // part3 also takes b.b's partials, whose grid can be the largest of them all
   int np = S->P1 > S->P2 ? S->P1 : S->P2;
   if (dot_grid(c, S->len) > np) np = dot_grid(c, S->len);
+  if (S->kind != KIND_MIXED && k2_grid_f64(S) > np) np = k2_grid_f64(S);
+  // the FP32 block-Jacobi K2 (k_cg_update_w) leaves x += alpha p to K3
+  S->k3_xupd = S->kind == KIND_MIXED && S->prec == PK_BLOCK3;
   SG_TRY(alloc_dev(S, (void **)&S->ctl, sizeof(SolveCtl)));
   SG_CHECK_CUDA(cudaMallocHost((void **)&S->hctl, sizeof(SolveCtl)));
   SG_TRY(alloc_dev(S, &S->r, S->len * vt));
@@ -848,9 +911,9 @@ int solver_init(Ctx *c, const sg_matrix *A, const sg_solve_opts *o_in, Solver *S
   SG_TRY(refresh_matrix(S));
   if (ext_setup) SG_TRY(ext_setup(S));
   switch (S->kind) {
-    case KIND_F64: return capture_batch<double, double, double>(S);
-    case KIND_F64_M32: return capture_batch<float, double, double>(S);
-    default: return capture_batch<float, float, float>(S);
+    case KIND_F64: return capture_batch<double, double>(S);
+    case KIND_F64_M32: return capture_batch<float, double>(S);
+    default: return capture_batch<float, float>(S);
   }
 }
 

@@ -37,19 +37,17 @@ struct Solver {
   std::vector<void *> allocs;
   // External preconditioner hooks (learned preconditioner).  ext_prec runs
   // inside the captured iteration between K2 and K3 (par: the iteration's
-  // parity slot): z = M(r) and the partials rr | rz | zq into part2, or,
-  // with ext_decides, the iteration already decided in ctl (status, beta),
-  // so that K3 only streams.  ext_prec_apply: z = M(r) and the partials of
+  // parity slot): z = M(r), and the iteration decided in ctl (status, beta) from
+  // the partials rr | rz | zq at part2, so that K3 only streams.  ext_prec_apply: z = M(r) and the partials of
   // r.z into part3 (set-up / restart).
   int (*ext_prec)(Solver *, cudaStream_t, int par) = nullptr;
-  int ext_decides = 0;
   int (*ext_prec_apply)(Solver *, cudaStream_t) = nullptr;
   void (*ext_free)(Solver *) = nullptr;
   // ext_k2 (optional) replaces the iteration's K2 (the folded learned
   // iteration's r update and x = L^-1 r)
   int (*ext_k2)(Solver *, cudaStream_t, int par) = nullptr;
-  // > 0: K3 sums this many partials per dot (the external preconditioner's
-  // last kernel wrote them with its own grid), else P2
+  // partials per dot of the external preconditioner's last kernel, if it runs
+  // on its own grid (part2 has room for them)
   int np2_ext = 0;
   // sg_solver_solve_ex: the FP64 copy of an FP32 right-hand side (allocated
   // on first use) and a zero initial guess for the current solve

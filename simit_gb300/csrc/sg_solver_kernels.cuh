@@ -11,8 +11,12 @@
 //                                   + partial sums of r.r, r.z (and z.q)
 //   K3  beta; p = z + beta p; decide RUNNING / NEED_CHECK / MAXITER
 // Every dot is an FP64 two-level sum: per-block partials in a fixed order,
-// then each consumer block re-sums the partials in the same fixed order, so
-// all blocks see identical scalars and results are run-to-run deterministic.
+// which the block that finishes last adds in index order, so results are
+// run-to-run deterministic.  This GPU issues one FP64 warp instruction per SM
+// every 16 cycles, however many lanes are active, so what the scalars cost is
+// counted in warp instructions: sums are packed into full warps (block_sums),
+// alpha is divided out by one warp per block while the block's vectors are
+// on their way (cg_alpha), beta by one thread of the grid (cg_decide).
 // Scalars that change per iteration live in two slots indexed by iteration
 // parity, so no kernel reads a slot that another block of the same kernel
 // writes.  A batch of iterations is captured once in a CUDA graph; kernels
@@ -54,6 +58,7 @@ struct SolveCtl {
   // the next write from the last read.
   double pq_tot;
   double beta;
+  float alpha32, beta32;  // last_alpha and beta rounded, for the FP32 kernels
   unsigned int tick1, tick2;
 };
 
@@ -75,54 +80,118 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return sh[32];
 }
 
-// Sum of np partials (every block computes the same value).
-__device__ __forceinline__ double sum_parts(const double *part, int np, double *sh) {
-  double a = 0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) a += part[i];
-  return block_sum(a, sh);
+// Block-wide FP64 sums of NV values per thread (NV <= 3, at most 8 full
+// warps), result in every lane of warp 0.  The additions are those of
+// block_sum, pair by pair, so the sums have the same bits; but between the
+// levels the operands go through shared memory (buf: NV * blockDim.x values)
+// and fill whole warps, because a warp instruction costs the same with one
+// active lane as with 32: three sums of 256 threads take 28 FP64 warp
+// instructions where three block_sums take 135 (0.23 against 1.1 us of the
+// SM's FP64 pipe per block).
+template <int NV>
+__device__ __forceinline__ void block_sums(const double *v, double *out, double *buf) {
+  const int T = blockDim.x, t = threadIdx.x;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) buf[k * T + t] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int L = 16; L >= 4; L >>= 1) {
+    for (int i = t; i < NV * T / 32 * L; i += T) {
+      double *e = buf + i / L * 32 + i % L;
+      e[0] += e[L];
+    }
+    __syncthreads();
+  }
+  if (t < 32) {
+    const int nw = T / 32, k = t / 8, w = t % 8;
+    double s = 0.0;
+    if (k < NV && w < nw) {
+      const double *e = buf + (k * nw + w) * 32;
+      s = (e[0] + e[2]) + (e[1] + e[3]);
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 8);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) out[j] = __shfl_sync(0xffffffffu, s, j * 8);
+  }
+}
+
+// The staged products keep block_sums' buffer (one sum) in their dynamic
+// shared memory, past the barriers; they ask for at least SUM_SMEM bytes.
+constexpr size_t SUM_OFF = 512, SUM_SMEM = SUM_OFF + RED_T * sizeof(double);
+__device__ __forceinline__ double *sum_buf(unsigned char *sm) {
+  return reinterpret_cast<double *>(sm + SUM_OFF);
 }
 
 template <typename T> __device__ __forceinline__ bool finite_(T v) { return isfinite(v); }
 
-// Last-CTA finalisation of per-CTA partial sums (nv arrays of gridDim.x
-// values at part, part + gridDim.x, ...): every CTA stores its partials and
+// Last-CTA finalisation of per-CTA sums (t: this block's NV sums, in thread
+// 0; part: NV arrays of gridDim.x values): every CTA stores its partials and
 // takes a ticket; the CTA that takes the last ticket sums each array in index
-// order (so the totals are deterministic), stores them in tot[0..nv) and
-// re-arms the ticket.  Returns true in that CTA.  Called by all threads;
-// nv <= 3.
-__device__ __forceinline__ bool finalize_partials(const double *t, int nv, double *part,
+// order (so the totals are deterministic), leaves them in tot[0..NV) of
+// thread 0 and re-arms the ticket.  Returns true in that CTA.  Called by all
+// threads; buf as in block_sums.
+template <int NV>
+__device__ __forceinline__ bool finalize_partials(const double *t, double *part,
                                                   unsigned int *ticket, double *tot,
-                                                  double *sh) {
+                                                  double *buf) {
   __shared__ int last;
   if (threadIdx.x == 0) {
-    for (int k = 0; k < nv; ++k) part[k * gridDim.x + blockIdx.x] = t[k];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) part[k * gridDim.x + blockIdx.x] = t[k];
     __threadfence();
     last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  // all nv arrays loaded in one pass (the last CTA works alone here, so its
-  // load latency is the kernel's tail), then reduced one after the other
-  double a[3] = {0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x)
+  // all NV arrays loaded in one pass (the last CTA works alone here, so its
+  // load latency is the kernel's tail)
+  double a[NV];
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-      if (k < nv) a[k] += __ldcg(part + k * gridDim.x + i);
+  for (int k = 0; k < NV; ++k)
+    a[k] = threadIdx.x < gridDim.x ? __ldcg(part + k * gridDim.x + threadIdx.x) : 0.0;
+  for (int i = threadIdx.x + blockDim.x; i < (int)gridDim.x; i += blockDim.x)
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    if (k >= nv) break;
-    const double s = block_sum(a[k], sh);
-    if (threadIdx.x == 0) tot[k] = s;
-  }
+    for (int k = 0; k < NV; ++k) a[k] += __ldcg(part + k * gridDim.x + i);
+  block_sums<NV>(a, tot, buf);
   if (threadIdx.x == 0) *ticket = 0;
   return true;
 }
 
-// The control decision after K2's dots (shared by the finalising K2 and the
-// reducing K3): iteration count, r.z slot, status, beta.  Executed by one
-// thread; returns the new status.
-__device__ __forceinline__ int cg_decide(SolveCtl *ctl, int par, double rr, double rznew,
+// alpha = r.z / p.q for every thread of a K2 block: one warp divides (24
+// warps of an SM doing so each would hold its FP64 pipe for 3 us) and the
+// others wait at the barrier, with their loads in flight.  False when p.q is
+// not a positive finite number; the last block to find so sets the status
+// (not before: a block reads it at its start).  sa: shared.
+__device__ __forceinline__ bool cg_alpha(SolveCtl *ctl, int par, double *sa, double *alpha,
+                                         float *alpha32) {
+  __shared__ int ok;
+  __shared__ float sf;
+  if (threadIdx.x < 32) {
+    const double pq = ctl->pq_tot;
+    const double a = ctl->rz[par] / pq;
+    if (threadIdx.x == 0) {
+      ok = pq > 0.0 && isfinite(pq);
+      *sa = a;
+      sf = (float)a;
+    }
+  }
+  __syncthreads();
+  if (!ok && threadIdx.x == 0 && atomicAdd(&ctl->tick2, 1u) == gridDim.x - 1) {
+    ctl->tick2 = 0;
+    ctl->status = isfinite(ctl->pq_tot) ? ST_BREAKDOWN : ST_NAN;
+  }
+  *alpha = *sa;
+  *alpha32 = sf;
+  return ok;
+}
+
+// The control decision after K2's dots (or the external preconditioner's):
+// iteration count, r.z slot, status, beta.  Executed by one thread of the
+// block that finished last, for K3.
+__device__ __forceinline__ void cg_decide(SolveCtl *ctl, int par, double rr, double rznew,
                                          double zq, double alpha) {
   const double rzold = ctl->rz[par];
   const int it = ctl->iter[par] + 1;
@@ -137,13 +206,16 @@ __device__ __forceinline__ int cg_decide(SolveCtl *ctl, int par, double rr, doub
   ctl->iter[par ^ 1] = it;
   ctl->rz[par ^ 1] = rznew;
   ctl->last_rr = rr;
+  ctl->last_alpha = alpha;
+  ctl->alpha32 = (float)alpha;
   if (lost) ctl->fallback = 1;
   // Fletcher-Reeves (the reference's beta = r'r_new / r'r_old, with z) or
   // Polak-Ribiere for a variable preconditioner: (z.r_new - z.r_old)/rz_old
   // where r_new - r_old = -alpha q.
-  ctl->beta = ctl->flexible ? (-alpha * zq) / rzold : rznew / rzold;
+  const double beta = ctl->flexible ? (-alpha * zq) / rzold : rznew / rzold;
+  ctl->beta = beta;
+  ctl->beta32 = (float)beta;
   if (st != ST_RUNNING) ctl->status = st;
-  return st;
 }
 
 // Per-thread dot-product accumulator.  FP64 arithmetic is scarce on this GPU
@@ -157,6 +229,16 @@ __device__ __forceinline__ int cg_decide(SolveCtl *ctl, int par, double rr, doub
 // contracted or reassociated by the compiler.  For FP64 operands the
 // accumulator is a plain FP64 sum.
 template <typename T> struct DotAcc;
+
+// (double)f without the FP64 pipe, which also runs the conversions: for a
+// normal number the exponent is rebiased and the fraction moved.
+__device__ __forceinline__ double widen(float f) {
+  const uint32_t u = __float_as_uint(f), m = u & 0x7fffffffu;
+  if (m != 0u && (m < 0x00800000u || m >= 0x7f800000u)) return (double)f;  // denormal, inf, NaN
+  return __hiloint2double((int)((u & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)),
+                          (int)(u << 29));
+}
+
 template <> struct DotAcc<float> {
   float hi = 0.f, lo = 0.f;
   __device__ __forceinline__ void add(float a, float b) {
@@ -168,7 +250,7 @@ template <> struct DotAcc<float> {
     hi = s;
     lo = __fadd_rn(lo, __fadd_rn(e, pe));
   }
-  __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+  __device__ __forceinline__ double value() const { return widen(hi) + widen(lo); }
 };
 template <> struct DotAcc<double> {
   double v = 0.0;
@@ -176,15 +258,16 @@ template <> struct DotAcc<double> {
   __device__ __forceinline__ double value() const { return v; }
 };
 
-// K1: q = A p, partial p.q.  BS = 3 or 1 (G lanes per row), 0 = any bs.
+// K1: q = A p; the last CTA leaves p.q in ctl->pq_tot.  BS = 3 or 1 (G lanes
+// per row), 0 = any bs.
 template <int BS, int G, typename MT, typename VT>
-__global__ void __launch_bounds__(RED_T) k_cg_spmv(const SolveCtl *__restrict__ ctl, int32_t n,
+__global__ void __launch_bounds__(RED_T) k_cg_spmv(SolveCtl *ctl, int32_t n,
                                                    int32_t bs, const uint32_t *__restrict__ rowptr,
                                                    const uint32_t *__restrict__ colidx,
                                                    const MT *__restrict__ vals,
                                                    const VT *__restrict__ p, VT *__restrict__ q,
                                                    double *__restrict__ part) {
-  __shared__ double sh[33];
+  __shared__ double sh[RED_T];
   if (ctl->status != ST_RUNNING) return;
   double acc = 0;
   if (BS == 3 || BS == 1) {
@@ -225,134 +308,128 @@ __global__ void __launch_bounds__(RED_T) k_cg_spmv(const SolveCtl *__restrict__ 
       }
     }
   }
-  double tot = block_sum(acc, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = tot;
+  double t, tot;
+  block_sums<1>(&acc, &t, sh);
+  if (finalize_partials<1>(&t, part, &ctl->tick1, &tot, sh) && threadIdx.x == 0)
+    ctl->pq_tot = tot;
 }
 
 // Preconditioner kinds applied inside K2.
 enum PrecKind : int { PK_NONE = 0, PK_JACOBI = 1, PK_BLOCK3 = 2, PK_EXTERNAL = 3 };
 
-// K2: alpha, x/r update, z = M r, partials of r.r, r.z, z.q.
-// part_in: np1 partials of p.q; part_out: 3 * gridDim.x (rr | rz | zq).
-template <typename VT, typename XT, int PREC>
-__global__ void __launch_bounds__(RED_T) k_cg_update(SolveCtl *ctl, int par, int64_t len,
-                                                     const double *__restrict__ part_in, int np1,
-                                                     const VT *__restrict__ p,
-                                                     const VT *__restrict__ q, VT *__restrict__ r,
-                                                     XT *__restrict__ x, VT *__restrict__ z,
-                                                     const VT *__restrict__ dinv,
-                                                     double *__restrict__ part_out) {
-  __shared__ double sh[33];
+// K2 in FP64 (vectors, x and preconditioner): alpha, x and r updated,
+// z = M r, r.r and r.z summed by the last CTA, which decides the iteration
+// for K3.  A thread takes two entries (16-byte accesses; the buffers are
+// cudaMalloc'd) or, with block Jacobi, one vertex.  Bound by the latency of
+// its loads and of the two-level sums at the sizes that fit in L2: heat 64^3
+// (275 k rows, 17.6 MB touched) 14.1 us when every block of the next kernel
+// summed the partials again, FIGK2F64 so.
+template <int PREC>
+__global__ void __launch_bounds__(RED_T, 4) k_cg_update_f64(
+    SolveCtl *ctl, int par, int64_t len, const double *__restrict__ p,
+    const double *__restrict__ q, double *__restrict__ r, double *__restrict__ x,
+    double *__restrict__ z, const double *__restrict__ dinv, double *__restrict__ part_out) {
+  __shared__ double sh[2 * RED_T], sa;
   if (ctl->status != ST_RUNNING) return;
-  const double pq = sum_parts(part_in, np1, sh);
-  const double rz = ctl->rz[par];
-  if (!(pq > 0.0) || !isfinite(pq)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->status = isfinite(pq) ? ST_BREAKDOWN : ST_NAN;
-    return;
-  }
-  const double alpha = rz / pq;
-  const VT a = (VT)alpha;
-  double rr = 0, rzs = 0, zq = 0;
+  double acc[2] = {0.0, 0.0}, alpha;  // r.r, r.z
+  float a32;
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (PREC == PK_BLOCK3) {
-    // 3x3 block-Jacobi: dinv holds 9 values per vertex; one thread per vertex
-    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v * 3 < len;
-         v += (int64_t)gridDim.x * blockDim.x) {
-      VT rv[3];
+    // 3x3 block-Jacobi: dinv holds 9 values per vertex
+    if (!cg_alpha(ctl, par, &sa, &alpha, &a32)) return;
+    for (int64_t v = t0; v * 3 < len; v += step) {
+      double rv[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const int64_t i = v * 3 + k;
-        x[i] = (XT)(x[i] + (XT)(a * p[i]));
-        rv[k] = r[i] - a * q[i];
+        x[i] = x[i] + alpha * p[i];
+        rv[k] = r[i] - alpha * q[i];
         r[i] = rv[k];
       }
-      const VT *D = dinv + v * 9;
+      const double *D = dinv + v * 9;
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        const VT zk = D[k * 3] * rv[0] + D[k * 3 + 1] * rv[1] + D[k * 3 + 2] * rv[2];
+        const double zk = D[k * 3] * rv[0] + D[k * 3 + 1] * rv[1] + D[k * 3 + 2] * rv[2];
         z[v * 3 + k] = zk;
-        rr += (double)rv[k] * (double)rv[k];
-        rzs += (double)rv[k] * (double)zk;
-        zq += (double)zk * (double)q[v * 3 + k];
+        acc[0] += rv[k] * rv[k];
+        acc[1] += rv[k] * zk;
       }
     }
   } else {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const VT pi = p[i], qi = q[i];
-      x[i] = (XT)(x[i] + (XT)(a * pi));
-      const VT ri = r[i] - a * qi;
-      r[i] = ri;
-      VT zi = ri;
-      if (PREC == PK_JACOBI) zi = dinv[i] * ri;
-      if (PREC != PK_EXTERNAL) {
-        if (PREC != PK_NONE) z[i] = zi;
-        rzs += (double)ri * (double)zi;
-        zq += (double)zi * (double)qi;
-      }
-      rr += (double)ri * (double)ri;
+    const double2 *p2 = reinterpret_cast<const double2 *>(p);
+    const double2 *q2 = reinterpret_cast<const double2 *>(q);
+    const double2 *d2 = reinterpret_cast<const double2 *>(dinv);
+    double2 *r2 = reinterpret_cast<double2 *>(r), *x2 = reinterpret_cast<double2 *>(x);
+    double2 *z2 = reinterpret_cast<double2 *>(z);
+    const int64_t nu = len / 2;
+    double2 pv, qv, rv, xv, dv;
+    auto load = [&](int64_t u) {
+      if (u >= nu) return;
+      pv = p2[u];
+      qv = q2[u];
+      rv = r2[u];
+      xv = x2[u];
+      if (PREC == PK_JACOBI) dv = d2[u];
+    };
+    load(t0);
+    if (!cg_alpha(ctl, par, &sa, &alpha, &a32)) return;
+    auto one = [&](double pi, double qi, double &ri, double &xi, double di) {
+      xi = xi + alpha * pi;
+      ri = ri - alpha * qi;
+      const double zi = PREC == PK_JACOBI ? di * ri : ri;
+      acc[0] += ri * ri;
+      if (PREC == PK_JACOBI) acc[1] += ri * zi;
+      return zi;
+    };
+    for (int64_t u = t0; u < nu; u += step) {
+      double2 zv;
+      zv.x = one(pv.x, qv.x, rv.x, xv.x, dv.x);
+      zv.y = one(pv.y, qv.y, rv.y, xv.y, dv.y);
+      x2[u] = xv;
+      r2[u] = rv;
+      if (PREC == PK_JACOBI) z2[u] = zv;
+      load(u + step);
     }
+    if ((len & 1) && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+      const int64_t i = len - 1;
+      double ri = r[i], xi = x[i];
+      const double zi = one(p[i], q[i], ri, xi, PREC == PK_JACOBI ? dinv[i] : 0.0);
+      x[i] = xi;
+      r[i] = ri;
+      if (PREC == PK_JACOBI) z[i] = zi;
+    }
+    if (PREC == PK_NONE) acc[1] = acc[0];  // z is r
   }
-  const double t0 = block_sum(rr, sh);
-  const double t1 = block_sum(rzs, sh);
-  const double t2 = block_sum(zq, sh);
-  if (threadIdx.x == 0) {
-    part_out[blockIdx.x] = t0;
-    part_out[gridDim.x + blockIdx.x] = t1;
-    part_out[2 * gridDim.x + blockIdx.x] = t2;
-    if (blockIdx.x == 0) ctl->last_alpha = alpha;
-  }
+  double t[2], tot[2];
+  block_sums<2>(acc, t, sh);
+  if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
+    cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
 }
 
-// K3: beta, direction update, control decisions.
-// part_in: 3 * np2 partials (rr | rz | zq) from K2 (or from the external
-// preconditioner's dot kernel).
-template <typename VT>
-__global__ void __launch_bounds__(RED_T) k_cg_direction(SolveCtl *ctl, int par, int64_t len,
-                                                        const double *__restrict__ part_in,
-                                                        int np2, const VT *__restrict__ z,
-                                                        VT *__restrict__ p) {
-  __shared__ double sh[33];
+// K3 in FP64: p = z + beta p, two entries per thread.
+static __global__ void __launch_bounds__(RED_T) k_cg_direction_f64(
+    const SolveCtl *__restrict__ ctl, int64_t len, const double *__restrict__ z,
+    double *__restrict__ p) {
   if (ctl->status != ST_RUNNING) return;
-  const double rr = sum_parts(part_in, np2, sh);
-  const double rznew = sum_parts(part_in + np2, np2, sh);
-  const double zq = sum_parts(part_in + 2 * np2, np2, sh);
-  const double rzold = ctl->rz[par];
-  const int it = ctl->iter[par] + 1;
-  int st = ST_RUNNING;
-  const bool lost = ctl->flexible && !ctl->fallback && !(rznew > 0.0);
-  if (lost) st = ST_NEED_CHECK;  // z is no descent direction: fall back
-  else if (!isfinite(rr) || !isfinite(rznew)) st = ST_NAN;
-  else if (rr <= ctl->tol2) st = ST_NEED_CHECK;
-  else if (ctl->upd2 > 0.0 && rr < ctl->upd2) st = ST_NEED_CHECK;
-  else if (ctl->check_every > 0 && it % ctl->check_every == 0) st = ST_NEED_CHECK;
-  else if (it >= ctl->maxiters) st = ST_MAXITER;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl->iter[par ^ 1] = it;
-    ctl->rz[par ^ 1] = rznew;
-    ctl->last_rr = rr;
-    if (lost) ctl->fallback = 1;
-    if (st != ST_RUNNING) ctl->status = st;
+  const double b = ctl->beta;
+  const int64_t nu = len / 2;
+  const double2 *z2 = reinterpret_cast<const double2 *>(z);
+  double2 *p2 = reinterpret_cast<double2 *>(p);
+  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu;
+       u += (int64_t)gridDim.x * blockDim.x) {
+    const double2 zv = z2[u], pv = p2[u];
+    p2[u] = make_double2(zv.x + b * pv.x, zv.y + b * pv.y);
   }
-  if (st != ST_RUNNING) return;
-  // Fletcher-Reeves (the reference's beta = r'r_new / r'r_old, with z) or
-  // Polak-Ribiere for a variable preconditioner: (z.r_new - z.r_old)/rz_old
-  // where r_new - r_old = -alpha q.
-  double beta;
-  if (ctl->flexible) beta = (-ctl->last_alpha * zq) / rzold;
-  else beta = rznew / rzold;
-  const VT b = (VT)beta;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len;
-       i += (int64_t)gridDim.x * blockDim.x)
-    p[i] = z[i] + b * p[i];
+  if ((len & 1) && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+    p[len - 1] = z[len - 1] + b * p[len - 1];
 }
 
 // ---------------------------------------------------------------------------
-// FP32 (mixed-precision) K2 / K3 with 16-byte loads and stores.  One thread
-// takes four vertices at a time: three float4 of each vector and nine of the
-// block-Jacobi inverse, all contiguous across the warp.  The buffers are
-// cudaMalloc'd (256-byte aligned); the last len % 12 (or len % 4) entries go
-// through the scalar loop of thread 0 of the last block.  Same partial sums
-// as the scalar kernels, in a different (fixed) order.
+// FP32 (mixed-precision) K2 / K3 with 16-byte loads and stores: one thread
+// takes four entries of each vector at a time, contiguous across the warp.
+// The buffers are cudaMalloc'd (256-byte aligned); the last len % 4 entries
+// go through the scalar loop of thread 0 of the last block.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void ld4(const float *p, int64_t i, float *o) {
   const float4 v = reinterpret_cast<const float4 *>(p)[i];
@@ -362,206 +439,152 @@ __device__ __forceinline__ void st4(float *p, int64_t i, const float *o) {
   reinterpret_cast<float4 *>(p)[i] = make_float4(o[0], o[1], o[2], o[3]);
 }
 
-// pq_fin: K1 left the p.q total in ctl->pq_tot (else the np1 partials are
-// summed here).  FIN (not with an external preconditioner, whose dots come
-// after K2): the last CTA sums r.r, r.z, z.q and takes K3's decision.
-template <int PREC, bool FIN>
-__global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(SolveCtl *ctl, int par, int64_t len,
-                                                        const double *__restrict__ part_in,
-                                                        int np1, int pq_fin,
-                                                        const float *__restrict__ p,
-                                                        const float *__restrict__ q,
-                                                        float *__restrict__ r,
-                                                        float *__restrict__ x,
-                                                        float *__restrict__ z,
-                                                        const float *__restrict__ dinv,
-                                                        double *__restrict__ part_out) {
+// With an external preconditioner (whose dots come after K2) only the
+// partials of r.r are left; otherwise the last CTA sums r.r and r.z and takes
+// the decision.
+template <int PREC>
+__global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
+    SolveCtl *ctl, int par, int64_t len, const float *__restrict__ p,
+    const float *__restrict__ q, float *__restrict__ r, float *__restrict__ x,
+    float *__restrict__ z, const float *__restrict__ dinv, double *__restrict__ part_out) {
   // FP32 block Jacobi runs k_cg_update_w, whose inverse blocks are packed
   static_assert(PREC != PK_BLOCK3, "FP32 block Jacobi: use k_cg_update_w");
-  __shared__ double sh[33];
+  __shared__ double sh[2 * RED_T], sa;
   if (ctl->status != ST_RUNNING) return;
-  const double pq = pq_fin ? ctl->pq_tot : sum_parts(part_in, np1, sh);
-  const double rz = ctl->rz[par];
-  if (!(pq > 0.0) || !isfinite(pq)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->status = isfinite(pq) ? ST_BREAKDOWN : ST_NAN;
-    return;
-  }
-  const double alpha = rz / pq;
-  const float a = (float)alpha;
-  DotAcc<float> rr, rzs, zq;
-  constexpr int W = PREC == PK_BLOCK3 ? 12 : 4;  // floats per thread step
-  constexpr int NV = W / 4;                      // float4 per vector
-  const int64_t nu = len / W;
-  for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu;
-       u += (int64_t)gridDim.x * blockDim.x) {
-    float pv[W], qv[W], rv[W], xv[W], zv[W];
+  DotAcc<float> rr, rzs;
+  const int64_t nu = len / 4;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  float pv[4], qv[4], rv[4], xv[4], dv[4], zv[4];
+  auto load = [&](int64_t i) {
+    if (i >= nu) return;
+    ld4(p, i, pv);
+    ld4(q, i, qv);
+    ld4(r, i, rv);
+    ld4(x, i, xv);
+    if (PREC == PK_JACOBI) ld4(dinv, i, dv);
+  };
+  load(u);
+  double alpha;
+  float a;
+  if (!cg_alpha(ctl, par, &sa, &alpha, &a)) return;
+  for (; u < nu; u += step) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      ld4(p, u * NV + k, pv + 4 * k);
-      ld4(q, u * NV + k, qv + 4 * k);
-      ld4(r, u * NV + k, rv + 4 * k);
-      ld4(x, u * NV + k, xv + 4 * k);
-    }
-    float dv[PREC == PK_BLOCK3 ? 36 : (PREC == PK_JACOBI ? 4 : 1)];
-    if (PREC == PK_BLOCK3) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) ld4(dinv, u * 9 + k, dv + 4 * k);
-    } else if (PREC == PK_JACOBI) {
-      ld4(dinv, u, dv);
-    }
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
+    for (int k = 0; k < 4; ++k) {
       xv[k] = xv[k] + a * pv[k];
       rv[k] = rv[k] - a * qv[k];
+      zv[k] = PREC == PK_JACOBI ? dv[k] * rv[k] : rv[k];
     }
-    if (PREC == PK_BLOCK3) {
+    st4(x, u, xv);
+    st4(r, u, rv);
+    if (PREC == PK_JACOBI) st4(z, u, zv);
 #pragma unroll
-      for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-          zv[v * 3 + k] = dv[v * 9 + k * 3] * rv[v * 3] + dv[v * 9 + k * 3 + 1] * rv[v * 3 + 1] +
-                          dv[v * 9 + k * 3 + 2] * rv[v * 3 + 2];
-    } else {
-#pragma unroll
-      for (int k = 0; k < W; ++k) zv[k] = PREC == PK_JACOBI ? dv[k] * rv[k] : rv[k];
-    }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      st4(x, u * NV + k, xv + 4 * k);
-      st4(r, u * NV + k, rv + 4 * k);
-      if (PREC == PK_BLOCK3 || PREC == PK_JACOBI) st4(z, u * NV + k, zv + 4 * k);
-    }
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
+    for (int k = 0; k < 4; ++k) {
       rr.add(rv[k], rv[k]);
-      if (PREC != PK_EXTERNAL) {
-        rzs.add(rv[k], zv[k]);
-        zq.add(zv[k], qv[k]);
-      }
+      if (PREC != PK_EXTERNAL) rzs.add(rv[k], zv[k]);
     }
+    load(u + step);
   }
-  // tail: the last len % W entries, scalar, by one thread
+  // tail: the last len % 4 entries, scalar, by one thread
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-    for (int64_t i0 = nu * W; i0 < len; i0 += (PREC == PK_BLOCK3 ? 3 : 1)) {
-      const int m = PREC == PK_BLOCK3 ? 3 : 1;
-      float rv[3], zv[3];
-      for (int k = 0; k < m; ++k) {
-        const int64_t i = i0 + k;
-        x[i] = x[i] + a * p[i];
-        rv[k] = r[i] - a * q[i];
-        r[i] = rv[k];
-      }
-      for (int k = 0; k < m; ++k) {
-        const int64_t i = i0 + k;
-        if (PREC == PK_BLOCK3) {
-          const float *D = dinv + (i0 / 3) * 9;
-          zv[k] = D[k * 3] * rv[0] + D[k * 3 + 1] * rv[1] + D[k * 3 + 2] * rv[2];
-        } else {
-          zv[k] = PREC == PK_JACOBI ? dinv[i] * rv[k] : rv[k];
-        }
-        if (PREC == PK_BLOCK3 || PREC == PK_JACOBI) z[i] = zv[k];
-        rr.add(rv[k], rv[k]);
-        if (PREC != PK_EXTERNAL) {
-          rzs.add(rv[k], zv[k]);
-          zq.add(zv[k], q[i]);
-        }
-      }
+    for (int64_t i = nu * 4; i < len; ++i) {
+      x[i] = x[i] + a * p[i];
+      const float ri = r[i] - a * q[i];
+      r[i] = ri;
+      const float zi = PREC == PK_JACOBI ? dinv[i] * ri : ri;
+      if (PREC == PK_JACOBI) z[i] = zi;
+      rr.add(ri, ri);
+      if (PREC != PK_EXTERNAL) rzs.add(ri, zi);
     }
   }
-  const double t[3] = {block_sum(rr.value(), sh), block_sum(rzs.value(), sh),
-                       block_sum(zq.value(), sh)};
-  if (FIN) {
-    double tot[3];  // written and read by thread 0 of the last CTA
-    if (finalize_partials(t, 3, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0) {
-      ctl->last_alpha = alpha;
-      cg_decide(ctl, par, tot[0], tot[1], tot[2], alpha);
+  const double acc[2] = {rr.value(), PREC != PK_EXTERNAL ? rzs.value() : 0.0};
+  double t[2], tot[2];
+  if (PREC == PK_EXTERNAL) {
+    block_sums<1>(acc, t, sh);
+    if (threadIdx.x == 0) {
+      part_out[blockIdx.x] = t[0];
+      if (blockIdx.x == 0) ctl->last_alpha = alpha;
     }
-  } else if (threadIdx.x == 0) {
-    part_out[blockIdx.x] = t[0];
-    part_out[gridDim.x + blockIdx.x] = t[1];
-    part_out[2 * gridDim.x + blockIdx.x] = t[2];
-    if (blockIdx.x == 0) ctl->last_alpha = alpha;
+  } else {
+    block_sums<2>(acc, t, sh);
+    if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
+      cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
   }
 }
 
 // K2 for FP32 vectors and 3x3 block Jacobi with warp-staged, fully coalesced
-// accesses.  A warp takes 128 vertices at a time: it loads the chunk of
-// p, q, r, x (96 float4 each) and of the packed symmetric D^-1 (6 values per
-// vertex, k_diag_inv PACK6: 192 float4) with lane-consecutive
-// 16-byte loads into its shared-memory slice, each lane then reads its four
-// vertices (3 and 9 consecutive float4, conflict-free), and the results go
-// back through shared memory to lane-consecutive stores.  Same arithmetic,
-// partial sums and finalisation as k_cg_update_v4<PK_BLOCK3>.  The last
-// len % 12 entries are done by the scalar tail of thread 0 of the last CTA.
-constexpr int K2W_WARPS = 8;
+// accesses.  A warp takes 128 vertices at a time: it copies the chunk of q, r
+// (96 float4 each) and of the packed symmetric D^-1 (6 values per vertex,
+// k_diag_inv PACK6: 192 float4) into its shared-memory slice with
+// lane-consecutive 16-byte asynchronous copies, each lane then reads its four
+// vertices (3 and 6 consecutive float4, conflict-free), and the results go
+// back through shared memory to lane-consecutive stores.  x += alpha p is
+// left to K3 (k_cg_direction_v4 with xupd).  The first chunk is on its way
+// while the status and alpha are fetched.  The last len % 12 entries are done
+// by the scalar tail of thread 0 of the last CTA.  Bound, below a few hundred
+// thousand vertices, by latency and the FP64 pipe of the SMs that hold the
+// (few) blocks: 36 k vertices, one chunk per warp, 11.5 us with alpha divided
+// by every warp, conversions on the FP64 pipe and three sums one after the
+// other, FIGK2W so.
+constexpr int K2W_WARPS = 8;  // at most; a block has blockDim.x / 32
 struct K2WarpSmem {
-  float4 p[96], q[96], r[96], x[96], d[192];
+  float4 q[96], r[96], d[192];
 };
 
-// XUPD = false: x += alpha p is left to K3 (k_cg_direction_v4 with xupd), so
-// this kernel neither reads p and x nor writes x.
-template <bool FIN, bool XUPD = true>
-__global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
-    SolveCtl *ctl, int par, int64_t len, const double *__restrict__ part_in, int np1,
-    int pq_fin, const float *__restrict__ p, const float *__restrict__ q, float *__restrict__ r,
-    float *__restrict__ x, float *__restrict__ z, const float *__restrict__ dinv,
-    double *__restrict__ part_out) {
+static __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
+    SolveCtl *ctl, int par, int64_t len, const float *__restrict__ q, float *__restrict__ r,
+    float *__restrict__ z, const float *__restrict__ dinv, double *__restrict__ part_out) {
   extern __shared__ __align__(16) unsigned char k2w_raw[];
-  __shared__ double sh[33];
+  __shared__ double sh[2 * K2W_WARPS * 32], sa;
   pdl_wait_and_release();
-  if (ctl->status != ST_RUNNING) return;
-  const double pq = pq_fin ? ctl->pq_tot : sum_parts(part_in, np1, sh);
-  const double rz = ctl->rz[par];
-  if (!(pq > 0.0) || !isfinite(pq)) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->status = isfinite(pq) ? ST_BREAKDOWN : ST_NAN;
-    return;
-  }
-  const double alpha = rz / pq;
-  const float a = (float)alpha;
   const int lane = threadIdx.x & 31;
   K2WarpSmem &w = reinterpret_cast<K2WarpSmem *>(k2w_raw)[threadIdx.x >> 5];
-  const float4 *p4 = reinterpret_cast<const float4 *>(p);
-  const float4 *q4 = reinterpret_cast<const float4 *>(q);
   float4 *r4 = reinterpret_cast<float4 *>(r);
-  float4 *x4 = reinterpret_cast<float4 *>(x);
   float4 *z4 = reinterpret_cast<float4 *>(z);
+  const float4 *q4 = reinterpret_cast<const float4 *>(q);
   const float4 *d4 = reinterpret_cast<const float4 *>(dinv);
   const int64_t nu = len / 12;          // complete 4-vertex units
   const int64_t nf = nu * 3;            // their float4 of each vector
   const int64_t nchunks = (nu + 31) / 32;
-  DotAcc<float> rr, rzs, zq;
-  for (int64_t c = (int64_t)blockIdx.x * K2W_WARPS + (threadIdx.x >> 5); c < nchunks;
-       c += (int64_t)gridDim.x * K2W_WARPS) {
+  auto load = [&](int64_t c) {
+    if (c >= nchunks) return;
     const int64_t f0 = c * 96, d0 = c * 192;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
       const int64_t f = f0 + lane + 32 * j;
       if (f < nf) {
-        if (XUPD) w.p[lane + 32 * j] = p4[f];
-        w.q[lane + 32 * j] = q4[f];
-        w.r[lane + 32 * j] = r4[f];
-        if (XUPD) w.x[lane + 32 * j] = x4[f];
+        cp_async16(&w.q[lane + 32 * j], q4 + f);
+        cp_async16(&w.r[lane + 32 * j], r4 + f);
       }
     }
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
       const int64_t f = d0 + lane + 32 * j;
-      if (f < nf * 2) w.d[lane + 32 * j] = d4[f];
+      if (f < nf * 2) cp_async16(&w.d[lane + 32 * j], d4 + f);
     }
+  };
+  const int64_t step = (int64_t)gridDim.x * (blockDim.x / 32);
+  int64_t c = (int64_t)blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+  load(c);
+  double alpha = 0.0;
+  float a = 0.f;
+  if (ctl->status != ST_RUNNING || !cg_alpha(ctl, par, &sa, &alpha, &a)) {
+    cp_async_wait_all();
+    return;
+  }
+  DotAcc<float> rr, rzs;
+  for (; c < nchunks; c += step) {
+    cp_async_wait_all();
     __syncwarp();
     const bool mine = c * 32 + lane < nu;
-    float pv[12], qv[12], rv[12], xv[12], zv[12], dv[24];
+    float rv[12], zv[12];
     if (mine) {
+      float qv[12], dv[24];
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
         const float4 b4 = w.q[3 * lane + j], c4 = w.r[3 * lane + j];
         qv[4 * j] = b4.x; qv[4 * j + 1] = b4.y; qv[4 * j + 2] = b4.z; qv[4 * j + 3] = b4.w;
         rv[4 * j] = c4.x; rv[4 * j + 1] = c4.y; rv[4 * j + 2] = c4.z; rv[4 * j + 3] = c4.w;
-        if (XUPD) {
-          const float4 a4 = w.p[3 * lane + j], e4 = w.x[3 * lane + j];
-          pv[4 * j] = a4.x; pv[4 * j + 1] = a4.y; pv[4 * j + 2] = a4.z; pv[4 * j + 3] = a4.w;
-          xv[4 * j] = e4.x; xv[4 * j + 1] = e4.y; xv[4 * j + 2] = e4.z; xv[4 * j + 3] = e4.w;
-        }
       }
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
@@ -569,10 +592,7 @@ __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
         dv[4 * j] = g4.x; dv[4 * j + 1] = g4.y; dv[4 * j + 2] = g4.z; dv[4 * j + 3] = g4.w;
       }
 #pragma unroll
-      for (int k = 0; k < 12; ++k) {
-        if (XUPD) xv[k] = xv[k] + a * pv[k];
-        rv[k] = rv[k] - a * qv[k];
-      }
+      for (int k = 0; k < 12; ++k) rv[k] = rv[k] - a * qv[k];
 #pragma unroll
       for (int v = 0; v < 4; ++v) {  // symmetric inverse, upper triangle
         const float *m = dv + v * 6, *rq = rv + v * 3;
@@ -584,30 +604,27 @@ __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
       for (int k = 0; k < 12; ++k) {
         rr.add(rv[k], rv[k]);
         rzs.add(rv[k], zv[k]);
-        zq.add(zv[k], qv[k]);
       }
     }
     __syncwarp();  // every lane has read its inputs
     if (mine) {
 #pragma unroll
       for (int j = 0; j < 3; ++j) {
-        if (XUPD)
-          w.x[3 * lane + j] = make_float4(xv[4 * j], xv[4 * j + 1], xv[4 * j + 2], xv[4 * j + 3]);
         w.r[3 * lane + j] = make_float4(rv[4 * j], rv[4 * j + 1], rv[4 * j + 2], rv[4 * j + 3]);
-        w.p[3 * lane + j] = make_float4(zv[4 * j], zv[4 * j + 1], zv[4 * j + 2], zv[4 * j + 3]);
+        w.q[3 * lane + j] = make_float4(zv[4 * j], zv[4 * j + 1], zv[4 * j + 2], zv[4 * j + 3]);
       }
     }
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      const int64_t f = f0 + lane + 32 * j;
+      const int64_t f = c * 96 + lane + 32 * j;
       if (f < nf) {
-        if (XUPD) x4[f] = w.x[lane + 32 * j];
         r4[f] = w.r[lane + 32 * j];
-        z4[f] = w.p[lane + 32 * j];
+        z4[f] = w.q[lane + 32 * j];
       }
     }
     __syncwarp();  // the slice is refilled by the next chunk
+    load(c + step);
   }
   // tail: the last len % 12 entries, scalar, by one thread
   if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
@@ -615,7 +632,6 @@ __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
       float rv[3];
       for (int k = 0; k < 3; ++k) {
         const int64_t i = i0 + k;
-        if (XUPD) x[i] = x[i] + a * p[i];
         rv[k] = r[i] - a * q[i];
         r[i] = rv[k];
       }
@@ -628,95 +644,27 @@ __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
         z[i0 + k] = zk;
         rr.add(rv[k], rv[k]);
         rzs.add(rv[k], zk);
-        zq.add(zk, q[i0 + k]);
       }
     }
   }
-  const double t[3] = {block_sum(rr.value(), sh), block_sum(rzs.value(), sh),
-                       block_sum(zq.value(), sh)};
-  if (FIN) {
-    double tot[3];
-    if (finalize_partials(t, 3, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0) {
-      ctl->last_alpha = alpha;
-      cg_decide(ctl, par, tot[0], tot[1], tot[2], alpha);
-    }
-  } else if (threadIdx.x == 0) {
-    part_out[blockIdx.x] = t[0];
-    part_out[gridDim.x + blockIdx.x] = t[1];
-    part_out[2 * gridDim.x + blockIdx.x] = t[2];
-    if (blockIdx.x == 0) ctl->last_alpha = alpha;
-  }
+  const double acc[2] = {rr.value(), rzs.value()};
+  double t[2], tot[2];
+  block_sums<2>(acc, t, sh);
+  if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
+    cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
 }
 
-// K3 for FP32 vectors: the control decisions of k_cg_direction, then
-// p = z + beta p with float4 accesses.
-// fin: K2 already took the decision and left beta in ctl->beta.
+// K3 for FP32 vectors: p = z + beta p with float4 accesses.
 // xupd: K2 left x += alpha p to this kernel, which applies it with the
-// direction it is about to replace; when K2 (fin) or this kernel (!fin)
-// stopped the batch, the host applies that last update instead (the early
-// returns below).
-static __global__ void __launch_bounds__(RED_T) k_cg_direction_v4(SolveCtl *ctl, int par, int64_t len,
-                                                           const double *__restrict__ part_in,
-                                                           int np2, int fin,
-                                                           const float *__restrict__ z,
-                                                           float *__restrict__ p,
-                                                           float *__restrict__ x, int xupd) {
-  __shared__ double sh[33];
+// direction it is about to replace; when the iteration stopped the batch
+// (the early return), the host applies that last update instead.
+static __global__ void __launch_bounds__(RED_T) k_cg_direction_v4(
+    const SolveCtl *__restrict__ ctl, int64_t len, const float *__restrict__ z,
+    float *__restrict__ p, float *__restrict__ x, int xupd) {
   pdl_wait_and_release();
   if (ctl->status != ST_RUNNING) return;
-  if (fin) {
-    const float b = (float)ctl->beta;
-    const float a = (float)ctl->last_alpha;
-    const int64_t nu = len / 4;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu;
-         u += (int64_t)gridDim.x * blockDim.x) {
-      float zv[4], pv[4];
-      ld4(z, u, zv);
-      ld4(p, u, pv);
-      if (xupd) {
-        float xv[4];
-        ld4(x, u, xv);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) xv[k] = xv[k] + a * pv[k];
-        st4(x, u, xv);
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) pv[k] = zv[k] + b * pv[k];
-      st4(p, u, pv);
-    }
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
-      for (int64_t i = nu * 4; i < len; ++i) {
-        if (xupd) x[i] = x[i] + a * p[i];
-        p[i] = z[i] + b * p[i];
-      }
-    return;
-  }
-  const double rr = sum_parts(part_in, np2, sh);
-  const double rznew = sum_parts(part_in + np2, np2, sh);
-  const double zq = sum_parts(part_in + 2 * np2, np2, sh);
-  const double rzold = ctl->rz[par];
-  const int it = ctl->iter[par] + 1;
-  int st = ST_RUNNING;
-  const bool lost = ctl->flexible && !ctl->fallback && !(rznew > 0.0);
-  if (lost) st = ST_NEED_CHECK;
-  else if (!isfinite(rr) || !isfinite(rznew)) st = ST_NAN;
-  else if (rr <= ctl->tol2) st = ST_NEED_CHECK;
-  else if (ctl->upd2 > 0.0 && rr < ctl->upd2) st = ST_NEED_CHECK;
-  else if (ctl->check_every > 0 && it % ctl->check_every == 0) st = ST_NEED_CHECK;
-  else if (it >= ctl->maxiters) st = ST_MAXITER;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl->iter[par ^ 1] = it;
-    ctl->rz[par ^ 1] = rznew;
-    ctl->last_rr = rr;
-    if (lost) ctl->fallback = 1;
-    if (st != ST_RUNNING) ctl->status = st;
-  }
-  if (st != ST_RUNNING) return;
-  const double beta = ctl->flexible ? (-ctl->last_alpha * zq) / rzold : rznew / rzold;
-  const float b = (float)beta;
-  // xupd: the iteration's x += alpha p, applied here with the direction it
-  // is about to replace (on a stop above the host applies it instead)
-  const float a = (float)ctl->last_alpha;
+  const float b = ctl->beta32;
+  const float a = ctl->alpha32;
   const int64_t nu = len / 4;
   for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < nu;
        u += (int64_t)gridDim.x * blockDim.x) {

@@ -26,7 +26,8 @@ __host__ __device__ inline size_t tma_cbytes(int capb) {
   return (((size_t)capb * 4 + 32) + 15) & ~size_t(15);
 }
 template <typename MT> inline size_t tma_smem_bytes(int capb, int nst) {
-  return 64 + (size_t)nst * (tma_vbytes<MT>(capb) + tma_cbytes(capb));
+  const size_t b = 64 + (size_t)nst * (tma_vbytes<MT>(capb) + tma_cbytes(capb));
+  return b > SUM_SMEM ? b : SUM_SMEM;
 }
 
 // y_r = (A x)_r for block row r from its tile's values vb and columns cb
@@ -144,7 +145,6 @@ __global__ void __launch_bounds__(ROWS *G)
                int *err) {
   static_assert(NST >= 2 && NST <= 6, "stages");
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double shred[33];
   __shared__ int ok_flag;
   if (ctl && ctl->status != ST_RUNNING) return;
   const size_t vbytes = tma_vbytes<MT>(capb), cbytes = tma_cbytes(capb);
@@ -244,9 +244,12 @@ __global__ void __launch_bounds__(ROWS *G)
     __syncthreads();
   }
   if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
-    const double t = block_sum(acc.value(), shred);
+    const double v = acc.value();
+    double t, tot;
+    block_sums<1>(&v, &t, sum_buf(sm));
     SolveCtl *c = const_cast<SolveCtl *>(ctl);
-    finalize_partials(&t, 1, part, &c->tick1, &c->pq_tot, shred);
+    if (finalize_partials<1>(&t, part, &c->tick1, &tot, sum_buf(sm)) && threadIdx.x == 0)
+      c->pq_tot = tot;
   }
 }
 
@@ -263,8 +266,9 @@ namespace sg {
 constexpr int WTMA_WARPS = 4;
 
 template <typename MT, int BB = 9> inline size_t wtma_smem_bytes(int capb, int nst) {
-  return (((size_t)WTMA_WARPS * nst * 8 + 15) & ~size_t(15)) +
-         (size_t)WTMA_WARPS * nst * (tma_vbytes<MT, BB>(capb) + tma_cbytes(capb));
+  const size_t b = (((size_t)WTMA_WARPS * nst * 8 + 15) & ~size_t(15)) +
+                   (size_t)WTMA_WARPS * nst * (tma_vbytes<MT, BB>(capb) + tma_cbytes(capb));
+  return b > SUM_SMEM ? b : SUM_SMEM;
 }
 
 // Body shared by the 3x3 (BS = 3) and scalar CSR (BS = 1) kernels.  A warp
@@ -276,8 +280,7 @@ __device__ __forceinline__ void wtma_body(const SolveCtl *__restrict__ ctl, int3
                                           const uint32_t *__restrict__ colidx,
                                           const MT *__restrict__ vals, const VT *__restrict__ x,
                                           VT *__restrict__ y, double *__restrict__ part,
-                                          int capb, int *err, unsigned char *sm,
-                                          double *shred) {
+                                          int capb, int *err, unsigned char *sm) {
   static_assert(NST >= 2 && NST <= 6, "stages");
   static_assert(BS == 1 || BS == 3, "block size");
   constexpr int RW = 32 / G * P;
@@ -380,9 +383,12 @@ __device__ __forceinline__ void wtma_body(const SolveCtl *__restrict__ ctl, int3
     __syncwarp();
   }
   if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
-    const double t = block_sum(acc.value(), shred);
+    const double v = acc.value();
+    double t, tot;
+    block_sums<1>(&v, &t, sum_buf(sm));
     SolveCtl *c = const_cast<SolveCtl *>(ctl);
-    finalize_partials(&t, 1, part, &c->tick1, &c->pq_tot, shred);
+    if (finalize_partials<1>(&t, part, &c->tick1, &tot, sum_buf(sm)) && threadIdx.x == 0)
+      c->pq_tot = tot;
   }
 }
 
@@ -393,9 +399,7 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32)
                 const VT *__restrict__ x, VT *__restrict__ y, double *__restrict__ part,
                 int capb, int *err) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double shred[33];
-  wtma_body<3, G, NST, 1, MT, VT, DOT>(ctl, n, rowptr, colidx, vals, x, y, part, capb, err, sm,
-                                       shred);
+  wtma_body<3, G, NST, 1, MT, VT, DOT>(ctl, n, rowptr, colidx, vals, x, y, part, capb, err, sm);
 }
 
 // Scalar CSR (bs = 1) with the same per-warp pipeline, tiles of P passes.
@@ -406,9 +410,7 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32)
                const VT *__restrict__ x, VT *__restrict__ y, double *__restrict__ part,
                int capb, int *err) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double shred[33];
-  wtma_body<1, G, NST, P, MT, VT, DOT>(ctl, n, rowptr, colidx, vals, x, y, part, capb, err, sm,
-                                       shred);
+  wtma_body<1, G, NST, P, MT, VT, DOT>(ctl, n, rowptr, colidx, vals, x, y, part, capb, err, sm);
 }
 
 // FP64 3x3 blocked SpMV, rows sorted by length inside a tile.
@@ -430,7 +432,8 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32)
 constexpr int F64_ROWS = 64, F64_T = 3 * F64_ROWS;
 constexpr int F64_U = 4;  // blocks whose gathers a lane has in flight
 inline size_t f64_smem_bytes(int capb) {
-  return 16 + tma_vbytes<double>(capb) + tma_cbytes(capb);
+  const size_t b = 16 + tma_vbytes<double>(capb) + tma_cbytes(capb);
+  return b > SUM_SMEM ? b : SUM_SMEM;
 }
 
 template <bool DOT>
@@ -473,7 +476,6 @@ __global__ void __launch_bounds__(F64_T, 3)
                const double *__restrict__ x, double *__restrict__ y, double *__restrict__ part,
                int capb, int *err) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double shred[33];
   __shared__ uint32_t rp[F64_ROWS + 1];
   __shared__ uint8_t order[F64_ROWS];
   if (ctl && ctl->status != ST_RUNNING) return;
@@ -548,9 +550,12 @@ __global__ void __launch_bounds__(F64_T, 3)
     }
   }
   if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
-    const double t = block_sum(acc.value(), shred);
+    const double v = acc.value();
+    double t, tot;
+    block_sums<1>(&v, &t, sum_buf(sm));
     SolveCtl *c = const_cast<SolveCtl *>(ctl);
-    finalize_partials(&t, 1, part, &c->tick1, &c->pq_tot, shred);
+    if (finalize_partials<1>(&t, part, &c->tick1, &tot, sum_buf(sm)) && threadIdx.x == 0)
+      c->pq_tot = tot;
   }
 }
 

@@ -35,8 +35,10 @@ inline __host__ __device__ size_t sym_vbytes(int capu) { return align16((size_t)
 inline __host__ __device__ size_t sym_cbytes(int capu) { return align16((size_t)capu * 4 + 32); }
 inline __host__ __device__ size_t sym_lbytes(int capl) { return align16((size_t)capl * 8 + 32); }
 inline size_t sym_smem_bytes(int capu, int capl, int nst) {
-  return align16((size_t)WTMA_WARPS * nst * 8) +
-         (size_t)WTMA_WARPS * nst * (sym_vbytes(capu) + sym_cbytes(capu) + sym_lbytes(capl));
+  const size_t b = align16((size_t)WTMA_WARPS * nst * 8) +
+                   (size_t)WTMA_WARPS * nst *
+                       (sym_vbytes(capu) + sym_cbytes(capu) + sym_lbytes(capl));
+  return b > SUM_SMEM ? b : SUM_SMEM;
 }
 
 // First slot of row v (in [s, e)) whose column is >= key.
@@ -230,7 +232,6 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32, 6)
                  const float *__restrict__ x, float *__restrict__ y, double *__restrict__ part,
                  int capu, int capl, int *err) {
   extern __shared__ __align__(16) unsigned char sm[];
-  __shared__ double shred[33];
   constexpr int RW = SYM_RW, G = SYM_G;
   static_assert(NST >= 2 && NST <= 4, "stages");
   if (ctl && ctl->status != ST_RUNNING) return;
@@ -329,9 +330,12 @@ __global__ void __launch_bounds__(WTMA_WARPS * 32, 6)
     __syncwarp();
   }
   if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
-    const double t = block_sum(acc.value(), shred);
+    const double v = acc.value();
+    double t, tot;
+    block_sums<1>(&v, &t, sum_buf(sm));
     SolveCtl *c = const_cast<SolveCtl *>(ctl);
-    finalize_partials(&t, 1, part, &c->tick1, &c->pq_tot, shred);
+    if (finalize_partials<1>(&t, part, &c->tick1, &tot, sum_buf(sm)) && threadIdx.x == 0)
+      c->pq_tot = tot;
   }
 }
 
