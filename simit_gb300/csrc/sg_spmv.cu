@@ -87,7 +87,14 @@ static int tma_config_t(Ctx *c, int32_t n, const PatternStats &ps, int *grid, si
   const size_t sh = tma_smem_bytes<MT>(capb, NST);
   if (sh > 200 * 1024) return SG_ERR_UNSUPPORTED;
   auto kern = k_bsr3_tma<G, ROWS, NST, MT, VT, DOT>;
-  SG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+  // the limit is the function's, not a matrix's: set once, to the largest any
+  // matrix asks for, or a second one would lower it under the first
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, [&]() -> int {
+    SG_CHECK_CUDA(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    return SG_OK;
+  }));
   int per_sm = 0;
   SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ROWS * G, sh));
   if (per_sm < 1) return SG_ERR_UNSUPPORTED;
@@ -118,7 +125,14 @@ static int wtma_config_t(Ctx *c, int32_t n, const PatternStats &ps, int *grid, s
   const size_t sh = wtma_smem_bytes<MT, BS * BS>(capb, NST);
   if (sh > 200 * 1024) return SG_ERR_UNSUPPORTED;
   auto kern = BS == 3 ? k_bsr3_wtma<G, NST, MT, VT, DOT> : k_csr_wtma<G, NST, P, MT, VT, DOT>;
-  SG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+  // the limit is the function's, not a matrix's: set once, to the largest any
+  // matrix asks for, or a second one would lower it under the first
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, [&]() -> int {
+    SG_CHECK_CUDA(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    return SG_OK;
+  }));
   int per_sm = 0;
   SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WTMA_WARPS * 32, sh));
   if (per_sm < 1) return SG_ERR_UNSUPPORTED;

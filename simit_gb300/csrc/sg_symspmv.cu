@@ -343,7 +343,14 @@ template <bool DOT, int NST> int sym_config_t(Ctx *c, SymBsr *S) {
   const size_t sh = sym_smem_bytes(S->capu, S->capl, NST);
   if (sh > 200 * 1024) return SG_ERR_UNSUPPORTED;
   auto kern = k_sbsr3_wtma<DOT, NST>;
-  SG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+  // the limit is the function's, not a matrix's: set once, to the largest any
+  // matrix asks for, or a second one would lower it under the first
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, [&]() -> int {
+    SG_CHECK_CUDA(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    return SG_OK;
+  }));
   int per_sm = 0;
   SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WTMA_WARPS * 32, sh));
   if (per_sm < 1) return SG_ERR_UNSUPPORTED;

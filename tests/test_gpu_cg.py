@@ -156,3 +156,40 @@ def test_breakdown_then_a_solve(ctx, mixed, precond):
     assert S.solve(b, x).status == 1
     S.close()
     assert np.linalg.norm(x.cpu().numpy() - x0) <= 1e-9 * np.linalg.norm(x0)
+
+
+@pytest.mark.parametrize("bs,opts", [
+    (1, dict(precision=_lib.SOLVE_MIXED, precond=_lib.PRECOND_JACOBI, lanes=-10)),
+    (3, dict(precision=_lib.SOLVE_MIXED, precond=_lib.PRECOND_BLOCK_JACOBI)),
+    (3, dict(precision=_lib.SOLVE_MIXED, precond=_lib.PRECOND_BLOCK_JACOBI, lanes=-2)),
+    (3, dict(precision=_lib.SOLVE_MIXED, precond=_lib.PRECOND_BLOCK_JACOBI, storage=1, wide=40)),
+    (3, dict(precision=_lib.SOLVE_F64, precond=_lib.PRECOND_BLOCK_JACOBI))])
+def test_two_matrices_in_turn(ctx, bs, opts):
+    """A matrix with long rows and one with short rows, whose products stage
+    tiles of different sizes, solved in turn by solvers that both live."""
+    d, n = ctx.device, 5000
+    opts = dict(opts)
+    wide = opts.pop("wide", 90)  # a dense leading block: rows this long
+    rp, ci, vals, mul, _ = _system(n, bs)
+    import scipy.sparse as sp
+    A = sp.bsr_matrix((vals.reshape(-1, bs, bs), ci, rp)).tocsr()
+    W = sp.kron(sp.csr_matrix((np.full((wide, wide), 1 / 64.0).reshape(-1),
+                               (np.repeat(np.arange(wide), wide), np.tile(np.arange(wide), wide))),
+                              shape=(n, n)), sp.identity(bs)).tocsr()
+    out = []
+    for M in (A + W, A):
+        B = M.tobsr((bs, bs))
+        B.sort_indices()
+        S = _solver(ctx, n, bs, B.indptr.astype(np.int32), B.indices.astype(np.int32),
+                    np.ascontiguousarray(B.data).reshape(-1),
+                    torch.float32 if opts["precision"] == _lib.SOLVE_MIXED else torch.float64,
+                    tol=1e-10, maxiters=300, **opts)
+        out.append((S, M))
+    x0 = np.random.default_rng(5).uniform(-1, 1, n * bs)
+    for S, M in out + out[::-1]:
+        b = torch.from_numpy(M @ x0).to(d)
+        x = torch.zeros_like(b)
+        assert S.solve(b, x).status == 1
+        assert np.linalg.norm(x.cpu().numpy() - x0) <= 1e-9 * np.linalg.norm(x0)
+    for S, _ in out:
+        S.close()
