@@ -28,6 +28,8 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <type_traits>
+
 #include "sg_mpnn.cuh"
 #include "sg_solver_kernels.cuh"
 #include "sg_tma.cuh"
@@ -428,7 +430,7 @@ __host__ __device__ constexpr size_t ht_smem_bytes() {
 }
 
 template <typename AT, bool FIN = false>
-__global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
+__global__ void __launch_bounds__(HT_WARPS * 32, 7)
     k_horner(const SolveCtl *ctl, int gate, FoldBufs B, int d,
                  const void *__restrict__ src, void *__restrict__ dst, int first, int *err,
                  FinArgs fa = FinArgs()) {
@@ -491,8 +493,6 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
     fin_partials();
     return;
   }
-  if (threadIdx.x < 9) G[threadIdx.x] = B.g[d * 9 + threadIdx.x];
-  else if (threadIdx.x < 18) G6[threadIdx.x - 9] = B.g[6 * 9 + threadIdx.x - 9];
   uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + warp * HT_NST;
   unsigned char *base =
       sm + (((size_t)HT_WARPS * HT_NST * 8 + 15) & ~size_t(15)) + (size_t)warp * HT_NST * STG;
@@ -500,16 +500,15 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
     for (int b = 0; b < HT_NST; ++b) mbar_init(&bar[b], 1);
     mbar_fence_init();
   }
-  __syncthreads();
+  __syncwarp();
   const AT *__restrict__ aw = (const AT *)B.a;
   const int64_t ns = B.sl.nslice;
   const int64_t gw = (int64_t)blockIdx.x * HT_WARPS + warp;
   const int64_t nw = (int64_t)gridDim.x * HT_WARPS;
   const int64_t my = gw < ns ? (ns - 1 - gw) / nw + 1 : 0;
-  // lane 0: stage slice s in buffer b (or arrive with no bytes when it is
-  // empty or longer than the buffer)
-  auto issue = [&](int64_t s, int b) {
-    const uint32_t p0 = B.sl.ptr[s], p1 = B.sl.ptr[s + 1];
+  // lane 0: stage slice [p0, p1) in buffer b (or arrive with no bytes when it
+  // is empty or longer than the buffer)
+  auto issue = [&](uint32_t p0, uint32_t p1, int b) {
     const uint32_t len = (p1 - p0) / SL_W;
     fence_proxy_async_smem();
     if (len == 0 || len > (uint32_t)HT_CAPL) {
@@ -521,13 +520,33 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
     bulk_g2s(base + (size_t)b * STG, B.sl.col + p0, cb, &bar[b]);
     bulk_g2s(base + (size_t)b * STG + CB, aw + p0, wb, &bar[b]);
   };
-  if (lane == 0)
-    for (int k = 0; k < HT_NST - 1 && k < my; ++k) issue(gw + k * nw, k);
+  // slice bounds of k, k + 1 (to stage next) and k + 2, fetched ahead
+  static_assert(HT_NST == 2, "bounds of one slice ahead");
+  uint32_t p0 = 0, p1 = 0, n0 = 0, n1 = 0;
+  auto bounds = [&](int64_t k, uint32_t &o0, uint32_t &o1) {
+    if (k >= my) return;
+    o0 = __ldg(B.sl.ptr + gw + k * nw);
+    o1 = __ldg(B.sl.ptr + gw + k * nw + 1);
+  };
+  bounds(0, p0, p1);
+  bounds(1, n0, n1);
+  if (lane == 0 && my > 0) issue(p0, p1, 0);
+  if (threadIdx.x < 9) G[threadIdx.x] = B.g[d * 9 + threadIdx.x];
+  else if (threadIdx.x < 18) G6[threadIdx.x - 9] = B.g[6 * 9 + threadIdx.x - 9];
+  __syncthreads();
   for (int64_t k = 0; k < my; ++k) {
     const int b = (int)(k % HT_NST);
     const int64_t s = gw + k * nw;
-    const int64_t kn = k + HT_NST - 1;
-    if (lane == 0 && kn < my) issue(gw + kn * nw, (int)(kn % HT_NST));
+    const int64_t kn = k + 1;
+    if (lane == 0 && kn < my) issue(n0, n1, (int)(kn % HT_NST));
+    // the row's own operands are fetched while the slice arrives
+    const uint32_t v = __ldg(B.sl.row + s * SL_W + lane);
+    float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+    if (v != SL_NONE) ld3<CV>(B.xin, v, x0, x1, x2);
+    const uint32_t q0 = p0, len = (p1 - p0) / SL_W;
+    p0 = n0;
+    p1 = n1;
+    bounds(k + 2, n0, n1);
     const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar[b], (uint32_t)((k / HT_NST) & 1)));
     if (!ok) {
       if (lane == 0) {
@@ -539,26 +558,25 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
       }
       break;
     }
-    const uint32_t v = __ldg(B.sl.row + s * SL_W + lane);
-    const uint32_t p0 = __ldg(B.sl.ptr + s), p1 = __ldg(B.sl.ptr + s + 1);
-    const uint32_t len = (p1 - p0) / SL_W;
     const bool staged = len <= (uint32_t)HT_CAPL;
     const uint32_t *cp = staged ? reinterpret_cast<const uint32_t *>(base + (size_t)b * STG) + lane
-                                : B.sl.col + p0 + lane;
+                                : B.sl.col + q0 + lane;
     const AT *ap = staged ? reinterpret_cast<const AT *>(base + (size_t)b * STG + CB) + lane
-                          : aw + p0 + lane;
+                          : aw + q0 + lane;
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+    // U entries, their gathers in flight together; the rest of a slice goes in
+    // groups of 4, 2 and 1 (an entry at a time, 7 of a 15-entry slice's
+    // gathers waited for one another)
     uint32_t e = 0;
-    constexpr int U = 8;
-    for (; e + U <= len; e += U) {
+    auto group = [&](auto width) {
+      constexpr int U = decltype(width)::value;
       uint32_t u[U];
-      float wq[U];
+      float wq[U], g0[U], g1[U], g2[U];
 #pragma unroll
       for (int j = 0; j < U; ++j) {
         u[j] = cp[(e + j) * SL_W];
         wq[j] = tofloat(ap[(e + j) * SL_W]);
       }
-      float g0[U], g1[U], g2[U];
 #pragma unroll
       for (int j = 0; j < U; ++j) ld3<CV>(src, u[j], g0[j], g1[j], g2[j]);
 #pragma unroll
@@ -567,16 +585,12 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
         m1 += wq[j] * g1[j];
         m2 += wq[j] * g2[j];
       }
-    }
-    for (; e < len; ++e) {
-      const uint32_t u = cp[e * SL_W];
-      const float wq = tofloat(ap[e * SL_W]);
-      float g0, g1, g2;
-      ld3<CV>(src, u, g0, g1, g2);
-      m0 += wq * g0;
-      m1 += wq * g1;
-      m2 += wq * g2;
-    }
+      e += U;
+    };
+    while (e + 8 <= len) group(std::integral_constant<int, 8>());
+    if (e + 4 <= len) group(std::integral_constant<int, 4>());
+    if (e + 2 <= len) group(std::integral_constant<int, 2>());
+    if (e < len) group(std::integral_constant<int, 1>());
     __syncwarp();
     if (v == SL_NONE) continue;
     if (first) {
@@ -585,8 +599,6 @@ __global__ void __launch_bounds__(HT_WARPS * 32, FIN ? 7 : 1)
       m1 = G6[3] * t0 + G6[4] * t1 + G6[5] * t2;
       m2 = G6[6] * t0 + G6[7] * t1 + G6[8] * t2;
     }
-    float x0, x1, x2;
-    ld3<CV>(B.xin, v, x0, x1, x2);
     const float w0 = m0 + G[0] * x0 + G[1] * x1 + G[2] * x2;
     const float w1 = m1 + G[3] * x0 + G[4] * x1 + G[5] * x2;
     const float w2 = m2 + G[6] * x0 + G[7] * x1 + G[8] * x2;

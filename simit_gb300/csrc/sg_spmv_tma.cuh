@@ -30,24 +30,24 @@ template <typename MT> inline size_t tma_smem_bytes(int capb, int nst) {
   return b > SUM_SMEM ? b : SUM_SMEM;
 }
 
-// y_r = (A x)_r for block row r from its tile's values vb and columns cb
-// (block q at vb[q*9 - voff], cb[q - coff]); G lanes per row, lane gl takes
-// blocks rowptr[r]+gl, +G, ...  The first U blocks of each lane (rows of up
+// y_r = (A x)_r for block row r (blocks [rb, e)) from its tile's values vb and
+// columns cb (block q at vb[q*9 - voff], cb[q - coff]); G lanes per row, lane
+// gl takes blocks rb + gl, + G, ...  The first U blocks of each lane (rows of up
 // to 24 blocks) use a fixed, predicated trip count so all of the lane's x
 // gathers are in flight at once; the remainder loop keeps the same
 // accumulation order.  With DOT, acc accumulates x_r . y_r (DotAcc).
 template <int G, typename MT, typename VT, bool DOT>
 __device__ __forceinline__ void tile_row(int64_t r, int gl, unsigned mask,
-                                         const uint32_t *__restrict__ rowptr,
+                                         uint32_t rb, uint32_t e,
                                          const MT *__restrict__ vb,
                                          const uint32_t *__restrict__ cb, size_t voff,
                                          size_t coff, const VT *__restrict__ x,
                                          VT *__restrict__ y, DotAcc<VT> &acc) {
-  const uint32_t e = rowptr[r + 1];
   VT a0 = 0, a1 = 0, a2 = 0;
   constexpr int U = (24 + G - 1) / G;
-  const uint32_t q0 = rowptr[r] + gl;
-  VT xg[U][3];
+  const uint32_t q0 = rb + gl;
+  VT xg[U][3], xr = 0;
+  if (DOT && G >= 3 && gl < 3) xr = x[(size_t)r * 3 + gl];  // in flight with the gathers
 #pragma unroll
   for (int k = 0; k < U; ++k) {
     const uint32_t q = q0 + k * G;
@@ -86,7 +86,7 @@ __device__ __forceinline__ void tile_row(int64_t r, int gl, unsigned mask,
     if (gl < 3) {
       const VT yv = gl == 0 ? a0 : (gl == 1 ? a1 : a2);
       y[(size_t)r * 3 + gl] = yv;
-      if (DOT) acc.add(x[(size_t)r * 3 + gl], yv);
+      if (DOT) acc.add(xr, yv);
     }
   } else if (gl == 0) {  // fewer than 3 lanes: lane 0 writes the row
     y[(size_t)r * 3 + 0] = a0;
@@ -104,16 +104,16 @@ __device__ __forceinline__ void tile_row(int64_t r, int gl, unsigned mask,
 // same lane split, predicated gathers and accumulation order as tile_row.
 template <int G, typename MT, typename VT, bool DOT>
 __device__ __forceinline__ void tile_row1(int64_t r, int gl, unsigned mask,
-                                          const uint32_t *__restrict__ rowptr,
+                                          uint32_t rb, uint32_t e,
                                           const MT *__restrict__ vb,
                                           const uint32_t *__restrict__ cb, size_t voff,
                                           size_t coff, const VT *__restrict__ x,
                                           VT *__restrict__ y, DotAcc<VT> &acc) {
-  const uint32_t e = rowptr[r + 1];
   VT a = 0;
   constexpr int U = (24 + G - 1) / G;
-  const uint32_t q0 = rowptr[r] + gl;
-  VT xg[U];
+  const uint32_t q0 = rb + gl;
+  VT xg[U], xr = 0;
+  if (DOT && gl == 0) xr = x[r];
 #pragma unroll
   for (int k = 0; k < U; ++k) {
     const uint32_t q = q0 + k * G;
@@ -129,7 +129,7 @@ __device__ __forceinline__ void tile_row1(int64_t r, int gl, unsigned mask,
   a = group_sum<G>(a, mask);
   if (gl == 0) {
     y[r] = a;
-    if (DOT) acc.add(x[r], a);
+    if (DOT) acc.add(xr, a);
   }
 }
 
@@ -237,9 +237,11 @@ __global__ void __launch_bounds__(ROWS *G)
       // two inlined copies: shared-memory loads for a staged tile, global
       // loads for an oversize one
       if (staged)
-        tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr, vbuf(b), cbuf(b), vs / S, cs / 4, x, y, acc);
+        tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr[r], rowptr[r + 1], vbuf(b), cbuf(b), vs / S,
+                                 cs / 4, x, y, acc);
       else
-        tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr, vals, colidx, 0, 0, x, y, acc);
+        tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr[r], rowptr[r + 1], vals, colidx, 0, 0, x, y,
+                                 acc);
     }
     __syncthreads();
   }
@@ -305,27 +307,47 @@ __device__ __forceinline__ void wtma_body(const SolveCtl *__restrict__ ctl, int3
   const int64_t gw = (int64_t)blockIdx.x * WTMA_WARPS + warp;
   const int64_t nw = (int64_t)gridDim.x * WTMA_WARPS;
   const int64_t my = gw < ntiles ? (ntiles - 1 - gw) / nw + 1 : 0;
-  auto issue = [&](int64_t tile, int b) {
-    const int64_t r0 = tile * RW;
-    const int64_t r1 = min((int64_t)n, r0 + RW);
-    const uint32_t b0 = rowptr[r0], b1 = rowptr[r1];
-    const size_t vs = ((size_t)b0 * BB * S) & ~size_t(15), ve = ((size_t)b1 * BB * S) & ~size_t(15);
-    const size_t cs = ((size_t)b0 * 4) & ~size_t(15), ce = ((size_t)b1 * 4) & ~size_t(15);
+  // Row pointers of tiles k .. k + NST, a lane each (value i of a tile in
+  // lane i % 32 of register i / 32), fetched a tile before they are needed:
+  // neither the copies nor the rows wait for them.
+  constexpr int NRP = RW / 32 + 1;
+  uint32_t rp[NST + 1][NRP];
+  auto fetch = [&](int64_t k, uint32_t *o) {
+    const int64_t r0 = (gw + k * nw) * RW;
+#pragma unroll
+    for (int j = 0; j < NRP; ++j) {
+      const int64_t i = min((int64_t)n, r0 + min(RW, 32 * j + lane));
+      o[j] = k < my ? rowptr[i] : 0u;
+    }
+  };
+  auto pointer = [&](const uint32_t *o, int i) {
+    return __shfl_sync(0xffffffffu, o[i / 32], i % 32);
+  };
+  // A tile's copies are rounded up to 16 bytes where the matrix goes on
+  // behind it; vlim, clim: the last 16-byte boundary inside the arrays.
+  const size_t vlim = ((size_t)rowptr[n] * BB * S) & ~size_t(15);
+  const size_t clim = ((size_t)rowptr[n] * 4) & ~size_t(15);
+  auto up = [](size_t bytes, size_t lim) { return min((bytes + 15) & ~size_t(15), lim); };
+  auto issue = [&](uint32_t b0, uint32_t b1, int b) {
+    const size_t vs = ((size_t)b0 * BB * S) & ~size_t(15), ve = up((size_t)b1 * BB * S, vlim);
+    const size_t cs = ((size_t)b0 * 4) & ~size_t(15), ce = up((size_t)b1 * 4, clim);
     fence_proxy_async_smem();
     if (b1 - b0 > (uint32_t)capb) {  // larger than the buffers: read from global
       mbar_arrive_expect_tx(&bar[b], 0);
       return;
     }
-    mbar_arrive_expect_tx(&bar[b], (uint32_t)((ve - vs) + (ce - cs)));
-    if (ve > vs)
-      bulk_g2s(vbuf(b), reinterpret_cast<const unsigned char *>(vals) + vs, (uint32_t)(ve - vs),
-               &bar[b]);
-    if (ce > cs)
-      bulk_g2s(cbuf(b), reinterpret_cast<const unsigned char *>(colidx) + cs,
-               (uint32_t)(ce - cs), &bar[b]);
+    const uint32_t vb = ve > vs ? (uint32_t)(ve - vs) : 0u, cb = ce > cs ? (uint32_t)(ce - cs) : 0u;
+    mbar_arrive_expect_tx(&bar[b], vb + cb);
+    if (vb) bulk_g2s(vbuf(b), reinterpret_cast<const unsigned char *>(vals) + vs, vb, &bar[b]);
+    if (cb) bulk_g2s(cbuf(b), reinterpret_cast<const unsigned char *>(colidx) + cs, cb, &bar[b]);
   };
-  if (lane == 0)
-    for (int k = 0; k < NST - 1 && k < my; ++k) issue(gw + k * nw, k);
+#pragma unroll
+  for (int k = 0; k < NST; ++k) fetch(k, rp[k]);
+#pragma unroll
+  for (int k = 0; k < NST - 1; ++k) {
+    const uint32_t b0 = pointer(rp[k], 0), b1 = pointer(rp[k], RW);
+    if (lane == 0 && k < my) issue(b0, b1, k);
+  }
   const int gl = lane & (G - 1);
   const unsigned mask = group_mask<G>();
   DotAcc<VT> acc;
@@ -333,7 +355,11 @@ __device__ __forceinline__ void wtma_body(const SolveCtl *__restrict__ ctl, int3
     const int b = (int)(k % NST);
     const int64_t tile = gw + k * nw;
     const int64_t kn = k + NST - 1;
-    if (lane == 0 && kn < my) issue(gw + kn * nw, (int)(kn % NST));
+    {
+      const uint32_t b0 = pointer(rp[NST - 1], 0), b1 = pointer(rp[NST - 1], RW);
+      if (lane == 0 && kn < my) issue(b0, b1, (int)(kn % NST));
+    }
+    fetch(k + NST, rp[NST]);
     const bool ok = __all_sync(0xffffffffu, mbar_wait(&bar[b], (uint32_t)((k / NST) & 1)));
     if (!ok) {
       if (lane == 0) {
@@ -347,40 +373,51 @@ __device__ __forceinline__ void wtma_body(const SolveCtl *__restrict__ ctl, int3
       break;
     }
     const int64_t r0 = tile * RW;
-    const uint32_t b0 = rowptr[r0], b1 = rowptr[min((int64_t)n, r0 + RW)];
+    const uint32_t b0 = pointer(rp[0], 0), b1 = pointer(rp[0], RW);
     const bool staged = b1 - b0 <= (uint32_t)capb;
     const size_t vs = staged ? ((size_t)b0 * BB * S) & ~size_t(15) : 0;
     const size_t cs = staged ? ((size_t)b0 * 4) & ~size_t(15) : 0;
-    if (staged) {
-      // unaligned tails (< 16 bytes each)
-      const size_t ve = ((size_t)b1 * BB * S) & ~size_t(15), ce = ((size_t)b1 * 4) & ~size_t(15);
-      const int vt = (int)(((size_t)b1 * BB * S - ve) / S);
-      const int ct = (int)(((size_t)b1 * 4 - ce) / 4);
-      if (lane < vt) vbuf(b)[(ve - vs) / S + lane] = vals[ve / S + lane];
-      if (lane >= 16 && lane < 16 + ct)
-        cbuf(b)[(ce - cs) / 4 + lane - 16] = colidx[ce / 4 + lane - 16];
+    if (staged && ((size_t)b1 * BB * S > vlim || (size_t)b1 * 4 > clim)) {
+      // the matrix's end: unaligned tails (< 16 bytes each)
+      const size_t ve = max(vs, up((size_t)b1 * BB * S, vlim)), ce = max(cs, up((size_t)b1 * 4, clim));
+      if (ve / S + lane < (size_t)b1 * BB)
+        vbuf(b)[(ve - vs) / S + lane] = vals[ve / S + lane];
+      if (ce / 4 + lane < b1) cbuf(b)[(ce - cs) / 4 + lane] = colidx[ce / 4 + lane];
+      __syncwarp();
+    }
+#pragma unroll
+    for (int pp = 0; pp < P; ++pp) {
+      const int i = pp * (32 / G) + lane / G;  // the row within the tile
+      constexpr int NP = NRP - 1;
+      const int j = pp * (32 / G) / 32;
+      const uint32_t rb = __shfl_sync(0xffffffffu, rp[0][j], i % 32);
+      uint32_t re = __shfl_sync(0xffffffffu, rp[0][j], (i + 1) % 32);
+      if (NP > 0) {
+        const uint32_t re2 = __shfl_sync(0xffffffffu, rp[0][min(j + 1, NP)], (i + 1) % 32);
+        if ((i + 1) / 32 != j) re = re2;
+      }
+      const int64_t r = r0 + i;
+      if (r < n) {
+        if (BS == 3) {
+          if (staged)
+            tile_row<G, MT, VT, DOT>(r, gl, mask, rb, re, vbuf(b), cbuf(b), vs / S, cs / 4, x, y,
+                                     acc);
+          else
+            tile_row<G, MT, VT, DOT>(r, gl, mask, rb, re, vals, colidx, 0, 0, x, y, acc);
+        } else {
+          if (staged)
+            tile_row1<G, MT, VT, DOT>(r, gl, mask, rb, re, vbuf(b), cbuf(b), vs / S, cs / 4, x, y,
+                                      acc);
+          else
+            tile_row1<G, MT, VT, DOT>(r, gl, mask, rb, re, vals, colidx, 0, 0, x, y, acc);
+        }
+      }
     }
     __syncwarp();
 #pragma unroll
-    for (int pp = 0; pp < P; ++pp) {
-    const int64_t r = r0 + pp * (32 / G) + lane / G;
-    if (r < n) {
-      if (BS == 3) {
-        if (staged)
-          tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr, vbuf(b), cbuf(b), vs / S, cs / 4, x, y,
-                                   acc);
-        else
-          tile_row<G, MT, VT, DOT>(r, gl, mask, rowptr, vals, colidx, 0, 0, x, y, acc);
-      } else {
-        if (staged)
-          tile_row1<G, MT, VT, DOT>(r, gl, mask, rowptr, vbuf(b), cbuf(b), vs / S, cs / 4, x, y,
-                                    acc);
-        else
-          tile_row1<G, MT, VT, DOT>(r, gl, mask, rowptr, vals, colidx, 0, 0, x, y, acc);
-      }
-    }
-    }
-    __syncwarp();
+    for (int t = 0; t < NST; ++t)
+#pragma unroll
+      for (int j = 0; j < NRP; ++j) rp[t][j] = rp[t + 1][j];
   }
   if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
     const double v = acc.value();
