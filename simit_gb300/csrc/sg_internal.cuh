@@ -50,6 +50,7 @@ struct Ctx {
   int32_t mr_t4[MAXROW_CACHE] = {};   // largest 4-row tile
   int32_t mr_t8[MAXROW_CACHE] = {};   // largest 8-row tile
   int64_t mr_nnzb[MAXROW_CACHE] = {};
+  unsigned long long mr_wlong[MAXROW_CACHE] = {};
   int mr_next = 0;
   int refs = 1;  // sg_ctx_destroy + one per live solver
   // Set while a solver captures its iteration graph: kernels launched with

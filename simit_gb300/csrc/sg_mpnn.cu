@@ -86,10 +86,11 @@ __global__ void __launch_bounds__(RED_T) k_rz_zq(SolveCtl *ctl, int par, int64_t
   }
   const double v[2] = {rz.value(), zq.value()};
   double t[3], tot[3];
+  const DecideIn in = decide_in(ctl, par);
   block_sums<2>(v, t + 1, sh);
   t[0] = part[blockIdx.x];
   if (finalize_partials<3>(t, part, &ctl->tick2, tot, sh) && threadIdx.x == 0)
-    cg_decide(ctl, par, tot[0], tot[1], tot[2], ctl->last_alpha);
+    cg_decide(ctl, par, in, tot[0], tot[1], tot[2]);
 }
 
 // ---------------------------------------------------------------------------

@@ -474,9 +474,10 @@ __global__ void __launch_bounds__(HT_WARPS * 32, 7)
     static_assert(ht_smem_bytes<AT>() >= SUM_OFF + 3 * HT_WARPS * 32 * 8, "sums");
     const double v[3] = {rr.value(), rz.value(), zq.value()};
     double t[3], tot[3];
+    const DecideIn in = decide_in(fa.ctl, fa.par);
     block_sums<3>(v, t, sum_buf(sm));
     if (finalize_partials<3>(t, fa.part, &fa.ctl->tick2, tot, sum_buf(sm)) && threadIdx.x == 0)
-      cg_decide(fa.ctl, fa.par, tot[0], tot[1], tot[2], fa.ctl->last_alpha);
+      cg_decide(fa.ctl, fa.par, in, tot[0], tot[1], tot[2]);
   };
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (FIN && fb) {

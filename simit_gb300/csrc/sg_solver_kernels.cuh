@@ -188,21 +188,44 @@ __device__ __forceinline__ bool cg_alpha(SolveCtl *ctl, int par, double *sa, dou
   return ok;
 }
 
+// What cg_decide reads of the control block.  No kernel that decides writes
+// it, so every block's thread 0 fetches it before the sums: the last block,
+// which works alone, would wait for each value in turn.
+struct DecideIn {
+  double rzold = 0.0, tol2 = 0.0, upd2 = 0.0, alpha = 0.0;
+  int it = 0, maxiters = 0, check_every = 0, flexible = 0, fallback = 0;
+};
+__device__ __forceinline__ DecideIn decide_in(const SolveCtl *ctl, int par) {
+  DecideIn d;
+  if (threadIdx.x == 0) {
+    d.rzold = ctl->rz[par];
+    d.tol2 = ctl->tol2;
+    d.upd2 = ctl->upd2;
+    d.alpha = ctl->last_alpha;
+    d.it = ctl->iter[par] + 1;
+    d.maxiters = ctl->maxiters;
+    d.check_every = ctl->check_every;
+    d.flexible = ctl->flexible;
+    d.fallback = ctl->fallback;
+  }
+  return d;
+}
+
 // The control decision after K2's dots (or the external preconditioner's):
 // iteration count, r.z slot, status, beta.  Executed by one thread of the
-// block that finished last, for K3.
-__device__ __forceinline__ void cg_decide(SolveCtl *ctl, int par, double rr, double rznew,
-                                         double zq, double alpha) {
-  const double rzold = ctl->rz[par];
-  const int it = ctl->iter[par] + 1;
+// block that finished last, for K3.  d.alpha: this iteration's.
+__device__ __forceinline__ void cg_decide(SolveCtl *ctl, int par, const DecideIn &d, double rr,
+                                         double rznew, double zq) {
+  const double rzold = d.rzold, alpha = d.alpha;
+  const int it = d.it;
   int st = ST_RUNNING;
-  const bool lost = ctl->flexible && !ctl->fallback && !(rznew > 0.0);
+  const bool lost = d.flexible && !d.fallback && !(rznew > 0.0);
   if (lost) st = ST_NEED_CHECK;  // z is no descent direction: fall back
   else if (!isfinite(rr) || !isfinite(rznew)) st = ST_NAN;
-  else if (rr <= ctl->tol2) st = ST_NEED_CHECK;
-  else if (ctl->upd2 > 0.0 && rr < ctl->upd2) st = ST_NEED_CHECK;
-  else if (ctl->check_every > 0 && it % ctl->check_every == 0) st = ST_NEED_CHECK;
-  else if (it >= ctl->maxiters) st = ST_MAXITER;
+  else if (rr <= d.tol2) st = ST_NEED_CHECK;
+  else if (d.upd2 > 0.0 && rr < d.upd2) st = ST_NEED_CHECK;
+  else if (d.check_every > 0 && it % d.check_every == 0) st = ST_NEED_CHECK;
+  else if (it >= d.maxiters) st = ST_MAXITER;
   ctl->iter[par ^ 1] = it;
   ctl->rz[par ^ 1] = rznew;
   ctl->last_rr = rr;
@@ -212,7 +235,7 @@ __device__ __forceinline__ void cg_decide(SolveCtl *ctl, int par, double rr, dou
   // Fletcher-Reeves (the reference's beta = r'r_new / r'r_old, with z) or
   // Polak-Ribiere for a variable preconditioner: (z.r_new - z.r_old)/rz_old
   // where r_new - r_old = -alpha q.
-  const double beta = ctl->flexible ? (-alpha * zq) / rzold : rznew / rzold;
+  const double beta = d.flexible ? (-alpha * zq) / rzold : rznew / rzold;
   ctl->beta = beta;
   ctl->beta32 = (float)beta;
   if (st != ST_RUNNING) ctl->status = st;
@@ -322,8 +345,8 @@ enum PrecKind : int { PK_NONE = 0, PK_JACOBI = 1, PK_BLOCK3 = 2, PK_EXTERNAL = 3
 // for K3.  A thread takes two entries (16-byte accesses; the buffers are
 // cudaMalloc'd) or, with block Jacobi, one vertex.  Bound by the latency of
 // its loads and of the two-level sums at the sizes that fit in L2: heat 64^3
-// (275 k rows, 17.6 MB touched) 14.1 us when every block of the next kernel
-// summed the partials again, FIGK2F64 so.
+// (275 k rows, 15 MB touched) 14.1 us when every warp divided alpha and summed
+// the partials of the kernel before, 10.1 so; K3 12.3 and 3.3.
 template <int PREC>
 __global__ void __launch_bounds__(RED_T, 4) k_cg_update_f64(
     SolveCtl *ctl, int par, int64_t len, const double *__restrict__ p,
@@ -402,9 +425,11 @@ __global__ void __launch_bounds__(RED_T, 4) k_cg_update_f64(
     if (PREC == PK_NONE) acc[1] = acc[0];  // z is r
   }
   double t[2], tot[2];
+  DecideIn d = decide_in(ctl, par);
+  d.alpha = alpha;
   block_sums<2>(acc, t, sh);
   if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
-    cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
+    cg_decide(ctl, par, d, tot[0], tot[1], 0.0);
 }
 
 // K3 in FP64: p = z + beta p, two entries per thread.
@@ -506,9 +531,11 @@ __global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
       if (blockIdx.x == 0) ctl->last_alpha = alpha;
     }
   } else {
+    DecideIn d = decide_in(ctl, par);
+    d.alpha = alpha;
     block_sums<2>(acc, t, sh);
     if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
-      cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
+      cg_decide(ctl, par, d, tot[0], tot[1], 0.0);
   }
 }
 
@@ -523,9 +550,9 @@ __global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
 // while the status and alpha are fetched.  The last len % 12 entries are done
 // by the scalar tail of thread 0 of the last CTA.  Bound, below a few hundred
 // thousand vertices, by latency and the FP64 pipe of the SMs that hold the
-// (few) blocks: 36 k vertices, one chunk per warp, 11.5 us with alpha divided
-// by every warp, conversions on the FP64 pipe and three sums one after the
-// other, FIGK2W so.
+// (few) blocks: 8,257 vertices 11.5 us with alpha divided by every warp,
+// conversions on the FP64 pipe, three sums one after the other and 8 chunks
+// to a block, 7.8 so.
 constexpr int K2W_WARPS = 8;  // at most; a block has blockDim.x / 32
 struct K2WarpSmem {
   float4 q[96], r[96], d[192];
@@ -649,9 +676,11 @@ static __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
   }
   const double acc[2] = {rr.value(), rzs.value()};
   double t[2], tot[2];
+  DecideIn d = decide_in(ctl, par);
+  d.alpha = alpha;
   block_sums<2>(acc, t, sh);
   if (finalize_partials<2>(t, part_out, &ctl->tick2, tot, sh) && threadIdx.x == 0)
-    cg_decide(ctl, par, tot[0], tot[1], 0.0, alpha);
+    cg_decide(ctl, par, d, tot[0], tot[1], 0.0);
 }
 
 // K3 for FP32 vectors: p = z + beta p with float4 accesses.

@@ -32,8 +32,21 @@ int default_tma_variant(int bs) { return bs == 1 ? kDefaultTmaVariant1 : kDefaul
 // g = 0).  Its tiles of 64 rows leave SMs without work on small matrices, where
 // the streaming kernel's shorter chain wins: 729 rows 9.2 us against 8.7, 4,913
 // rows 8.8 against 9.1, 9,261 rows 8.9 against 10.5.
+// Scalar FP64 matrices: k_csr_f64 (a lane per row, rows sorted by length
+// within 64) from 32,768 rows, up to 16 entries per row on average, and where
+// neighbouring rows are of like length: nnz at least kF64Fill1 of the 32-row
+// tiles' longest rows times 32.  Against the lanes per row that default_lanes
+// takes otherwise, L2 cold: 15-point lattices (0.98 and more) 48^3 15.0
+// against 17.0 us, 64^3 23.2 / 27.3, 96^3 49.8 / 74.4, 128^3 92.8 / 183;
+// 7-point 100^3 31.4 / 39.6; 7- and 19-point rows in turn (0.73) 64^3 19.1 /
+// 25.2, 100^3 43.7 / 60.1.  Slower, hence the bounds: random lengths 1 to 15
+// (0.54) 47.8 / 33.4 at 500,000 rows; 27-point 64^3 39.6 / 33.4; 15-point
+// 24^3 10.9 / 8.9.
 constexpr int kF64Variant = kNumTmaVariants;
-int default_f64_variant(int32_t n, int bs) { return bs == 3 && n >= 4096 ? kF64Variant : -1; }
+constexpr double kF64Fill1 = 0.64;
+int default_f64_variant(int32_t n, int bs) {
+  return (bs == 3 && n >= 4096) || (bs == 1 && n >= 32768) ? kF64Variant : -1;
+}
 
 template <bool DOT>
 static int f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size_t *smem,
@@ -79,6 +92,43 @@ static int tile_cap(int rows, const PatternStats &ps) {
               : rows == 4  ? ps.tile4
               : rows == 8  ? ps.tile8 : 0;
   return (t > 0 && t < bound) ? t : bound;
+}
+
+// Largest number of entries in a tile of k_csr_f64.
+static int csr_f64_cap(const PatternStats &ps) {
+  const int bound = C1_ROWS * (ps.maxrow > 0 ? ps.maxrow : 1);
+  const int t = ps.tile32 * (C1_ROWS / 32);
+  return t > 0 && t < bound ? t : bound;
+}
+
+template <bool DOT>
+static int csr_f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size_t *smem) {
+  *smem = c1_smem_bytes(csr_f64_cap(ps));
+  if (*smem > 200 * 1024) return SG_ERR_UNSUPPORTED;
+  static PerDeviceOnce attr;
+  SG_TRY(once_per_device(attr, c->device, []() -> int {
+    SG_CHECK_CUDA(cudaFuncSetAttribute(k_csr_f64<DOT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       200 * 1024));
+    return SG_OK;
+  }));
+  int per_sm = 0;
+  SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_csr_f64<DOT>,
+                                                              WTMA_WARPS * 32, *smem));
+  if (per_sm < 1) return SG_ERR_UNSUPPORTED;
+  const int64_t rows = (int64_t)C1_ROWS * WTMA_WARPS, need = ((int64_t)n + rows - 1) / rows;
+  const int64_t all = (int64_t)per_sm * c->num_sms;
+  *grid = (int)(need < all ? need : all);
+  return SG_OK;
+}
+
+template <bool DOT>
+static int csr_f64_launch(Ctx *c, cudaStream_t st, const SolveCtl *ctl, int32_t n,
+                          const uint32_t *rp, const uint32_t *ci, const void *v, const void *x,
+                          void *y, double *part, const PatternStats &ps, int grid, size_t smem) {
+  SG_CHECK_CUDA(launch_k(c, k_csr_f64<DOT>, grid, WTMA_WARPS * 32, smem, st, ctl, n, rp, ci,
+                         (const double *)v, (const double *)x, (double *)y, part, csr_f64_cap(ps),
+                         c->d_err));
+  return SG_OK;
 }
 
 template <int G, int ROWS, int NST, typename MT, typename VT, bool DOT>
@@ -226,7 +276,17 @@ static int tma_any(Ctx *c, cudaStream_t st, bool launch, int bs, int vdt, int xd
                    int *grid, size_t *smem) {
   const SolveCtl *k = (const SolveCtl *)ctl;
   if (var == kF64Variant) {
-    if (bs != 3 || vdt != SG_F64 || xdt != SG_F64) return SG_ERR_UNSUPPORTED;
+    if ((bs != 3 && bs != 1) || vdt != SG_F64 || xdt != SG_F64) return SG_ERR_UNSUPPORTED;
+    if (bs == 1) {
+      if (!launch && (ps.nnzb > 16 * (int64_t)n ||
+                      (double)ps.nnzb < kF64Fill1 * 32.0 * (double)ps.wlong))
+        return SG_ERR_UNSUPPORTED;
+      if (launch)
+        return dot ? csr_f64_launch<true>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid, *smem)
+                   : csr_f64_launch<false>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid, *smem);
+      return dot ? csr_f64_config<true>(c, n, ps, grid, smem)
+                 : csr_f64_config<false>(c, n, ps, grid, smem);
+    }
     if (launch)
       return dot ? f64_launch<true>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid)
                  : f64_launch<false>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid);
@@ -264,9 +324,14 @@ int bsr3_tma_launch(Ctx *c, cudaStream_t st, const void *ctl, int bs, int vdt, i
 __global__ void k_pattern_stats(const uint32_t *rowptr, int32_t n, uint32_t *out) {
   if (blockIdx.x == 0 && threadIdx.x == 0) out[5] = rowptr[n];
   uint32_t mr = 0, t16 = 0, t32 = 0, t4 = 0, t8 = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    mr = max(mr, rowptr[i + 1] - rowptr[i]);
+  unsigned long long wl = 0;  // longest rows of the 32-row tiles, added up
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < n;
+       i0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = i0 + (threadIdx.x & 31);
+    const uint32_t len = i < n ? rowptr[i + 1] - rowptr[i] : 0u;
+    wl += __reduce_max_sync(0xffffffffu, len);
+    if (i >= n) continue;
+    mr = max(mr, len);
     if (i % 16 == 0) t16 = max(t16, rowptr[min((int64_t)n, i + 16)] - rowptr[i]);
     if (i % 32 == 0) t32 = max(t32, rowptr[min((int64_t)n, i + 32)] - rowptr[i]);
     if (i % 4 == 0) t4 = max(t4, rowptr[min((int64_t)n, i + 4)] - rowptr[i]);
@@ -285,6 +350,7 @@ __global__ void k_pattern_stats(const uint32_t *rowptr, int32_t n, uint32_t *out
     atomicMax(&out[2], t32);
     atomicMax(&out[3], t4);
     atomicMax(&out[4], t8);
+    atomicAdd(reinterpret_cast<unsigned long long *>(out + 6), wl);
   }
 }
 
@@ -304,6 +370,7 @@ int cached_stats(Ctx *c, int32_t n, const uint32_t *rowptr, PatternStats *ps, bo
     ps->tile4 = c->mr_t4[slot];
     ps->tile8 = c->mr_t8[slot];
     ps->nnzb = c->mr_nnzb[slot];
+    ps->wlong = c->mr_wlong[slot];
     return SG_OK;
   }
   Scratch s(c);
@@ -326,6 +393,7 @@ int cached_stats(Ctx *c, int32_t n, const uint32_t *rowptr, PatternStats *ps, bo
   c->mr_t4[slot] = ps->tile4 = (int32_t)h[3];
   c->mr_t8[slot] = ps->tile8 = (int32_t)h[4];
   c->mr_nnzb[slot] = ps->nnzb = h[5];
+  c->mr_wlong[slot] = ps->wlong = *(const unsigned long long *)(h + 6);
   return SG_OK;
 }
 
@@ -501,8 +569,7 @@ extern "C" int sg_bspmv(sg_ctx *h, int32_t n, int32_t bs, const uint32_t *rowptr
   const int fvar = f64 ? default_f64_variant(n, bs) : default_tma_variant(bs);
   if ((g == 0 && (bs == 3 || bs == 1) && aligned && fvar >= 0) || g < 0) {
     // TMA-staged kernel (lanes per row from the row length unless given).
-    // Small and scalar FP64 matrices default to the plain kernel, which keeps
-    // more warps in flight for the FP64 pipe.
+    // Small FP64 matrices default to the plain kernel.
     int grid = 0;
     size_t sh = 0;
     PatternStats ps;

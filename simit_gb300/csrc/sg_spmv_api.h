@@ -8,6 +8,7 @@ struct Ctx;
 struct PatternStats {
   int maxrow = 0, tile16 = 0, tile32 = 0, tile4 = 0, tile8 = 0;
   int64_t nnzb = 0;
+  unsigned long long wlong = 0;  // sum of the longest rows of the 32-row tiles
 };
 int default_lanes(int32_t n, int64_t nnzb, int32_t bs);
 int default_tma_variant(int bs);

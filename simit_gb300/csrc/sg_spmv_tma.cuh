@@ -596,4 +596,193 @@ __global__ void __launch_bounds__(F64_T, 3)
   }
 }
 
+// FP64 scalar row, one lane per row, called by the whole warp (a lane without
+// a row passes rb = re).  Entries go 8 at a time, their gathers in flight together,
+// the rest in one group of the exact width (a predicated-off multiply-add
+// still takes its place on the pipe); lanes whose row has ended add 0 * 0.
+// Even and odd entries have a sum each: half the dependent chain.
+template <bool DOT>
+__device__ __forceinline__ void csr_row_f64(int64_t r, bool row, uint32_t rb, uint32_t re,
+                                            const double *__restrict__ vb,
+                                            const uint32_t *__restrict__ cb, size_t voff,
+                                            size_t coff, const double *__restrict__ x,
+                                            double *__restrict__ y, DotAcc<double> &acc) {
+  const uint32_t longest = __reduce_max_sync(0xffffffffu, re - rb);
+  double a[2] = {0.0, 0.0}, xr = 0.0;
+  if (DOT && row) xr = x[r];
+  uint32_t k = 0;
+  auto group = [&](auto width) {
+    constexpr int U = decltype(width)::value;
+    double xg[U], vg[U];
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const uint32_t q = rb + k + j;
+      xg[j] = vg[j] = 0.0;
+      if (q < re) {
+        xg[j] = ldg(x + cb[q - coff]);
+        vg[j] = vb[q - voff];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < U; ++j) a[j & 1] = fma(vg[j], xg[j], a[j & 1]);
+    k += U;
+  };
+  while (k + 8 <= longest) group(std::integral_constant<int, 8>());
+  switch (longest - k) {
+    case 7: group(std::integral_constant<int, 7>()); break;
+    case 6: group(std::integral_constant<int, 6>()); break;
+    case 5: group(std::integral_constant<int, 5>()); break;
+    case 4: group(std::integral_constant<int, 4>()); break;
+    case 3: group(std::integral_constant<int, 3>()); break;
+    case 2: group(std::integral_constant<int, 2>()); break;
+    case 1: group(std::integral_constant<int, 1>()); break;
+    default: break;
+  }
+  const double yv = a[0] + a[1];
+  if (row) {
+    y[r] = yv;
+    if (DOT) acc.add(xr, yv);
+  }
+}
+
+// FP64 scalar SpMV, a lane per row, rows sorted by length inside a warp's
+// tile.  Bound by the FP64 pipe, which takes a warp's multiply-add every 16
+// cycles whether 32 lanes use it or one.  G lanes per row waste lanes where G
+// does not divide the row and add shuffle sums on the same pipe; a lane per
+// row wastes what its row is shorter than the warp's longest.  So a warp
+// takes C1_ROWS rows at a time, copies their values and columns to shared
+// memory (one bulk copy each), sorts the rows by length meanwhile (radix sort
+// on the bits in which the lengths differ, by ballots: no order depends on
+// timing), and takes them in two passes of like rows: the 64^3 heat lattice,
+// whose rows of 7 and 19 entries alternate, uses 99 % of its lanes (68 %
+// unsorted): 22.3 us with two lanes per row inside its solve, 17.1 so.  One
+// stage per warp; 16 or more warps per SM overlap one another.  x is gathered
+// through L1, adjacent rows mostly at adjacent columns.
+constexpr int C1_ROWS = 64;
+
+inline size_t c1_smem_bytes(int capb) {
+  const size_t b = 64 + (size_t)WTMA_WARPS * (tma_vbytes<double, 1>(capb) + tma_cbytes(capb));
+  return b > SUM_SMEM ? b : SUM_SMEM;
+}
+
+template <bool DOT>
+__global__ void __launch_bounds__(WTMA_WARPS * 32)
+    k_csr_f64(const SolveCtl *__restrict__ ctl, int32_t n, const uint32_t *__restrict__ rowptr,
+              const uint32_t *__restrict__ colidx, const double *__restrict__ vals,
+              const double *__restrict__ x, double *__restrict__ y, double *__restrict__ part,
+              int capb, int *err) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ uint32_t keys[WTMA_WARPS][C1_ROWS];
+  pdl_wait_and_release();
+  if (ctl && ctl->status != ST_RUNNING) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr unsigned FULL = 0xffffffffu;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + warp;
+  const size_t vbytes = tma_vbytes<double, 1>(capb);
+  unsigned char *base = sm + 64 + (size_t)warp * (vbytes + tma_cbytes(capb));
+  double *vb = reinterpret_cast<double *>(base);
+  uint32_t *cb = reinterpret_cast<uint32_t *>(base + vbytes), *key = keys[warp];
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    mbar_fence_init();
+  }
+  __syncwarp();
+  const int64_t ntiles = ((int64_t)n + C1_ROWS - 1) / C1_ROWS;
+  const int64_t nw = (int64_t)gridDim.x * WTMA_WARPS;
+  int64_t tile = (int64_t)blockIdx.x * WTMA_WARPS + warp;
+  // copies are rounded up to 16 bytes where the matrix goes on behind them
+  const size_t vlim = ((size_t)rowptr[n] * 8) & ~size_t(15);
+  const size_t clim = ((size_t)rowptr[n] * 4) & ~size_t(15);
+  auto up = [](size_t bytes, size_t lim) { return min((bytes + 15) & ~size_t(15), lim); };
+  uint32_t c[3], nx[3] = {0, 0, 0};  // row pointers: value i in lane i % 32 of c[i / 32]
+  auto fetch = [&](int64_t t) {
+    if (t >= ntiles) return;
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+      nx[j] = rowptr[min((int64_t)n, t * C1_ROWS + min(C1_ROWS, 32 * j + lane))];
+  };
+  fetch(tile);
+  DotAcc<double> acc;
+  uint32_t phase = 0;
+  for (; tile < ntiles; tile += nw) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) c[j] = nx[j];
+    const int64_t r0 = tile * C1_ROWS;
+    const uint32_t b0 = __shfl_sync(FULL, c[0], 0), b1 = __shfl_sync(FULL, c[2], 0);
+    const bool staged = b1 - b0 <= (uint32_t)capb;
+    const size_t vs = staged ? ((size_t)b0 * 8) & ~size_t(15) : 0;
+    const size_t cs = staged ? ((size_t)b0 * 4) & ~size_t(15) : 0;
+    const size_t ve = max(vs, up((size_t)b1 * 8, vlim)), ce = max(cs, up((size_t)b1 * 4, clim));
+    __syncwarp();  // the previous tile's buffers are free
+    if (staged && lane == 0) {
+      fence_proxy_async_smem();
+      mbar_arrive_expect_tx(bar, (uint32_t)(ve - vs + (ce - cs)));
+      if (ve > vs)
+        bulk_g2s(vb, reinterpret_cast<const unsigned char *>(vals) + vs, (uint32_t)(ve - vs), bar);
+      if (ce > cs)
+        bulk_g2s(cb, reinterpret_cast<const unsigned char *>(colidx) + cs, (uint32_t)(ce - cs), bar);
+    }
+    fetch(tile + nw);
+    // keys: row length (short rows first) | row, rows lane and 32 + lane
+    uint32_t ea = __shfl_down_sync(FULL, c[0], 1), eb = __shfl_down_sync(FULL, c[1], 1);
+    const uint32_t c1 = __shfl_sync(FULL, c[1], 0);
+    if (lane == 31) {
+      ea = c1;
+      eb = b1;
+    }
+    uint32_t ka = min(ea - c[0], (1u << 26) - 1) << 6 | lane;
+    uint32_t kb = min(eb - c[1], (1u << 26) - 1) << 6 | (32 + lane);
+    const uint32_t k0 = __shfl_sync(FULL, ka, 0);
+    uint32_t diff = __reduce_or_sync(FULL, (ka ^ k0) | (kb ^ k0)) & ~63u;
+    const unsigned below = (1u << lane) - 1u;
+    for (; diff; diff &= diff - 1) {
+      const uint32_t bit = diff & (0u - diff);
+      const unsigned ma = __ballot_sync(FULL, ka & bit), mb = __ballot_sync(FULL, kb & bit);
+      const int za = 32 - __popc(ma), z = za + 32 - __popc(mb);
+      const int oa = __popc(ma & below), ob = __popc(mb & below);
+      key[ka & bit ? z + oa : lane - oa] = ka;
+      key[kb & bit ? z + 32 - za + ob : za + lane - ob] = kb;
+      __syncwarp();
+      ka = key[lane];
+      kb = key[32 + lane];
+      __syncwarp();
+    }
+    if (staged) {
+      const bool ok = __all_sync(FULL, mbar_wait(bar, phase));
+      if (!ok) {
+        if (lane == 0) {
+          atomicCAS(err, 0, 6 /* DEV_TMA_TIMEOUT */);
+          if (!mbar_wait(bar, phase)) atomicExch(err, 8 /* DEV_TMA_UNDRAINED */);
+        }
+        break;
+      }
+      phase ^= 1u;
+      if ((size_t)b1 * 8 > ve || (size_t)b1 * 4 > ce) {  // the matrix's end: unaligned tails
+        if (ve / 8 + lane < b1) vb[(ve - vs) / 8 + lane] = vals[ve / 8 + lane];
+        if (ce / 4 + lane < b1) cb[(ce - cs) / 4 + lane] = colidx[ce / 4 + lane];
+        __syncwarp();
+      }
+    }
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+      const int i = (int)((pass ? kb : ka) & 63u), j = i + 1;
+      const uint32_t s0 = __shfl_sync(FULL, c[0], i & 31), s1 = __shfl_sync(FULL, c[1], i & 31);
+      const uint32_t e0 = __shfl_sync(FULL, c[0], j & 31), e1 = __shfl_sync(FULL, c[1], j & 31);
+      const uint32_t rb = i < 32 ? s0 : s1, re = j < 32 ? e0 : j < 64 ? e1 : b1;
+      if (staged)
+        csr_row_f64<DOT>(r0 + i, r0 + i < n, rb, re, vb, cb, vs / 8, cs / 4, x, y, acc);
+      else
+        csr_row_f64<DOT>(r0 + i, r0 + i < n, rb, re, vals, colidx, 0, 0, x, y, acc);
+    }
+  }
+  if (DOT) {  // CG K1: the last CTA leaves the p.q total in ctl->pq_tot
+    const double v = acc.value();
+    double t, tot;
+    block_sums<1>(&v, &t, sum_buf(sm));
+    SolveCtl *s = const_cast<SolveCtl *>(ctl);
+    if (finalize_partials<1>(&t, part, &s->tick1, &tot, sum_buf(sm)) && threadIdx.x == 0)
+      s->pq_tot = tot;
+  }
+}
+
 }  // namespace sg

@@ -313,3 +313,35 @@ def test_fp64_fma_rate_is_plausible(ctx):
     from simit_gb300.runtime import fp64_fma_rate
     r = fp64_fma_rate(ctx)
     assert 0.1 < r < 20.0, r
+
+
+@pytest.mark.parametrize("n", [32767, 32768, 32769, 32831, 32833, 40000])
+def test_spmv_f64_scalar_sorted_rows(ctx, oracle, n):
+    """The FP64 scalar product at the sizes around its tiles of 64 rows (and
+    below its smallest matrix): rows of 7 and 15 entries in turn, empty rows
+    and one of 40; then rows beyond the buffers under statistics cached for
+    the first pattern.  An entry's products are exact to one rounding each and
+    at most 640 are added: 1e-13 of the sum of magnitudes."""
+    from simit_gb300.runtime import bspmv
+    d = ctx.device
+    t = lambda a: torch.from_numpy(a.view(np.int32) if a.dtype == np.uint32 else a).to(d)  # noqa
+    g = meshgen.rng(n)
+    rp_d = torch.zeros(n + 1, dtype=torch.int32, device=d)
+    ci_d = torch.zeros(20 * n, dtype=torch.int32, device=d)
+    for long_rows in (0, 1):
+        L = np.where(np.arange(n) % 2, 7, 15)
+        L[5::97] = 0
+        L[n - 3] = 40
+        if long_rows:
+            L[64 * 100:64 * 101] = 640
+        rp = np.concatenate([[0], np.cumsum(L)]).astype(np.uint32)
+        ci = ((np.repeat(np.arange(n), L) + np.arange(rp[-1]) * 37) % n).astype(np.uint32)
+        vals, x = g.uniform(-1, 1, size=len(ci)), g.uniform(-1, 1, size=n)
+        rp_d.copy_(t(rp))
+        ci_d[:len(ci)].copy_(t(ci))
+        ref = oracle.spmv(n, 1, rp, ci, vals, x)
+        scale = oracle.spmv(n, 1, rp, ci, np.abs(vals), np.abs(x))
+        y = bspmv(ctx, n, 1, rp_d, ci_d, t(vals), t(x),
+                  y=torch.full((n,), float("nan"), dtype=torch.float64, device=d))
+        ctx.sync()
+        assert np.all(np.abs(y.cpu().numpy() - ref) <= 1e-13 * scale + 1e-300)
