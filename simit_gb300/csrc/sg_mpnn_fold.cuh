@@ -713,7 +713,9 @@ __global__ void __launch_bounds__(RED_T) k_lrn_update(SolveCtl *ctl, int par, in
                                                       const void *__restrict__ l6,
                                                       void *__restrict__ xin) {
   __shared__ double sa;
-  if (ctl->status != ST_RUNNING) return;
+  const int status = ctl->status;
+  const double pq = ctl->pq_tot, rz = ctl->rz[par];
+  if (status != ST_RUNNING) return;
   const int64_t nu = n / 4;
   const float4 *q4 = reinterpret_cast<const float4 *>(q);
   float4 *r4 = reinterpret_cast<float4 *>(r);
@@ -733,7 +735,7 @@ __global__ void __launch_bounds__(RED_T) k_lrn_update(SolveCtl *ctl, int par, in
   load(u);
   double alpha;
   float a;
-  if (!cg_alpha(ctl, par, &sa, &alpha, &a)) return;
+  if (!cg_alpha(ctl, rz, pq, &sa, &alpha, &a)) return;
   if (blockIdx.x == 0 && threadIdx.x == 0) ctl->last_alpha = alpha;
   for (; u < nu; u += step) {
     float rv[12];

@@ -140,12 +140,17 @@ __device__ __forceinline__ bool finalize_partials(const double *t, double *part,
   if (threadIdx.x == 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k) part[k * gridDim.x + blockIdx.x] = t[k];
-    __threadfence();
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    // releases this block's partials and acquires the others'; the barrier
+    // passes that on to the block's other threads
+    unsigned int n;
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;"
+                 : "=r"(n)
+                 : "l"(__cvta_generic_to_global(ticket))
+                 : "memory");
+    last = n == gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return false;
-  __threadfence();
   // all NV arrays loaded in one pass (the last CTA works alone here, so its
   // load latency is the kernel's tail)
   double a[NV];
@@ -164,14 +169,14 @@ __device__ __forceinline__ bool finalize_partials(const double *t, double *part,
 // warps of an SM doing so each would hold its FP64 pipe for 3 us) and the
 // others wait at the barrier, with their loads in flight.  False when p.q is
 // not a positive finite number; the last block to find so sets the status
-// (not before: a block reads it at its start).  sa: shared.
-__device__ __forceinline__ bool cg_alpha(SolveCtl *ctl, int par, double *sa, double *alpha,
-                                         float *alpha32) {
+// (not before: a block reads it at its start).  rz, pq: ctl->rz[par] and
+// ctl->pq_tot, fetched by the caller together with the status.  sa: shared.
+__device__ __forceinline__ bool cg_alpha(SolveCtl *ctl, double rz, double pq, double *sa,
+                                         double *alpha, float *alpha32) {
   __shared__ int ok;
   __shared__ float sf;
   if (threadIdx.x < 32) {
-    const double pq = ctl->pq_tot;
-    const double a = ctl->rz[par] / pq;
+    const double a = rz / pq;
     if (threadIdx.x == 0) {
       ok = pq > 0.0 && isfinite(pq);
       *sa = a;
@@ -181,7 +186,7 @@ __device__ __forceinline__ bool cg_alpha(SolveCtl *ctl, int par, double *sa, dou
   __syncthreads();
   if (!ok && threadIdx.x == 0 && atomicAdd(&ctl->tick2, 1u) == gridDim.x - 1) {
     ctl->tick2 = 0;
-    ctl->status = isfinite(ctl->pq_tot) ? ST_BREAKDOWN : ST_NAN;
+    ctl->status = isfinite(pq) ? ST_BREAKDOWN : ST_NAN;
   }
   *alpha = *sa;
   *alpha32 = sf;
@@ -353,14 +358,16 @@ __global__ void __launch_bounds__(RED_T, 4) k_cg_update_f64(
     const double *__restrict__ q, double *__restrict__ r, double *__restrict__ x,
     double *__restrict__ z, const double *__restrict__ dinv, double *__restrict__ part_out) {
   __shared__ double sh[2 * RED_T], sa;
-  if (ctl->status != ST_RUNNING) return;
+  const int status = ctl->status;
+  const double pq = ctl->pq_tot, rz = ctl->rz[par];
+  if (status != ST_RUNNING) return;
   double acc[2] = {0.0, 0.0}, alpha;  // r.r, r.z
   float a32;
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   if (PREC == PK_BLOCK3) {
     // 3x3 block-Jacobi: dinv holds 9 values per vertex
-    if (!cg_alpha(ctl, par, &sa, &alpha, &a32)) return;
+    if (!cg_alpha(ctl, rz, pq, &sa, &alpha, &a32)) return;
     for (int64_t v = t0; v * 3 < len; v += step) {
       double rv[3];
 #pragma unroll
@@ -396,7 +403,7 @@ __global__ void __launch_bounds__(RED_T, 4) k_cg_update_f64(
       if (PREC == PK_JACOBI) dv = d2[u];
     };
     load(t0);
-    if (!cg_alpha(ctl, par, &sa, &alpha, &a32)) return;
+    if (!cg_alpha(ctl, rz, pq, &sa, &alpha, &a32)) return;
     auto one = [&](double pi, double qi, double &ri, double &xi, double di) {
       xi = xi + alpha * pi;
       ri = ri - alpha * qi;
@@ -475,7 +482,9 @@ __global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
   // FP32 block Jacobi runs k_cg_update_w, whose inverse blocks are packed
   static_assert(PREC != PK_BLOCK3, "FP32 block Jacobi: use k_cg_update_w");
   __shared__ double sh[2 * RED_T], sa;
-  if (ctl->status != ST_RUNNING) return;
+  const int status = ctl->status;
+  const double pq = ctl->pq_tot, rz = ctl->rz[par];
+  if (status != ST_RUNNING) return;
   DotAcc<float> rr, rzs;
   const int64_t nu = len / 4;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -492,7 +501,7 @@ __global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
   load(u);
   double alpha;
   float a;
-  if (!cg_alpha(ctl, par, &sa, &alpha, &a)) return;
+  if (!cg_alpha(ctl, rz, pq, &sa, &alpha, &a)) return;
   for (; u < nu; u += step) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -595,7 +604,9 @@ static __global__ void __launch_bounds__(K2W_WARPS * 32) k_cg_update_w(
   load(c);
   double alpha = 0.0;
   float a = 0.f;
-  if (ctl->status != ST_RUNNING || !cg_alpha(ctl, par, &sa, &alpha, &a)) {
+  const int status = ctl->status;
+  const double pq = ctl->pq_tot, rz = ctl->rz[par];
+  if (status != ST_RUNNING || !cg_alpha(ctl, rz, pq, &sa, &alpha, &a)) {
     cp_async_wait_all();
     return;
   }
