@@ -295,7 +295,6 @@ constexpr int GB_ST = 2;            // bulk-copy stages of a warp
 constexpr int GB_SEG = 16;          // segments kept in shared memory
 constexpr int GB_K = 4;             // passes a confirmation is spread over
 constexpr int GB_MAXSMEM = 220 * 1024;
-constexpr uint32_t GB_SPINS = 1u << 22;  // barrier polls (seconds)
 enum GridState : int { GS_RUN = 0, GS_CONFIRM = 1, GS_DONE = 2 };
 
 struct GridArgs {
@@ -358,31 +357,6 @@ __global__ void __launch_bounds__(1024) k_grid_plan(BatchArgs a, int32_t *chunk_
     base += sh[31];
     __syncthreads();
   }
-}
-
-// Every CTA of the (co-resident) grid arrives; false when the others did not
-// within the poll limit.
-__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, int *err,
-                                             int *ok_sh) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(bar, 1u);
-    // (relaxed polls: an acquire each would empty the SM's L1 under the CTAs
-    // that still work)
-    bool ok = false;
-    for (uint32_t i = 0; i < GB_SPINS && !ok; ++i) {
-      unsigned int v;
-      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-      ok = (int)(v - target) >= 0;
-      if (!ok) __nanosleep(40);  // leave the counter's cache line to the arrivals
-    }
-    if (!ok) atomicCAS(err, 0, DEV_GRID_TIMEOUT);
-    __threadfence();
-    *ok_sh = ok;
-  }
-  __syncthreads();
-  return *ok_sh != 0;
 }
 
 // Row r (blocks q0 .. e) of q = A p from its staged (or global) values and

@@ -300,6 +300,54 @@ static int horner_grid(GraphH *G, bool half_a, int *out) {
   return SG_OK;
 }
 
+// k_lrn_grid's blocks and warps per block: a block per SM, a warp per slice;
+// *grid = 0 where the slices are more than that (above 136 k rows on 152 SMs):
+// there the separate kernels keep 28 warps per SM as well, work through
+// several slices each, and their launches are a small part.
+static int lrn_grid_config(GraphH *G, bool half_a, int *grid, int *warps) {
+  Ctx *c = G->c;
+  static PerDeviceOnce once;
+  static int fits[SG_MAX_DEVICES] = {};
+  const int dev = (c->device >= 0 && c->device < SG_MAX_DEVICES) ? c->device : 0;
+  SG_TRY(once_per_device(once, dev, [&]() -> int {
+    const size_t sh = lrn_grid_smem<__half>(LG_GRID_WARPS), sf = lrn_grid_smem<float>(LG_GRID_WARPS);
+    SG_CHECK_CUDA(cudaFuncSetAttribute(k_lrn_grid<__half>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+    SG_CHECK_CUDA(cudaFuncSetAttribute(k_lrn_grid<float>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
+    int a = 0, b = 0, coop = 0;
+    SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_lrn_grid<__half>,
+                                                                LG_GRID_WARPS * 32, sh));
+    SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_lrn_grid<float>,
+                                                                LG_GRID_WARPS * 32, sf));
+    SG_CHECK_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+    fits[dev] = a >= 1 && b >= 1 && coop;
+    return SG_OK;
+  }));
+  const int64_t ns = G->fb.sl.nslice, sms = c->num_sms;
+  int64_t w = (ns + sms - 1) / sms;
+  if (w < 1) w = 1;
+  *grid = 0;
+  if (!fits[dev] || w > LG_GRID_WARPS) return SG_OK;
+  *warps = (int)w;
+  *grid = (int)((ns + w - 1) / w);
+  if (*grid < 1) *grid = 1;
+  return SG_OK;
+}
+
+static int lrn_grid_launch(GraphH *G, cudaStream_t st, SolveCtl *ctl, int par, bool half_a,
+                           int grid, int warps, const float *q, float *r, float *z,
+                           double *part) {
+  FoldBufs B = G->fb;
+  B.a = half_a ? (const void *)G->ah : (const void *)G->af;
+  int *err = G->c->d_err;
+  void *args[] = {&ctl, &par, &B, &q, &r, &z, &part, &err};
+  SG_CHECK_CUDA(cudaLaunchCooperativeKernel(
+      half_a ? (const void *)k_lrn_grid<__half> : (const void *)k_lrn_grid<float>, grid,
+      warps * 32, args, half_a ? lrn_grid_smem<__half>(warps) : lrn_grid_smem<float>(warps), st));
+  return SG_OK;
+}
+
 static int horner_launch(GraphH *G, cudaStream_t st, const SolveCtl *ctl, int gate, bool half_a,
                          const FoldBufs &B, int d, const void *src, void *dst,
                          const FinArgs *fa = nullptr) {
@@ -531,6 +579,7 @@ struct LearnedExt {
   mpnn::GraphH *G = nullptr;
   const float *prm = nullptr;
   int exec = SG_MPNN_EXEC_FOLDED;  // folded (FP16 or FP32 edge weights) or layered
+  int grid = 0, warps = 0;         // > 0: the iteration runs k_lrn_grid
 };
 
 static bool folded(const LearnedExt *L) { return L->exec != SG_MPNN_EXEC_LAYERED; }
@@ -539,6 +588,7 @@ static bool folded(const LearnedExt *L) { return L->exec != SG_MPNN_EXEC_LAYERED
 // x = L^-1 r; x += alpha p moves to K3.
 static int learned_k2(Solver *S, cudaStream_t st, int par) {
   LearnedExt *L = (LearnedExt *)S->ext;
+  if (L->grid) return SG_OK;  // part of k_lrn_grid
   const mpnn::FoldBufs &B = L->G->fb;
   if (L->exec == SG_MPNN_EXEC_FOLDED)
     mpnn::k_lrn_update<true><<<S->P2, RED_T, 0, st>>>(S->ctl, par, S->A.n, (const float *)S->q,
@@ -552,6 +602,10 @@ static int learned_k2(Solver *S, cudaStream_t st, int par) {
 
 static int learned_prec(Solver *S, cudaStream_t st, int par) {
   LearnedExt *L = (LearnedExt *)S->ext;
+  if (L->grid)
+    return mpnn::lrn_grid_launch(L->G, st, S->ctl, par, L->exec == SG_MPNN_EXEC_FOLDED, L->grid,
+                                 L->warps, (const float *)S->q, (float *)S->r, (float *)S->z,
+                                 S->part2);
   if (folded(L))
     // the last Horner step leaves r.r | r.z | z.q summed and the iteration
     // decided (status, beta) in ctl for K3
@@ -628,10 +682,11 @@ static int learned_setup(Solver *S) {
     // runs on the steps' grid and leaves that many partials per dot for K3
     int g0 = 0;
     SG_TRY(mpnn::horner_grid(L->G, L->exec == SG_MPNN_EXEC_FOLDED, &g0));
-    const int np = S->P1 > S->P2 ? S->P1 : S->P2;
-    if (g0 > np) {
+    SG_TRY(mpnn::lrn_grid_config(L->G, L->exec == SG_MPNN_EXEC_FOLDED, &L->grid, &L->warps));
+    const int np = S->P1 > S->P2 ? S->P1 : S->P2, g2 = g0 > L->grid ? g0 : L->grid;
+    if (g2 > np) {
       void *p2 = nullptr;
-      SG_CHECK_CUDA(cudaMalloc(&p2, (size_t)g0 * 3 * 8));
+      SG_CHECK_CUDA(cudaMalloc(&p2, (size_t)g2 * 3 * 8));
       S->allocs.push_back(p2);
       S->part2 = (double *)p2;
     }

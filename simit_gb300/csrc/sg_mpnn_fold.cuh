@@ -415,6 +415,24 @@ struct FinArgs {
   int par = 0;
 };
 
+// len entries of a slice in groups of 8, the rest in one group of its exact
+// width (group(integral_constant)): two rounds of gathers for 15 entries.  An
+// entry at a time, 7 of them would wait for one another; a predicated group
+// of 8 takes 106 registers and a third of the warps with them.
+template <typename F> __device__ __forceinline__ void gather_groups(uint32_t len, const F &group) {
+  for (uint32_t e = 0; e + 8 <= len; e += 8) group(std::integral_constant<int, 8>());
+  switch (len % 8) {
+    case 7: group(std::integral_constant<int, 7>()); break;
+    case 6: group(std::integral_constant<int, 6>()); break;
+    case 5: group(std::integral_constant<int, 5>()); break;
+    case 4: group(std::integral_constant<int, 4>()); break;
+    case 3: group(std::integral_constant<int, 3>()); break;
+    case 2: group(std::integral_constant<int, 2>()); break;
+    case 1: group(std::integral_constant<int, 1>()); break;
+    default: break;
+  }
+}
+
 constexpr int HT_WARPS = 4;   // warps per CTA
 constexpr int HT_NST = 2;     // slices in flight per warp
 constexpr int HT_CAPL = 20;   // longest staged slice (entries per lane)
@@ -565,9 +583,7 @@ __global__ void __launch_bounds__(HT_WARPS * 32, 7)
     const AT *ap = staged ? reinterpret_cast<const AT *>(base + (size_t)b * STG + CB) + lane
                           : aw + q0 + lane;
     float m0 = 0.f, m1 = 0.f, m2 = 0.f;
-    // U entries, their gathers in flight together; the rest of a slice goes in
-    // groups of 4, 2 and 1 (an entry at a time, 7 of a 15-entry slice's
-    // gathers waited for one another)
+    // U entries, their gathers in flight together
     uint32_t e = 0;
     auto group = [&](auto width) {
       constexpr int U = decltype(width)::value;
@@ -588,10 +604,7 @@ __global__ void __launch_bounds__(HT_WARPS * 32, 7)
       }
       e += U;
     };
-    while (e + 8 <= len) group(std::integral_constant<int, 8>());
-    if (e + 4 <= len) group(std::integral_constant<int, 4>());
-    if (e + 2 <= len) group(std::integral_constant<int, 2>());
-    if (e < len) group(std::integral_constant<int, 1>());
+    gather_groups(len, group);
     __syncwarp();
     if (v == SL_NONE) continue;
     if (first) {
@@ -767,6 +780,187 @@ __global__ void __launch_bounds__(RED_T) k_lrn_update(SolveCtl *ctl, int par, in
       st3<CV>(xin, (size_t)v, L[0] * R[0], L[1] * R[0] + L[2] * R[1],
               L[3] * R[0] + L[4] * R[1] + L[5] * R[2]);
     }
+}
+
+// The learned iteration's K2, its six Horner steps and the end of the
+// application in one cooperative launch, for graphs whose slices all have a
+// warp at once (one block per SM, at most LG_GRID_WARPS warps each).  A warp
+// keeps one slice: its indices and weights are copied to shared memory once
+// for all six steps, and a lane keeps its row's r, q and x in registers.
+// Between the steps the grid meets at a barrier (bounded: on a timeout the
+// blocks record it, stop the solve and return).  The vectors that other SMs
+// write are read with ordinary cached loads: the barrier's fences order them.
+// Same arithmetic as k_lrn_update and k_horner, same bits.
+// Bound by the latency of gathers (two or three rounds a step) and barriers.
+// 48^3 (117,649 rows, 25 warps per SM): 39.7 us instead of 54.5 for the seven
+// kernels (4.9 K2, 6.7 a step at 1.3 us of traffic, most of it launch,
+// fetching the slice and draining, 16.1 the last); solves of 4,913, 50,653
+// and 132,651 rows 17.5 -> 13.6, 45.3 -> 33.3 and 85.0 -> 63.8 ms.
+constexpr int LG_GRID_WARPS = 28;  // 72 registers per thread
+
+template <typename AT>
+__host__ __device__ constexpr size_t lrn_grid_smem(int warps) {
+  return SUM_OFF + (size_t)warps * ht_stage_bytes<AT>();
+}
+
+template <bool CV>
+__device__ __forceinline__ void ld3_shared(const void *p, size_t v, float &a, float &b, float &c) {
+  if (CV) {
+    cv_decode(__ldca(reinterpret_cast<const uint2 *>(p) + v), a, b, c);
+  } else {
+    const float4 t = __ldca(reinterpret_cast<const float4 *>(p) + v);
+    a = t.x;
+    b = t.y;
+    c = t.z;
+  }
+}
+
+template <typename AT>
+__global__ void __launch_bounds__(LG_GRID_WARPS * 32, 1)
+    k_lrn_grid(SolveCtl *ctl, int par, FoldBufs B, const float *q, float *r, float *z,
+               double *part, int *err) {
+  constexpr bool CV = sizeof(AT) == 2;
+  constexpr size_t CB = (size_t)HT_CAPL * SL_W * 4;
+  static_assert(ht_stage_bytes<AT>() >= 3 * 32 * 8 && LG_GRID_WARPS * 8 <= SUM_OFF, "sums");
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ float G[7 * 9];
+  __shared__ double sa;
+  __shared__ int ok_sh;
+  const int status = ctl->status;
+  const double pq = ctl->pq_tot, rz0 = ctl->rz[par];
+  const bool fb = ctl->fallback;
+  if (status != ST_RUNNING) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t s = (int64_t)blockIdx.x * (blockDim.x / 32) + warp;
+  const bool have = s < B.sl.nslice;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(sm) + warp;
+  unsigned char *stage = sm + SUM_OFF + (size_t)warp * ht_stage_bytes<AT>();
+  const uint32_t p0 = have ? __ldg(B.sl.ptr + s) : 0u, p1 = have ? __ldg(B.sl.ptr + s + 1) : 0u;
+  uint32_t len = (p1 - p0) / SL_W;
+  const bool staged = len > 0 && len <= (uint32_t)HT_CAPL;
+  if (lane == 0) {
+    mbar_init(bar, 1);
+    mbar_fence_init();
+    if (staged && !fb) {
+      fence_proxy_async_smem();
+      const uint32_t cb = len * SL_W * 4, wb = len * SL_W * (uint32_t)sizeof(AT);
+      mbar_arrive_expect_tx(bar, cb + wb);
+      bulk_g2s(stage, B.sl.col + p0, cb, bar);
+      bulk_g2s(stage + CB, (const AT *)B.a + p0, wb, bar);
+    }
+  }
+  const uint32_t v = have ? __ldg(B.sl.row + s * SL_W + lane) : SL_NONE;
+  const bool row = v != SL_NONE;
+  const void *l6 = CV ? (const void *)B.l6b : (const void *)B.l6;
+  float R[3] = {0.f, 0.f, 0.f}, Q[3] = {0.f, 0.f, 0.f}, L[6] = {};
+  if (row) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      Q[k] = q[(size_t)v * 3 + k];
+      R[k] = r[(size_t)v * 3 + k];
+    }
+    ld_linv<CV>(l6, v, L);
+  }
+  for (int i = threadIdx.x; i < 7 * 9; i += blockDim.x) G[i] = B.g[i];
+  double alpha;
+  float a;
+  __syncwarp();  // the barrier is initialised
+  const bool good = cg_alpha(ctl, rz0, pq, &sa, &alpha, &a);  // (a block barrier: G is there)
+  // the slice has arrived (it is waited for before anything can return)
+  if (staged && !fb && !__all_sync(0xffffffffu, mbar_wait(bar, 0))) {
+    len = 0;  // the stage holds no indices to follow
+    if (lane == 0) {
+      atomicCAS(err, 0, 6 /* DEV_TMA_TIMEOUT */);
+      if (!mbar_wait(bar, 0)) atomicExch(err, 8 /* DEV_TMA_UNDRAINED */);
+    }
+  }
+  if (!good) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->last_alpha = alpha;
+  // K2: r -= alpha q; x = L^-1 r, rounded as it is stored
+  float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+  if (row) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      R[k] = R[k] - a * Q[k];
+      r[(size_t)v * 3 + k] = R[k];
+    }
+    x0 = L[0] * R[0];
+    x1 = L[1] * R[0] + L[2] * R[1];
+    x2 = L[3] * R[0] + L[4] * R[1] + L[5] * R[2];
+    st3<CV>(B.xin, v, x0, x1, x2);
+    if (CV) cv_decode(cv_encode(x0, x1, x2), x0, x1, x2);
+  }
+  float w0 = x0, w1 = x1, w2 = x2;  // fallback: z = L^-T x
+  if (!fb) {
+    const uint32_t *cp = staged ? reinterpret_cast<const uint32_t *>(stage) + lane
+                                : B.sl.col + p0 + lane;
+    const AT *ap = staged ? reinterpret_cast<const AT *>(stage + CB) + lane
+                          : (const AT *)B.a + p0 + lane;
+    unsigned int arrived = 0;
+    for (int d = 5; d >= 0; --d) {
+      arrived += gridDim.x;
+      if (!grid_barrier(&ctl->gbar, arrived, err, &ok_sh)) {
+        ctl->status = ST_NAN;
+        return;
+      }
+      const void *src = d == 5 ? B.xin : d & 1 ? B.w[0] : B.w[1];
+      float m0 = 0.f, m1 = 0.f, m2 = 0.f;
+      uint32_t e = 0;
+      auto group = [&](auto width) {
+        constexpr int U = decltype(width)::value;
+        uint32_t u[U];
+        float wq[U], g0[U], g1[U], g2[U];
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          u[j] = cp[(e + j) * SL_W];
+          wq[j] = tofloat(ap[(e + j) * SL_W]);
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j) ld3_shared<CV>(src, u[j], g0[j], g1[j], g2[j]);
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          m0 += wq[j] * g0[j];
+          m1 += wq[j] * g1[j];
+          m2 += wq[j] * g2[j];
+        }
+        e += U;
+      };
+      gather_groups(len, group);
+      const float *Gd = G + d * 9, *G6 = G + 6 * 9;
+      if (d == 5) {
+        const float t0 = m0, t1 = m1, t2 = m2;
+        m0 = G6[0] * t0 + G6[1] * t1 + G6[2] * t2;
+        m1 = G6[3] * t0 + G6[4] * t1 + G6[5] * t2;
+        m2 = G6[6] * t0 + G6[7] * t1 + G6[8] * t2;
+      }
+      w0 = m0 + Gd[0] * x0 + Gd[1] * x1 + Gd[2] * x2;
+      w1 = m1 + Gd[3] * x0 + Gd[4] * x1 + Gd[5] * x2;
+      w2 = m2 + Gd[6] * x0 + Gd[7] * x1 + Gd[8] * x2;
+      if (d > 0 && row) st3<CV>(d & 1 ? B.w[1] : B.w[0], v, w0, w1, w2);
+    }
+    if (CV) cv_decode(cv_encode(w0, w1, w2), w0, w1, w2);  // as a stored w_0 would be
+  }
+  DotAcc<float> rr, rz, zq;
+  if (row) {
+    ld_linv<CV>(l6, v, L);
+    const float Z[3] = {L[0] * w0 + L[1] * w1 + L[3] * w2, L[2] * w1 + L[4] * w2, L[5] * w2};
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      z[(size_t)v * 3 + k] = Z[k];
+      rr.add(R[k], R[k]);
+      rz.add(R[k], Z[k]);
+      zq.add(Z[k], Q[k]);
+    }
+  }
+  const double t3[3] = {rr.value(), rz.value(), zq.value()};
+  double t[3], tot[3];
+  DecideIn in = decide_in(ctl, par);
+  in.alpha = alpha;
+  block_sums<3>(t3, t, sum_buf(sm));
+  if (finalize_partials<3>(t, part, &ctl->tick2, tot, sum_buf(sm)) && threadIdx.x == 0) {
+    ctl->gbar = 0;
+    cg_decide(ctl, par, in, tot[0], tot[1], tot[2]);
+  }
 }
 
 }  // namespace mpnn

@@ -25,6 +25,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sg_internal.cuh"
 #include "sg_spmv.cuh"
 #include "sg_tma.cuh"
 
@@ -60,6 +61,7 @@ struct SolveCtl {
   double beta;
   float alpha32, beta32;  // last_alpha and beta rounded, for the FP32 kernels
   unsigned int tick1, tick2;
+  unsigned int gbar;  // arrivals at the grid barriers of one k_lrn_grid launch
 };
 
 constexpr int RED_T = 256;
@@ -80,8 +82,9 @@ __device__ __forceinline__ double block_sum(double v, double *sh) {
   return sh[32];
 }
 
-// Block-wide FP64 sums of NV values per thread (NV <= 3, at most 8 full
-// warps), result in every lane of warp 0.  The additions are those of
+// Block-wide FP64 sums of NV values per thread (NV <= 3, full warps; more
+// than 8 of them take a warp per value for the last level), result in every
+// lane of warp 0.  The additions are those of
 // block_sum, pair by pair, so the sums have the same bits; but between the
 // levels the operands go through shared memory (buf: NV * blockDim.x values)
 // and fill whole warps, because a warp instruction costs the same with one
@@ -103,8 +106,26 @@ __device__ __forceinline__ void block_sums(const double *v, double *out, double 
     }
     __syncthreads();
   }
+  const int nw = T / 32;
+  if (nw > 8) {
+    double s = 0.0;
+    if (t < NV * 32 && t % 32 < nw) {
+      const double *e = buf + (t / 32 * nw + t % 32) * 32;
+      s = (e[0] + e[2]) + (e[1] + e[3]);
+    }
+    if (t < NV * 32) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    }
+    __syncthreads();  // the values of the last level have been read
+    if (t < NV * 32 && t % 32 == 0) buf[t / 32] = s;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NV; ++j) out[j] = buf[j];
+    return;
+  }
   if (t < 32) {
-    const int nw = T / 32, k = t / 8, w = t % 8;
+    const int k = t / 8, w = t % 8;
     double s = 0.0;
     if (k < NV && w < nw) {
       const double *e = buf + (k * nw + w) * 32;
@@ -125,6 +146,33 @@ __device__ __forceinline__ double *sum_buf(unsigned char *sm) {
 }
 
 template <typename T> __device__ __forceinline__ bool finite_(T v) { return isfinite(v); }
+
+constexpr uint32_t GRID_SPINS = 1u << 22;  // barrier polls (seconds)
+
+// Every CTA of the (co-resident) grid arrives; false when the others did not
+// within the poll limit.
+__device__ __forceinline__ bool grid_barrier(unsigned int *bar, unsigned int target, int *err,
+                                             int *ok_sh) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    // (relaxed polls: an acquire each would empty the SM's L1 under the CTAs
+    // that still work)
+    bool ok = false;
+    for (uint32_t i = 0; i < GRID_SPINS && !ok; ++i) {
+      unsigned int v;
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+      ok = (int)(v - target) >= 0;
+      if (!ok) __nanosleep(40);  // leave the counter's cache line to the arrivals
+    }
+    if (!ok) atomicCAS(err, 0, DEV_GRID_TIMEOUT);
+    __threadfence();
+    *ok_sh = ok;
+  }
+  __syncthreads();
+  return *ok_sh != 0;
+}
 
 // Last-CTA finalisation of per-CTA sums (t: this block's NV sums, in thread
 // 0; part: NV arrays of gridDim.x values): every CTA stores its partials and

@@ -253,3 +253,47 @@ def test_folded_forward_long_rows(ctx, mode):
     err = np.linalg.norm(zt.cpu().numpy() - z_ref)
     assert err <= 1e-5 * np.linalg.norm(z_ref), err
     g.close()
+
+
+@pytest.mark.parametrize("mode", [_lib.MPNN_EXEC_FOLDED, _lib.MPNN_EXEC_FOLDED_F32])
+@pytest.mark.parametrize("ncell", [1, 4, 16, 36, 50, 51])
+def test_learned_solve_at_grid_edges(ctx, ncell, mode):
+    """Learned solves around the sizes where the iteration's one launch
+    changes shape: fewer slices of 32 rows than SMs, two warps per SM, more
+    than 8, the 28 it can hold, and one more than that (separate kernels).
+    Each reaches the verified tolerance without falling back, twice with the
+    same bits; the FP32 evaluation, the layered one's operator, in its number
+    of iterations at the small sizes."""
+    from simit_gb300 import learned
+    from simit_gb300.runtime import Solver, solve_opts
+    w = learned.load_weights("sym")
+    host = problems.reorder_hetero(problems.hetero_mesh(ncell, seed=5))
+    prob = problems.HeteroElasticity(ctx, host, dtype=torch.float32,
+                                     precond=_lib.PRECOND_BLOCK_JACOBI)
+    m = prob.mesh
+    wt = torch.tensor(np.asarray(w, np.float32), device=ctx.device)
+    b = torch.randn(m.n * 3, dtype=torch.float64, generator=torch.Generator().manual_seed(7))
+    b = b.to(ctx.device)
+    torch.cuda.synchronize()
+
+    def solve(exec_mode):
+        S = Solver(ctx, m.n, 3, m.pattern.rowptr, m.pattern.colidx, prob.A, m.nnzb,
+                   solve_opts(precision=_lib.SOLVE_MIXED, precond=_lib.PRECOND_LEARNED, tol=1e-8,
+                              maxiters=5000, learned_params=wt,
+                              learned_form=learned.FORMS["sym"], learned_exec=exec_mode),
+                   learned_params_keep=wt)
+        out = []
+        for _ in range(2):
+            x = torch.zeros_like(b)
+            torch.cuda.synchronize()
+            r = S.solve(b, x)
+            assert r.status == 1 and r.fallbacks == 0
+            assert r.true_normr2 <= 1e-16 * r.bnorm2
+            out.append((x, r.iters))
+        S.close()
+        assert torch.equal(out[0][0], out[1][0])
+        return out[0][1]
+    it = solve(mode)
+    if ncell <= 16 and mode == _lib.MPNN_EXEC_FOLDED_F32:
+        assert abs(it - solve(_lib.MPNN_EXEC_LAYERED)) <= max(2, 0.03 * it)
+    prob.close()
