@@ -418,7 +418,7 @@ def run_cloth(args, rank=0, world=1, local=0):
 
 def run_solve_only(args):
     """Profiling driver: the --size heterogeneous-elasticity step as the
-    headline runs it (FP32 assembly with the element-blocks plan + flexible
+    headline runs it (FP32 assembly by row tiles + flexible
     mixed PCG with the learned preconditioner; --block-jacobi for mixed
     block-Jacobi PCG) with the solver capped at --iters iterations; the
     second step is event-timed."""
@@ -496,8 +496,8 @@ def run_learned_solve(args):
 
 def run_assembly_only(args):
     """Profiling driver: the --size heterogeneous-elasticity step's assembly
-    (stiffness map in place + force map, FP32) with the element-blocks +
-    gather plan, the coloured plan and the row owners, each event-timed over
+    (stiffness map in place + force map, FP32) with the row tiles over the
+    gather plan's element lists, the coloured plan and the row owners, each event-timed over
     --reps calls; also each plan's set-up time."""
     import torch
     from simit_gb300 import _lib, problems
@@ -1017,10 +1017,9 @@ def run_ours(args, rank, world, local):
     value = dofs * world / (ms / 1e3)
     relres = max((r.true_normr2 / r.bnorm2) ** 0.5 for r in results)
     iters = results[-1].iters
-    # kernels per step: stiffness + force assembly (the gather plan: element
-    # blocks, slot gather; element vectors, vertex gather), the solver's
-    # refresh and its own count (graph kernel nodes included)
-    launches = sum(int(r.kernels) + 4 + 6 for r in results)
+    # kernels per step: stiffness + force assembly (the row tiles: one each),
+    # the solver's refresh and its own count (graph kernel nodes included)
+    launches = sum(int(r.kernels) + 2 + 6 for r in results)
 
     # --- end to end through host buffers (pinned) -------------------------
     n3 = prob.dofs
@@ -1086,8 +1085,8 @@ def run_ours(args, rank, world, local):
     # --- the step's assembly alone (stiffness map in place + force map) ----
     # algorithmic bytes: element ids and parameters (B 9, W, mu, lam) once,
     # vertex positions once, the matrix values and the force written once;
-    # the gather plan also writes and reads its element blocks and vectors
-    # and reads the inverse slot map (implementation bytes)
+    # the row tiles also read the plan's incidence and slot maps
+    # (implementation bytes)
     nE = m.nE
     for _ in range(2):
         prob.assemble_in_place()
@@ -1100,15 +1099,14 @@ def run_ours(args, rank, world, local):
     a1.synchronize()
     asm_ms = a0.elapsed_time(a1) / 3
     asm_bytes = nE * (4 * 4 + 12 * 4) + m.n * 3 * 4 + m.nnzb * 36 + m.n * 3 * 4
-    impl_bytes = asm_bytes + 2 * nE * 16 * 36 + nE * 16 * 4 + (m.nnzb + 1) * 4 + 2 * nE * 4 * 12
+    impl_bytes = asm_bytes + nE * 16 * 4 + 2 * nE * 4 * 4 + 2 * (m.n + 1) * 4
     assembly = {"ms": asm_ms, "elements_per_s": nE / (asm_ms / 1e3),
                 "algorithmic_bytes": asm_bytes, "GBps": asm_bytes / (asm_ms / 1e3) / 1e9,
                 "implementation_bytes": impl_bytes,
                 "implementation_GBps": impl_bytes / (asm_ms / 1e3) / 1e9,
                 "plan": m.plan, "tile": int(m.s.asm_tile) or 256,
-                "kernels": {"gather": "element-blocks plan: k_elem_blocks<LinTetElem> + "
-                                      "k_slot_gather (stiffness), k_elem_blocks<TetForceElem> "
-                                      "+ k_vert_gather (force)",
+                "kernels": {"gather": "row tiles: k_tile<LinTetTile> (stiffness), "
+                                      "k_tile<TetForceTile> (force)",
                             "colored": "coloured plan: k_colored<LinTetElem>, "
                                        "k_colored<TetForceElem> per colour",
                             None: "row owners: k_rows<LinTetElem>, k_rows<TetForceElem>"}[m.plan]}
@@ -1209,7 +1207,7 @@ def run_ours(args, rank, world, local):
         "data": "synthetic (seeded Philox mesh, parameters and displacements)",
         "config": {"workload": workload_name(args.size, not args.no_reorder), "dofs": dofs,
                    "nnzb": m.nnzb,
-                   "method": "FP32 assembly (element-blocks plan) + learned-preconditioned "
+                   "method": "FP32 assembly (row tiles) + learned-preconditioned "
                              "flexible mixed-precision PCG (symmetric form of the 3-layer "
                              "hidden-64 message-passing network, evaluated as its degree-6 "
                              "matrix polynomial; FP32 matrix/vectors, FP64 dots, FP64 reliable "

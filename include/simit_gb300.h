@@ -167,11 +167,11 @@ typedef struct sg_mesh {
   int32_t ncolors;
   const uint32_t *slot_src_ptr; /* device [nnzb+1] (sg_slot_sources) */
   const uint32_t *slot_src;     /* device [nE*card*card] */
-  int32_t asm_tile;             /* read by no kernel (it was the element-blocks
-                                   plan's tile); kept for the layout */
+  int32_t asm_tile;             /* read by no kernel (it was an element tile of
+                                   the gather plan); kept for the layout */
 } sg_mesh;
 
-/* The inverse slot map for the element-blocks plan: for slot q, the element
+/* The inverse slot map for the gather plan: for slot q, the element
  * blocks (e*card + i)*card + j with slots[...] == q, ascending, at
  * slot_src[slot_src_ptr[q] .. slot_src_ptr[q+1]).  Needs m->slots (and
  * nnzb).  Replaces the per-element `loc` searches of the reference's map

@@ -1,6 +1,6 @@
 // Assembly plans: the element colouring and the inverse slot map.
 //
-// Inverse slot map (the element-blocks + slot-gather plan): for every
+// Inverse slot map (the gather plan): for every
 // matrix slot the list of element blocks (e*card + i)*card + j whose slot it
 // is, ascending (ascending element, then i, j), as CSR (slot_src_ptr,
 // slot_src).  Every incidence of a vertex sends card blocks to slots of its

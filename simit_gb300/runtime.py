@@ -472,7 +472,7 @@ class Mesh:
     def tune_assembly(self, assemble, plans=("gather", "colored", None), tiles=(128, 256, 512),
                       reps=3):
         """Assembly autotuner: times `assemble()` (the caller's assembly
-        through this mesh) under every plan and, for the element-blocks plan,
+        through this mesh) under every plan and, for the gather plan,
         every element tile; keeps the fastest (plans are built as needed;
         the chosen one stays set).  The choice is cached per (n, nE, card,
         plan set).  Returns {"plan", "tile", "ms", "default_ms", "times"}."""
