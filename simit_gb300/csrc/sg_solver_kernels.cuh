@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(RED_T, 3) k_cg_update_v4(
 // thousand vertices, by latency and the FP64 pipe of the SMs that hold the
 // (few) blocks: 8,257 vertices 11.5 us with alpha divided by every warp,
 // conversions on the FP64 pipe, three sums one after the other and 8 chunks
-// to a block, 7.8 so.
+// to a block, 7.4 so.
 constexpr int K2W_WARPS = 8;  // at most; a block has blockDim.x / 32
 struct K2WarpSmem {
   float4 q[96], r[96], d[192];
