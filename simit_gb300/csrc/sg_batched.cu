@@ -267,7 +267,10 @@ __global__ void k_batched_pcg(BatchArgs a) {
 // segment's dot products go to part[k][b + s] (b + s grows by at least one
 // from segment to segment, and a system's segments are consecutive); after
 // the barrier every CTA that holds rows of a system sums them in the same
-// order and takes the same decision.  A system whose iterated residual passes
+// order and takes the same decision.  k: a DotSlot; no slot is read and written
+// between two barriers, or a CTA that is ahead would overwrite what one behind
+// has still to read (b.b shared the slot of r.r, which the first pass writes
+// right after b.b's sum).  A system whose iterated residual passes
 // spends the first phase of the next GB_K passes on its true residual, a part
 // in each (CONFIRM): FP64 work that only its own CTAs share would otherwise
 // make one pass four times as long for every system.
@@ -296,18 +299,20 @@ constexpr int GB_SEG = 16;          // segments kept in shared memory
 constexpr int GB_K = 4;             // passes a confirmation is spread over
 constexpr int GB_MAXSMEM = 220 * 1024;
 enum GridState : int { GS_RUN = 0, GS_CONFIRM = 1, GS_DONE = 2 };
+// partial sums: b.b (first pass), p.q or the true residual's r.r, r.r, r.z
+enum DotSlot : int { DS_BB = 0, DS_PQ = 1, DS_RR = 2, DS_RZ = 3, DS_N = 4 };
 
 struct GridArgs {
   BatchArgs b;
   int64_t nnzb;
   float4 *p;                 // [n] directions
   const int32_t *chunk_ptr;  // [nsys+1] chunks before each system
-  double *part;              // [3][nb + nsys]
+  double *part;              // [DS_N][nb + nsys]
   unsigned int *bar;         // barrier arrivals (zeroed before launch)
   int *ndone;                // systems finished (zeroed before launch)
   int *err;
   struct Seg *segs;          // [nb + nsys] segments of CTAs that meet more than GB_SEG
-  double *wps;               // [nb + nsys][3][GB_W]
+  double *wps;               // [nb + nsys][DS_N][GB_W]
   int capb;                  // blocks per warp stage
 };
 
@@ -446,8 +451,8 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
   const int nb = gridDim.x, b = blockIdx.x;
   const size_t vbytes = tma_vbytes<float>(g.capb), stage = vbytes + tma_cbytes(g.capb);
   Seg *seg = reinterpret_cast<Seg *>(gsm);
-  double *wp = reinterpret_cast<double *>(seg + GB_SEG);  // [segment][3][GB_W]
-  unsigned char *raw = reinterpret_cast<unsigned char *>(wp + GB_SEG * 3 * GB_W);
+  double *wp = reinterpret_cast<double *>(seg + GB_SEG);  // [segment][DS_N][GB_W]
+  unsigned char *raw = reinterpret_cast<unsigned char *>(wp + GB_SEG * DS_N * GB_W);
   uint64_t *bar = reinterpret_cast<uint64_t *>(raw) + warp * GB_ST;
   unsigned char *base = raw + GB_W * GB_ST * 8 + (size_t)warp * GB_ST * stage;
   if (lane == 0) {
@@ -470,7 +475,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
       for (int pass = 0; pass < 2; ++pass) {
         if (pass && ns_ > GB_SEG) {
           seg = g.segs + b + lo;
-          wp = g.wps + ((size_t)b + lo) * 3 * GB_W;
+          wp = g.wps + ((size_t)b + lo) * DS_N * GB_W;
         }
         ns_ = 0;
         for (int s0 = lo; s0 < a.nsys && g.chunk_ptr[s0] < c1; s0 += 32) {
@@ -506,7 +511,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
   const int ns = ns_sh;
   if (ns > GB_SEG) {
     seg = g.segs + b + lo_sh;
-    wp = g.wps + ((size_t)b + lo_sh) * 3 * GB_W;
+    wp = g.wps + ((size_t)b + lo_sh) * DS_N * GB_W;
   }
   const int64_t np = (int64_t)nb + a.nsys;
   unsigned int arrived = 0;
@@ -517,7 +522,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
       const int j = t / (ke - kb), k = kb + t % (ke - kb);
       if (seg[j].st == GS_DONE) continue;
       double v = 0;
-      for (int w = 0; w < GB_W; ++w) v += wp[(j * 3 + k) * GB_W + w];
+      for (int w = 0; w < GB_W; ++w) v += wp[(j * DS_N + k) * GB_W + w];
       g.part[k * np + b + seg[j].sys] = v;
     }
   };
@@ -560,7 +565,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
     double bb = 0;
     for (int i = q.ra * 3 + tid; i < q.rb * 3; i += GB_T) bb += (double)a.b[i] * a.b[i];
     bb = warp_sum(bb);
-    if (lane == 0) wp[(j * 3 + 1) * GB_W + warp] = bb;
+    if (lane == 0) wp[(j * DS_N + DS_BB) * GB_W + warp] = bb;
   }
 
   const int gl = lane & (G - 1);
@@ -679,7 +684,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
         const int j = cur.j;
         if (!more || ahead.j != j) {  // the segment's last tile of this warp
           const double t = warp_sum(run ? acc.value() : racc);
-          if (lane == 0) wp[(j * 3) * GB_W + warp] = t;
+          if (lane == 0) wp[(j * DS_N + DS_PQ) * GB_W + warp] = t;
           acc = DotAcc<float>();
           racc = 0;
         }
@@ -692,16 +697,17 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
       for (int j = 0; j < ns; ++j) {
         const int skip = seg[j].st == GS_CONFIRM && seg[j].sl < GB_K ? seg[j].sl : 0;
         if (lane == 0 && seg[j].ra + skip * GB_C + warp * GB_R >= seg[j].rb)
-          wp[(j * 3) * GB_W + warp] = 0.0;
+          wp[(j * DS_N + DS_PQ) * GB_W + warp] = 0.0;
       }
     }
-    publish(0, pass == 0 ? 2 : 1);
+    publish(pass == 0 ? DS_BB : DS_PQ, DS_PQ + 1);
     if (!sync_grid()) return;
     // phase 2: alpha; r and z of the running systems, z of the others that
     // have not converged
     for (int j = warp; j < ns; j += GB_W) {
       if (seg[j].st == GS_DONE) continue;
-      const double t = total(seg[j].sys, 0), bb = pass == 0 ? total(seg[j].sys, 1) : 0.0;
+      const double t = total(seg[j].sys, DS_PQ);
+      const double bb = pass == 0 ? total(seg[j].sys, DS_BB) : 0.0;
       if (lane == 0) {
         Seg &q = seg[j];
         if (pass == 0) {
@@ -763,16 +769,16 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
       }
       const double s_rr = warp_sum(rra.value()), s_rz = warp_sum(t.value());
       if (lane == 0) {
-        wp[(j * 3 + 1) * GB_W + warp] = s_rr;
-        wp[(j * 3 + 2) * GB_W + warp] = s_rz;
+        wp[(j * DS_N + DS_RR) * GB_W + warp] = s_rr;
+        wp[(j * DS_N + DS_RZ) * GB_W + warp] = s_rz;
       }
     }
-    publish(1, 3);
+    publish(DS_RR, DS_RZ + 1);
     if (!sync_grid()) return;
     // phase 3: the decision; x and p
     for (int j = warp; j < ns; j += GB_W) {
       if (seg[j].st == GS_DONE || (seg[j].st == GS_CONFIRM && seg[j].sl < GB_K)) continue;
-      const double rr = total(seg[j].sys, 1), rz = total(seg[j].sys, 2);
+      const double rr = total(seg[j].sys, DS_RR), rz = total(seg[j].sys, DS_RZ);
       if (lane == 0) {
         Seg &q = seg[j];
         bool turn = true;  // a new direction
@@ -872,7 +878,7 @@ int grid_config(Ctx *c, int32_t n, int64_t nnzb, int nsys, int *grid, int *capb,
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GB_MAXSMEM));
     return SG_OK;
   }));
-  *smem = GB_SEG * (sizeof(Seg) + 3 * GB_W * 8) + GB_W * GB_ST * 8 +
+  *smem = GB_SEG * (sizeof(Seg) + DS_N * GB_W * 8) + GB_W * GB_ST * 8 +
           (size_t)GB_W * GB_ST * (tma_vbytes<float>(cap) + tma_cbytes(cap));
   int per_sm = 0;
   SG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, GB_T, *smem));
@@ -956,7 +962,7 @@ extern "C" int sg_batched_pcg(sg_ctx *h, int32_t nsys, const int32_t *sys_ptr,
   const size_t nid = (size_t)c->num_sms * GB_MAXCTAS + nsys;  // grid-wide: segment numbers
   SG_TRY(s.reserve(Scratch::bytes_for(len, 4) * 3 + Scratch::bytes_for(A->n, sizeof(float4)) +
                    Scratch::bytes_for((size_t)A->n * 9, 4) +
-                   Scratch::bytes_for(3 * nid, 8) + Scratch::bytes_for(3 * GB_W * nid, 8) +
+                   Scratch::bytes_for(DS_N * nid, 8) + Scratch::bytes_for(DS_N * GB_W * nid, 8) +
                    Scratch::bytes_for(nid, sizeof(Seg)) + Scratch::bytes_for((size_t)nsys + 1, 4) +
                    4096));
   GridScratch w;
@@ -981,8 +987,8 @@ extern "C" int sg_batched_pcg(sg_ctx *h, int32_t nsys, const int32_t *sys_ptr,
   a.relres = relres;
   a.tol = tol;
   a.maxiters = maxiters;
-  w.part = s.alloc<double>(3 * nid);
-  w.wps = s.alloc<double>(3 * GB_W * nid);
+  w.part = s.alloc<double>(DS_N * nid);
+  w.wps = s.alloc<double>(DS_N * GB_W * nid);
   w.segs = s.alloc<Seg>(nid);
   w.chunk_ptr = s.alloc<int32_t>((size_t)nsys + 1);
   w.bar = s.alloc<unsigned int>(2);

@@ -143,3 +143,20 @@ def test_grid_wide_systems_without_rows(ctx):
         ctx.sync()
         assert np.array_equal(cb.status.cpu().numpy(), st)
         assert np.all(cb.iters.cpu().numpy()[it == 0] == 0)
+
+
+def test_grid_wide_systems_over_many_ctas_repeat(ctx):
+    """Systems whose rows belong to many CTAs, with small ones between them so
+    that the CTAs of one system have unequal work: every run takes the same
+    decisions on every system (equal bits, iterations and statuses)."""
+    host = problems.cloth_batch(nsheets=40, lo=8, hi=120, seed=17)
+    cb = problems.ClothBatch(ctx, host, config=3)
+    for cfg in GRID_CONFIGS:
+        first = None
+        for _ in range(12):
+            cb.step(config=cfg)
+            ctx.sync()
+            got = [t.clone() for t in (cb.vout, cb.iters, cb.status, cb.relres)]
+            assert bool((cb.status == 1).all()) and float(cb.relres.max()) <= 1e-6
+            first = first or got
+            assert all(torch.equal(a, b) for a, b in zip(first, got))
