@@ -557,7 +557,10 @@ int sg_residual(sg_ctx *ctx, const sg_matrix *A, const double *x, const double *
  * (SG_STATUS_*), relres per system (device).  config selects the schedule,
  * threads per CTA and lanes per row (0 .. sg_batched_configs()-1: 0..5 one CTA
  * per system, 6 and 7 the whole grid on all; the autotuner in the host runtime
- * picks one).  Asynchronous; capturable after a first call has
+ * picks one).  No configuration needs alignment beyond the element types';
+ * 6 and 7 stage A in shared memory where its values and columns start on
+ * 16-byte boundaries and read it from global memory otherwise.
+ * Asynchronous; capturable after a first call has
  * sized the context scratch.  Replaces running one Simit program per mesh
  * (no batched counterpart in the reference).
  * ------------------------------------------------------------------- */

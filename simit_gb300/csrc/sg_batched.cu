@@ -313,7 +313,7 @@ struct GridArgs {
   int *err;
   struct Seg *segs;          // [nb + nsys] segments of CTAs that meet more than GB_SEG
   double *wps;               // [nb + nsys][DS_N][GB_W]
-  int capb;                  // blocks per warp stage
+  int capb;                  // blocks per warp stage; -1: every tile is read from global memory
 };
 
 struct Seg {
@@ -449,7 +449,8 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
   const BatchArgs &a = g.b;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = gridDim.x, b = blockIdx.x;
-  const size_t vbytes = tma_vbytes<float>(g.capb), stage = vbytes + tma_cbytes(g.capb);
+  const int cap = max(g.capb, 0);
+  const size_t vbytes = tma_vbytes<float>(cap), stage = vbytes + tma_cbytes(cap);
   Seg *seg = reinterpret_cast<Seg *>(gsm);
   double *wp = reinterpret_cast<double *>(seg + GB_SEG);  // [segment][DS_N][GB_W]
   unsigned char *raw = reinterpret_cast<unsigned char *>(wp + GB_SEG * DS_N * GB_W);
@@ -609,7 +610,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
         const size_t ce = min(((size_t)b1 * 4 + 15) & ~size_t(15), cend);
         unsigned char *vb = base + (size_t)st * stage;
         fence_proxy_async_smem();
-        if (b1 - b0 > (uint32_t)g.capb) {  // larger than the stage: read from global
+        if ((int)(b1 - b0) > g.capb) {  // larger than the stage: read from global
           mbar_arrive_expect_tx(&bar[st], 0);
           return;
         }
@@ -650,7 +651,7 @@ __global__ void __launch_bounds__(GB_T, 2) k_batched_grid(GridArgs g) {
         ++nth;
         const uint32_t b0 = __shfl_sync(0xffffffffu, cur.rp, 0);
         const uint32_t b1 = __shfl_sync(0xffffffffu, cur.rp, GB_R);
-        const bool staged = b1 - b0 <= (uint32_t)g.capb;
+        const bool staged = (int)(b1 - b0) <= g.capb;
         const size_t vs = staged ? ((size_t)b0 * 36) & ~size_t(15) : 0;
         const size_t cs = staged ? ((size_t)b0 * 4) & ~size_t(15) : 0;
         float *vb = reinterpret_cast<float *>(base + (size_t)st * stage);
@@ -864,13 +865,16 @@ constexpr int kNumCfgs = sizeof(kCfgs) / sizeof(kCfgs[0]);
 // in nsys systems.
 constexpr int GB_MAXCTAS = 2;  // CTAs an SM (the kernel's launch bounds)
 template <int G>
-int grid_config(Ctx *c, int32_t n, int64_t nnzb, int nsys, int *grid, int *capb, size_t *smem) {
+int grid_config(Ctx *c, int32_t n, int64_t nnzb, int nsys, bool aligned, int *grid, int *capb,
+                size_t *smem) {
   // room for a tile 15 % above the average (every byte of the stages comes off
   // the L1 that the gathers live in: stages of a third above cost 10 %);
-  // larger ones are read from global memory
+  // larger ones are read from global memory.  Bulk copies start on 16-byte
+  // boundaries, so a matrix that does not is read from global memory throughout
   int cap = (int)((double)nnzb / n * GB_R * 1.15) + 6;
   if (cap > 256) cap = 256;
-  *capb = cap;
+  if (!aligned) cap = 0;
+  *capb = aligned ? cap : -1;
   auto kern = k_batched_grid<G>;
   static PerDeviceOnce attr;
   SG_TRY(once_per_device(attr, c->device, [&]() -> int {
@@ -906,8 +910,9 @@ int launch(Ctx *c, cudaStream_t st, const BatchArgs &a, int cfg, int32_t n, int6
     GridArgs g;
     int grid = 0;
     size_t smem = 0;
-    SG_TRY(k.G == 4 ? grid_config<4>(c, n, nnzb, a.nsys, &grid, &g.capb, &smem)
-                    : grid_config<8>(c, n, nnzb, a.nsys, &grid, &g.capb, &smem));
+    const bool al = (uintptr_t)a.vals % 16 == 0 && (uintptr_t)a.colidx % 16 == 0;
+    SG_TRY(k.G == 4 ? grid_config<4>(c, n, nnzb, a.nsys, al, &grid, &g.capb, &smem)
+                    : grid_config<8>(c, n, nnzb, a.nsys, al, &grid, &g.capb, &smem));
     SG_REQUIRE(grid >= 1, "sg_batched_pcg: the grid-wide kernel does not fit an SM");
     g.b = a;
     g.nnzb = nnzb;

@@ -1,4 +1,6 @@
 """GPU checks of the batched PCG (many uneven cloth sheets in one launch)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -160,3 +162,33 @@ def test_grid_wide_systems_over_many_ctas_repeat(ctx):
             assert bool((cb.status == 1).all()) and float(cb.relres.max()) <= 1e-6
             first = first or got
             assert all(torch.equal(a, b) for a, b in zip(first, got))
+
+
+def test_every_config_takes_unaligned_arrays(ctx):
+    """Values and columns that start one element past a 16-byte boundary: every
+    configuration solves every system, to the solution of the aligned arrays
+    (1e-4, as two solves to a 1e-6 residual agree above)."""
+    from simit_gb300.runtime import call, ptr
+    host = problems.cloth_batch(nsheets=5, lo=6, hi=70, seed=23)
+    cb = problems.ClothBatch(ctx, host, config=3)
+    cb.step()
+    ctx.sync()
+    ref = cb.vout.clone()
+    nnzb = cb.mesh.nnzb
+    with ctx.stream():
+        vals = torch.empty(nnzb * 9 + 1, dtype=torch.float32, device=ctx.device)[1:]
+        cols = torch.empty(nnzb + 1, dtype=torch.int32, device=ctx.device)[1:]
+        vals.copy_(cb.A[:nnzb * 9])
+        cols.copy_(cb.mesh.pattern.colidx[:nnzb].view(torch.int32))
+    assert vals.data_ptr() % 16 and cols.data_ptr() % 16
+    A = _lib.Matrix(cb.mesh.n, 3, nnzb, cb.mesh.pattern.rowptr.data_ptr(), cols.data_ptr(),
+                    _lib.F32, vals.data_ptr())
+    for cfg in range(_lib.load().sg_batched_configs()):
+        with ctx.stream():
+            x = cb.v.clone()
+        call("sg_batched_pcg", ctx.h, cb.nsys, ptr(cb.sys_ptr), ptr(cb.order), ctypes.byref(A),
+             ptr(cb.f), ptr(x), problems.CLOTH["tol"], 10000, cfg, ptr(cb.iters), ptr(cb.status),
+             ptr(cb.relres))
+        ctx.sync()
+        assert bool((cb.status == 1).all()) and float(cb.relres.max()) <= 1e-6, cfg
+        assert float((x - ref).norm()) <= 1e-4 * float(ref.norm()), cfg
