@@ -28,7 +28,7 @@
 // (element blocks written out and gathered, or one group of lanes a row):
 //   linear FP32 stiffness + force 3.20 -> 1.6 ms (with the element-blocks
 //   plan), 7.6 -> 1.65 ms (without); neo-Hookean FP32 10.3 -> 2.1, FP64
-//   60 -> 18; heat FP32 1.4 -> 0.78, FP64 10.3 -> 2.1 ms.
+//   60 -> 18; heat FP32 1.4 -> 0.77, FP64 10.3 -> 2.3 ms.
 // At 128^3 the linear map takes 3.7 ms (was 7.6), at 64^3 the neo-Hookean
 // one 0.63 (3.0).
 // 32 rows a tile: 16 rows cost 2.35 ms in the linear map (3.0 evaluations an
@@ -223,9 +223,13 @@ template <typename T> struct NeoTile : TileFin<T> {
 
 // P1 heat: the ten distinct values of the element matrix and the four of its
 // vector, once per element, so that a slot's sum is one addition a block (the
-// FP64 pipe bounds the FP64 map).  EXACT: HeatElem's operations in its order;
-// else the pairs with the fourth vertex come from the other three
-// (g_3 = -(g_0 + g_1 + g_2)) and the vector from the sum of T0.
+// FP64 pipe bounds the FP64 map).  EXACT: the reference's operations in its
+// order; else contracted, with the vector from the sum of T0.  The fourth
+// gradient is formed before it is multiplied: products with it taken from the
+// other three vertices' (g_3 . g_3 = sum of g_i . g_j) lose the square of a
+// slender element's aspect ratio instead of the ratio itself, in FP32 the sign
+// of the diagonal at 1,000.  (At 96^3 that saves FP64 2.28 -> 2.10 ms, FP32
+// nothing: 0.77.)
 template <typename T, bool EXACT> struct HeatTile : TileFin<T> {
   static constexpr int CARD = 4, BS = 1;
   static constexpr bool HAS_MAT = true, HAS_VEC = true;
@@ -236,12 +240,12 @@ template <typename T, bool EXACT> struct HeatTile : TileFin<T> {
 #pragma unroll
     for (int q = 0; q < 9; ++q) g[q / 3][q % 3] = a.B[9 * e + q];
 #pragma unroll
+    for (int d = 0; d < 3; ++d) g[3][d] = -((g[0][d] + g[1][d]) + g[2][d]);
+#pragma unroll
     for (int j = 0; j < 4; ++j) t[j] = a.T0[vv[j]];
     const T W = a.W[e], kw = (a.dt * a.kappa[e]) * W;
     if (EXACT) {
       const T mw = W / T(20.0), mw2 = T(2.0) * mw;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) g[3][d] = -((g[0][d] + g[1][d]) + g[2][d]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         T bi = 0;
@@ -257,20 +261,13 @@ template <typename T, bool EXACT> struct HeatTile : TileFin<T> {
       }
     } else {
       const T mw = W * T(0.05), mw2 = T(2.0) * mw;
-      T d[3][3], s[3];
 #pragma unroll
-      for (int i = 0; i < 3; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = i; j < 3; ++j)
-          d[i][j] = d[j][i] = (g[i][0] * g[j][0] + g[i][1] * g[j][1]) + g[i][2] * g[j][2];
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        s[i] = (d[i][0] + d[i][1]) + d[i][2];
-#pragma unroll
-        for (int j = i; j < 3; ++j) rec[tri_index(4, i, j)] = (i == j ? mw2 : mw) + kw * d[i][j];
-        rec[tri_index(4, i, 3)] = mw - kw * s[i];
-      }
-      rec[9] = mw2 + kw * ((s[0] + s[1]) + s[2]);
+        for (int j = i; j < 4; ++j)
+          rec[tri_index(4, i, j)] =
+              (i == j ? mw2 : mw) +
+              kw * ((g[i][0] * g[j][0] + g[i][1] * g[j][1]) + g[i][2] * g[j][2]);
       const T ts = (t[0] + t[1]) + (t[2] + t[3]);
 #pragma unroll
       for (int i = 0; i < 4; ++i) rec[10 + i] = mw * (ts + t[i]);

@@ -148,3 +148,43 @@ def test_tets(ctx, oracle, kind, plan):
         f = assemble_tet_force(mesh, model, x, v, c, B, W, mu, lam, 0.01, 1e3, grav, exact=False)
         close(K, oK, 1e-12)
         close(f, of, 1e-12)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("exact", [False, True])
+def test_heat_slender_elements(ctx, dtype, exact):
+    """Needles (a face of side h, the fourth vertex at distance 1, listed last),
+    one element a row, every entry against the same inputs in higher precision.
+    Rounding g_3 = -(g_0 + g_1 + g_2) twice moves it by d_3 = 2u (|g_0| + |g_1| +
+    |g_2|); an entry then moves by the products with d_3 and by 8u of its terms'
+    magnitudes (three products, their two sums, kw's two roundings, the
+    constant, the last addition)."""
+    from simit_gb300.runtime import Mesh, assemble_heat
+    g = meshgen.rng(31)
+    N = 4000
+    h = 10 ** g.uniform(-3, 0, N)
+    q = g.normal(size=(N, 3, 3))
+    B = q / h[:, None, None]
+    B[:, 2] = -(B[:, 0] + B[:, 1]) + g.normal(size=(N, 3))
+    W, kappa, dt = g.uniform(0.5, 1, N) * 1e-3, g.uniform(0.5, 1, N) * 1e3, 1.0
+    np_t = np.float32 if dtype == torch.float32 else np.float64
+    B, W, kappa = (a.astype(np_t) for a in (B, W, kappa))
+    mesh = Mesh(ctx, 4 * N, np.arange(4 * N, dtype=np.int32), 4)
+    A, _ = assemble_heat(mesh, B.reshape(-1), W, kappa, dt, np.zeros(4 * N), dtype=dtype,
+                         exact=exact)
+    ctx.sync()
+    got = _np(A)[:16 * N].reshape(N, 4, 4)
+    up = np.float64 if dtype == torch.float32 else np.longdouble
+    u = up(np.finfo(np_t).eps) / 2
+    Bu, Wu = B.astype(up), W.astype(up)
+    G = np.concatenate([Bu, -Bu.sum(1, keepdims=True)], 1)
+    d = np.zeros_like(G)
+    d[:, 3] = 2 * u * np.abs(Bu).sum(1)
+    kw = (kappa.astype(up) * Wu)[:, None, None]
+    mass = Wu[:, None, None] / 20 * (1 + np.eye(4, dtype=up))
+    ref = mass + kw * np.einsum("nik,njk->nij", G, G)
+    aG = np.abs(G)
+    moved = np.einsum("nik,njk->nij", d, aG) + np.einsum("nik,njk->nij", aG, d) + \
+        np.einsum("nik,njk->nij", d, d)
+    bound = kw * moved + 8 * u * (mass + kw * np.einsum("nik,njk->nij", aG + d, aG + d))
+    assert np.all(np.abs(got - ref) <= bound)
