@@ -74,8 +74,8 @@ class HeteroElasticity:
                  plan="gather", learned_params=None, learned_exec=_lib.MPNN_EXEC_FOLDED,
                  tune=False, reliable_delta=0.1):
         self.ctx, self.host, self.dtype = ctx, host, dtype
-        # plan: the element-parallel assembly plan ("gather", "colored"; each
-        # element computed once), or None for the row-owner kernels
+        # plan: whose slot map the row tiles read ("gather", "colored"), or None:
+        # they search the rows' columns
         self.mesh = Mesh(ctx, host["n"], host["tets"], 4, plan=plan)
         d = ctx.device
         with ctx.stream():
@@ -89,15 +89,16 @@ class HeteroElasticity:
             self.f = torch.zeros(host["n"] * 3, dtype=dtype, device=d)
         self.B, self.W, _ = tet_precompute(self.mesh, self.X0, RHO, dtype=dtype)
         self.assemble()
-        # tune: the assembly plan and element tile, and the solver's SpMV
-        # schedule, from timings on this mesh and matrix
+        # tune: the assembly timed, and the solver's SpMV schedule chosen, on
+        # this mesh and matrix
         if precision is None:
             precision = _lib.SOLVE_MIXED if dtype == torch.float32 else _lib.SOLVE_F64
         self.tuned = None
         if tune:
             from .runtime import tune_spmv
             m = self.mesh
-            self.tuned = {"assembly": m.tune_assembly(self.assemble_in_place)}
+            # (one candidate: the linear maps run one kernel under every plan)
+            self.tuned = {"assembly": m.tune_assembly(self.assemble_in_place, plans=(plan,))}
             xdt = torch.float32 if precision == _lib.SOLVE_MIXED else torch.float64
             # timed here (and cached); the solver's set-up takes the cached choice
             self.tuned["spmv"] = tune_spmv(ctx, m.n, 3, m.pattern.rowptr, m.pattern.colidx,

@@ -80,3 +80,22 @@ def test_tuned_assembly_not_slower_than_default(ctx, ncell):
     assert p.tuned["spmv"]["g"] == p.tuned["spmv"]["g"]
     ref.close()
     p.close()
+
+
+def test_assembly_tuner_keeps_the_first_of_equal_plans(ctx):
+    """The linear maps run one kernel under every plan, and the plans round
+    differently: tuned instances have the same plan and the same bits every
+    time, and the tuner, given the choice, keeps the first plan."""
+    from simit_gb300 import runtime
+    h = problems.reorder_hetero(problems.hetero_mesh(40))
+    runtime._ASM_TUNE_CACHE.clear()
+    p = problems.HeteroElasticity(ctx, h, dtype=torch.float32, tune=True)
+    A = p.A.clone()
+    for _ in range(8):
+        runtime._ASM_TUNE_CACHE.clear()
+        t = p.mesh.tune_assembly(p.assemble_in_place)
+        p.assemble_in_place()
+        ctx.sync()
+        assert t["plan"] == "gather" and len(t["times"]) == 3
+        assert torch.equal(A, p.A)
+    p.close()
