@@ -496,9 +496,9 @@ def run_learned_solve(args):
 
 def run_assembly_only(args):
     """Profiling driver: the --size heterogeneous-elasticity step's assembly
-    (stiffness map in place + force map, FP32) with the row tiles over the
-    gather plan's element lists, the coloured plan and the row owners, each event-timed over
-    --reps calls; also each plan's set-up time."""
+    (stiffness map in place + force map, FP32) by row tiles with the slot map
+    of the gather plan, with that of the coloured plan and with searched
+    columns, each event-timed over --reps calls; also each plan's set-up time."""
     import torch
     from simit_gb300 import _lib, problems
     from simit_gb300.runtime import Context
@@ -508,7 +508,7 @@ def run_assembly_only(args):
     if not args.no_reorder:
         h = problems.reorder_hetero(h)
     out = {"size": args.size}
-    for name, plan in (("gather", "gather"), ("colored", "colored"), ("row_owner", None)):
+    for name, plan in (("gather", "gather"), ("colored", "colored"), ("no_plan", None)):
         p = problems.HeteroElasticity(ctx, h, dtype=torch.float32,
                                       precond=_lib.PRECOND_BLOCK_JACOBI, plan=plan)
         if plan is not None:
@@ -942,6 +942,11 @@ def _step_timing(prob, st, steps, warmup, barrier):
     return e0.elapsed_time(e1) / steps, results
 
 
+# the linear maps' kernels with exact=False, under every plan
+ASSEMBLY_KERNELS = ("row tiles: k_tile<LinTetTile> (stiffness), k_tile<TetForceTile> (force); "
+                    "a plan's slot map gives the columns, without one they are searched")
+
+
 def _tuned_summary(t):
     """The autotuners' choices for the bench line."""
     if not t:
@@ -950,8 +955,8 @@ def _tuned_summary(t):
     return {"spmv": {"g": sp["g"], "ms": sp["ms"], "default_ms": sp["default_ms"],
                      "meaning": "g < 0: TMA variant -g-1 of sg_bspmv's table; g > 0: lanes "
                                 "per block row of the streaming kernel; 0: default"},
-            "assembly": {"plan": a["plan"], "tile": a["tile"], "ms": a["ms"],
-                         "default_ms": a["default_ms"], "times": a["times"]}}
+            "assembly": {"plan": a["plan"], "ms": a["ms"], "default_ms": a["default_ms"],
+                         "times": a["times"]}}
 
 
 def run_ours(args, rank, world, local):
@@ -980,8 +985,8 @@ def run_ours(args, rank, world, local):
     with ctx.stream():
         prm = torch.tensor(lrn.load_weights("sym"), device=ctx.device)
     # the metric's method: FP32 assembly + learned-preconditioned mixed PCG
-    # tune: the assembly plan / element tile and the SpMV schedule from
-    # timings on this mesh (set-up, outside the timed steps)
+    # tune: the assembly timed and the SpMV schedule chosen on this mesh
+    # (set-up, outside the timed steps)
     prob = problems.HeteroElasticity(ctx, host, dtype=torch.float32,
                                      precond=_lib.PRECOND_LEARNED, learned_params=prm,
                                      storage=_lib.STORAGE_SYMMETRIC if args.sym
@@ -1104,12 +1109,7 @@ def run_ours(args, rank, world, local):
                 "algorithmic_bytes": asm_bytes, "GBps": asm_bytes / (asm_ms / 1e3) / 1e9,
                 "implementation_bytes": impl_bytes,
                 "implementation_GBps": impl_bytes / (asm_ms / 1e3) / 1e9,
-                "plan": m.plan, "tile": int(m.s.asm_tile) or 256,
-                "kernels": {"gather": "row tiles: k_tile<LinTetTile> (stiffness), "
-                                      "k_tile<TetForceTile> (force)",
-                            "colored": "coloured plan: k_colored<LinTetElem>, "
-                                       "k_colored<TetForceElem> per colour",
-                            None: "row owners: k_rows<LinTetElem>, k_rows<TetForceElem>"}[m.plan]}
+                "plan": m.plan, "kernels": ASSEMBLY_KERNELS}
     if not args.no_jit:
         assembly["jit_stiffness"] = time_jit_stiffness(ctx, prob)
 
@@ -1279,8 +1279,9 @@ def run_secondary(args):
 
 def time_jit_stiffness(ctx, prob):
     """The linear-tet stiffness map of the step from its element function
-    compiled at run time (sg_jit_assembly_create), timed beside the
-    precompiled k_rows<LinTetElem>; both write the same matrix, bit for bit."""
+    compiled at run time (sg_jit_assembly_create, a row-owner kernel), timed
+    beside the precompiled k_tile<LinTetTile> without a plan; both write the
+    same matrix, bit for bit."""
     import torch
     from simit_gb300 import _lib, jit_elements, problems
     from simit_gb300.runtime import JitAssembly, call, dtype_code, ptr
@@ -1293,7 +1294,7 @@ def time_jit_stiffness(ctx, prob):
     with ctx.stream():
         out = torch.empty_like(prob.A)
 
-    # the precompiled row-owner kernel (the same sg_mesh without its plan)
+    # the precompiled map without a plan (the same sg_mesh without its own)
     import ctypes
     plain = _lib.Mesh.from_buffer_copy(m.s)
     plain.slots = plain.color_order = plain.color_ptr = None
