@@ -214,3 +214,35 @@ def test_gather_plan_repeated_endpoints(ctx):
     b = assemble_blocks(gat, eb, 3, exact=False)
     ctx.sync()
     assert np.allclose(_np(a), _np(b), rtol=1e-13, atol=1e-13 * np.abs(_np(a)).max())
+
+
+@pytest.mark.parametrize("plan", ["colored", "gather", None])
+@pytest.mark.parametrize("card,bs", [(2, 1), (2, 3), (3, 1), (3, 2), (4, 2), (4, 3)])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_blocks_in_the_plan_s_order(ctx, oracle, plan, card, bs, dtype):
+    """Caller-evaluated blocks, some elements with a vertex twice, written over
+    NaNs: the oracle's loop over the elements in the plan's order (colour by
+    colour, or ascending) -- FP64 only adds, so the same bits; FP32 within the
+    rounding of a slot's sum, (terms + 1) u of the terms' magnitudes."""
+    from simit_gb300.runtime import Mesh, call, dtype_code, ptr
+    g = meshgen.rng(41)
+    n, nE = 150, 900
+    ep = np.stack([g.permutation(n)[:card] for _ in range(nE)]).astype(np.int32)
+    ep[::6, card - 1] = ep[::6, 0]
+    eb = g.normal(size=(nE, card * card * bs * bs)) * 10 ** g.uniform(-3, 3, size=(nE, 1))
+    mesh = Mesh(ctx, n, ep.reshape(-1), card, plan=plan)
+    rp, ci = mesh.pattern.host()
+    with ctx.stream():
+        vals = torch.full((mesh.nnzb * bs * bs,), float("nan"), dtype=dtype, device=ctx.device)
+        d_eb = torch.tensor(eb, device=ctx.device).to(dtype)
+    call("sg_assemble_blocks", ctx.h, mesh.ref(), dtype_code(vals), bs, ptr(d_eb), ptr(vals), 0)
+    ctx.sync()
+    e64 = _np(d_eb).astype(np.float64)
+    order = mesh.colors()[1] if plan == "colored" else np.arange(nE)
+    ref = oracle.assemble_blocks(ep[order].reshape(-1), card, bs, e64[order], rp, ci)
+    if dtype == torch.float64:
+        assert np.array_equal(_np(vals), ref)
+        return
+    scale = oracle.assemble_blocks(ep.reshape(-1), card, bs, np.abs(e64), rp, ci)
+    terms = oracle.assemble_blocks(ep.reshape(-1), card, bs, np.ones_like(e64), rp, ci)
+    assert np.all(np.abs(_np(vals) - ref) <= (terms + 1) * 2.0 ** -24 * scale)
