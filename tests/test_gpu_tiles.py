@@ -188,3 +188,104 @@ def test_heat_slender_elements(ctx, dtype, exact):
         np.einsum("nik,njk->nij", d, d)
     bound = kw * moved + 8 * u * (mass + kw * np.einsum("nik,njk->nij", aG + d, aG + d))
     assert np.all(np.abs(got - ref) <= bound)
+
+
+def _magnitudes(X, x, T, B, W):
+    """Per element: n_i, the sums of |components| of the four gradients (the
+    fourth from the others', as its rounding is), and f, the largest sum of
+    |products| in an entry of F."""
+    Ds = (x[T[:, :3]] - x[T[:, 3:]]).transpose(0, 2, 1)
+    B3 = B.reshape(-1, 3, 3)
+    f = np.abs(Ds) @ np.abs(B3)
+    n = np.abs(B3).sum(2)
+    return np.concatenate([n, n.sum(1, keepdims=True)], 1), f.max((1, 2))
+
+
+@pytest.mark.parametrize("kind", ["fan", "parts", "lattice"])
+@pytest.mark.parametrize("plan", [None, "gather"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_tets_entry_by_entry(ctx, oracle, kind, plan, dtype):
+    """The contracted maps where the tiles change path, every entry against the
+    oracle on the same rounded inputs: rows past the tile's buffers (fan), and
+    11,500 vertices in random order, whose 32-row tiles hold more distinct elements
+    than records and are taken in parts.  Bound: u (64 + the row's elements) of
+    the entry's terms, each term's factors taken by magnitude -- a sum of that
+    many terms, and for a term its products, F's rounding (4 u f in an entry of
+    F, up to 20 u f + 40 u in F^-T g, log J and their products) and g_3's; twice
+    that in FP64, where the oracle rounds as well."""
+    from simit_gb300.runtime import (Mesh, assemble_heat, assemble_tet_force,
+                                     assemble_tet_stiffness)
+    if kind == "parts":
+        g = meshgen.rng(12)
+        mg = meshgen.tet_grid(22, 21, 22)
+        X, T = mg["X0"].reshape(-1, 3), mg["tets"].reshape(-1, 4).astype(int)
+        new = g.permutation(len(X))
+        Y = np.empty_like(X)
+        Y[new] = X
+        X, T = Y, new[T][g.permutation(len(T))]
+    else:
+        X, T = _tets(kind)
+    n, nT = len(X), len(T)
+    tets = T.astype(np.int32).reshape(-1)
+    np_t = np.float32 if dtype == torch.float32 else np.float64
+    g = meshgen.rng(13)
+    edge = min(np.linalg.norm(X[T[:, i]] - X[T[:, j]], axis=1).min()
+               for i in range(4) for j in range(i))
+
+    def inp(a):  # the values the kernels see, as float64
+        return np.asarray(a, np.float64).astype(np_t).astype(np.float64)
+    x = inp(X + 0.02 * edge * g.uniform(-1, 1, (n, 3)))
+    v = inp(g.normal(size=n * 3))
+    mu, lam = inp(g.uniform(1e3, 1e5, nT)), inp(g.uniform(1e3, 1e5, nT))
+    kappa, T0 = inp(10 ** g.uniform(-2, 2, nT)), inp(g.uniform(size=n))
+    c = (g.uniform(size=n) < 0.2).astype(np.int32)
+    h, dt, rho, grav = 2.0 ** -7, 2.0 ** -6, 1024.0, np.array([0.125, 0.25, -9.75])
+    oB, oW, _ = oracle.tet_precompute(X.reshape(-1), tets, rho)
+    B, W = inp(oB), inp(oW)
+    mesh = Mesh(ctx, n, tets, 4, plan=plan)
+    rp, ci = mesh.pattern.host()
+    sl = oracle.slots(tets, 4, rp, ci).astype(np.int64).reshape(nT, 4, 4)
+    cnt = np.bincount(tets, minlength=n)
+    crow = cnt[np.repeat(np.arange(n), np.diff(rp.astype(np.int64)))]
+    u = float(np.finfo(np_t).eps) / 2 * (1 if dtype == torch.float32 else 2)
+    mag, f = _magnitudes(X, x, T, B, W)
+
+    def slots_of(per):  # sums of [nT, 4, 4] terms by slot
+        out = np.zeros(len(ci))
+        np.add.at(out, sl.reshape(-1), per.reshape(-1))
+        return out
+
+    def verts_of(per):  # sums of [nT, 4] terms by vertex
+        out = np.zeros(n)
+        np.add.at(out, tets, per.reshape(-1))
+        return out
+    nn = mag[:, :, None] * mag[:, None, :]
+    mass = (0.25 * rho * W)[:, None, None] * np.eye(4)
+    # heat
+    A, b = assemble_heat(mesh, B, W, kappa, dt, T0, dtype=dtype, exact=False)
+    oA, ob = oracle.heat_assemble(n, tets, B, W, kappa, dt, T0, rp, ci)
+    ctx.sync()
+    w20 = (W / 20)[:, None, None] * (1 + np.eye(4))
+    bound = u * (64 + crow) * slots_of(w20 + (dt * kappa * W)[:, None, None] * nn)
+    assert np.all(np.abs(_np(A) - oA) <= bound)
+    bound = u * (64 + cnt) * verts_of((w20 * np.abs(T0[T])[:, None, :]).sum(2))
+    assert np.all(np.abs(_np(b) - ob) <= bound)
+    # elasticity, model by model
+    for model in (0, 1):
+        grow = 1 + (f if model else 0 * f)
+        oK = oracle.tet_stiffness(model, x.reshape(-1), c, tets, B, W, mu, lam, h, rho, rp, ci)
+        K = assemble_tet_stiffness(mesh, model, x.reshape(-1), c, B, W, mu, lam, h, rho,
+                                   dtype=dtype, exact=False)
+        ctx.sync()
+        k = (h * h * W * (2 * mu + lam) * grow)[:, None, None] * nn + mass
+        bound = u * (64 + crow) * slots_of(k)
+        assert np.all(np.abs(_np(K).reshape(-1, 9) - oK.reshape(-1, 9)).max(1) <= bound), model
+        of = oracle.tet_force(model, x.reshape(-1), v, c, tets, B, W, mu, lam, h, rho, grav)
+        F = assemble_tet_force(mesh, model, x.reshape(-1), v, c, B, W, mu, lam, h, rho, grav,
+                               dtype=dtype, exact=False)
+        ctx.sync()
+        vm = np.abs(v.reshape(n, 3)).max(1)[T]
+        t = (h * W * (2 * mu + 3 * lam) * (1 + f))[:, None] * mag + \
+            (0.25 * rho * W)[:, None] * (h * np.abs(grav).max() + vm)
+        bound = u * (64 + cnt) * verts_of(t)
+        assert np.all(np.abs(_np(F).reshape(n, 3) - of.reshape(n, 3)).max(1) <= bound), model
