@@ -48,13 +48,16 @@ int default_f64_variant(int32_t n, int bs) {
   return (bs == 3 && n >= 4096) || (bs == 1 && n >= 32768) ? kF64Variant : -1;
 }
 
-template <bool DOT>
-static int f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size_t *smem,
-                      int *capb) {
+// Largest number of blocks in a tile of k_bsr3_f64.
+static int f64_cap(const PatternStats &ps) {
   const int bound = F64_ROWS * (ps.maxrow > 0 ? ps.maxrow : 1);
   const int t = ps.tile32 * (F64_ROWS / 32);
-  *capb = t > 0 && t < bound ? t : bound;
-  *smem = f64_smem_bytes(*capb);
+  return t > 0 && t < bound ? t : bound;
+}
+
+template <bool DOT>
+static int f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size_t *smem) {
+  *smem = f64_smem_bytes(f64_cap(ps));
   if (*smem > 200 * 1024) return SG_ERR_UNSUPPORTED;
   static PerDeviceOnce attr;
   SG_TRY(once_per_device(attr, c->device, []() -> int {
@@ -74,12 +77,9 @@ static int f64_config(Ctx *c, int32_t n, const PatternStats &ps, int *grid, size
 template <bool DOT>
 static int f64_launch(Ctx *c, cudaStream_t st, const SolveCtl *ctl, int32_t n, const uint32_t *rp,
                       const uint32_t *ci, const void *v, const void *x, void *y, double *part,
-                      const PatternStats &ps, int grid) {
-  int g = 0, capb = 0;
-  size_t smem = 0;
-  SG_TRY(f64_config<DOT>(c, n, ps, &g, &smem, &capb));
+                      const PatternStats &ps, int grid, size_t smem) {
   k_bsr3_f64<DOT><<<grid, F64_T, smem, st>>>(ctl, n, rp, ci, (const double *)v, (const double *)x,
-                                             (double *)y, part, capb, c->d_err);
+                                             (double *)y, part, f64_cap(ps), c->d_err);
   SG_CHECK_LAUNCH();
   return SG_OK;
 }
@@ -288,11 +288,9 @@ static int tma_any(Ctx *c, cudaStream_t st, bool launch, int bs, int vdt, int xd
                  : csr_f64_config<false>(c, n, ps, grid, smem);
     }
     if (launch)
-      return dot ? f64_launch<true>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid)
-                 : f64_launch<false>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid);
-    int capb = 0;
-    return dot ? f64_config<true>(c, n, ps, grid, smem, &capb)
-               : f64_config<false>(c, n, ps, grid, smem, &capb);
+      return dot ? f64_launch<true>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid, *smem)
+                 : f64_launch<false>(c, st, k, n, rp, ci, v, x, y, part, ps, *grid, *smem);
+    return dot ? f64_config<true>(c, n, ps, grid, smem) : f64_config<false>(c, n, ps, grid, smem);
   }
   if (vdt == SG_F32 && xdt == SG_F32)
     return tma_dispatch<float, float>(c, st, launch, bs, var, dot, k, n, rp, ci, v, x, y, part, ps,
