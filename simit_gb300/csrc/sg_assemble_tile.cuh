@@ -234,7 +234,6 @@ template <typename T, bool EXACT> struct HeatTile : TileFin<T> {
   static constexpr int CARD = 4, BS = 1;
   static constexpr bool HAS_MAT = true, HAS_VEC = true;
   static constexpr int NREC = 15;
-  __device__ static uint32_t flag(const AsmArgs<T> &, int32_t) { return 0u; }
   __device__ static void stage(const AsmArgs<T> &a, int64_t e, const int32_t *vv, T *rec) {
     T g[4][3], t[4];
 #pragma unroll
@@ -370,7 +369,6 @@ template <typename T> struct ScalarSpringTile {
   static constexpr int CARD = 2, BS = 1;
   static constexpr bool HAS_MAT = true, HAS_VEC = false;
   static constexpr int NREC = 1;
-  __device__ static uint32_t flag(const AsmArgs<T> &, int32_t) { return 0u; }
   __device__ static void stage(const AsmArgs<T> &a, int64_t e, const int32_t *vv, T *rec) {
     rec[0] = a.a[e];
   }

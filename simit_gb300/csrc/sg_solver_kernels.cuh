@@ -145,8 +145,6 @@ __device__ __forceinline__ double *sum_buf(unsigned char *sm) {
   return reinterpret_cast<double *>(sm + SUM_OFF);
 }
 
-template <typename T> __device__ __forceinline__ bool finite_(T v) { return isfinite(v); }
-
 constexpr uint32_t GRID_SPINS = 1u << 22;  // barrier polls (seconds)
 
 // Every CTA of the (co-resident) grid arrives; false when the others did not
