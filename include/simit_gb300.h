@@ -152,7 +152,8 @@ typedef struct sg_mesh {
   int32_t maxrow;             /* sg_pattern_maxrow */
   /* Optional plans.  The built-in maps read their elements' columns from
    * slots when it is set (and search the rows otherwise), in the same
-   * summation order.  The caller-evaluated blocks (sg_assemble_blocks) with
+   * summation order (with slot_src a linear tetrahedron's mass joins its
+   * block before the slot's sum).  The caller-evaluated blocks (sg_assemble_blocks) with
    * exact == 0 use a whole plan; exact == 1 keeps the reference's element
    * order bit for bit.  Both plans need slots.
    *  - slot_src_ptr / slot_src set (sg_slot_sources): every slot sums its
